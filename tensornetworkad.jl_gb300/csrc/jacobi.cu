@@ -232,7 +232,7 @@ void jacobi_round_launch(tnad_ctx* c, T* W, T* V, int64_t m, int64_t n, int r, i
     k_jacobi_round_cta<16, T, EIG><<<np2, 128, 0, c->stream>>>(W, V, m, n, r, NP, tol, ae, fro2, flag);
 }
 
-// Block variant of the FP32 round.  The columns are grouped in blocks of 4
+// Block variant of the FP32 round with the eigenvalue rule.  The columns are grouped in blocks of 4
 // (the last one may be short) and the circle-method tournament runs over the
 // NB blocks (NB even; with an odd count of real blocks, block NB − 1 is a bye
 // whose columns lie beyond n and count as absent).  CTA k takes the block pair
@@ -255,7 +255,7 @@ constexpr int kJBRows = 16;     // rows per thread
 // at the end, the 16 stores; the wait on the mbarrier is bounded (2 s of
 // %globaltimer), after which the CTA sets *err, waits once more (bounded) for
 // its copies in flight and returns without rotating.
-template <bool EIG, int TP>
+template <int TP>
 __global__ void __launch_bounds__(kJB * TP) k_jacobi_block(float* __restrict__ W, float* __restrict__ V, int m, int n,
                                                            int NB, int r, int intra, double tol, double abs_eps,
                                                            const double* __restrict__ fro2,
@@ -338,18 +338,12 @@ __global__ void __launch_bounds__(kJB * TP) k_jacobi_block(float* __restrict__ W
       }
 #pragma unroll
       for (int e = 0; e < kJBRows; ++e) {
-        if (EIG) {
-          A = fmaf(vx[e], x[e], A);
-          B = fmaf(vy[e], y[e], B);
-          G = fmaf(vx[e], y[e], G);
-          G2 = fmaf(vy[e], x[e], G2);
-        } else {
-          A = fmaf(x[e], x[e], A);
-          B = fmaf(y[e], y[e], B);
-          G = fmaf(x[e], y[e], G);
-        }
+        A = fmaf(vx[e], x[e], A);
+        B = fmaf(vy[e], y[e], B);
+        G = fmaf(vx[e], y[e], G);
+        G2 = fmaf(vy[e], x[e], G2);
       }
-      if (EIG) G = 0.5f * (G + G2);
+      G = 0.5f * (G + G2);
       A = wsum_t(A);
       B = wsum_t(B);
       G = wsum_t(G);
@@ -370,12 +364,7 @@ __global__ void __launch_bounds__(kJB * TP) k_jacobi_block(float* __restrict__ W
         B += red[slot][w][1];
         G += red[slot][w][2];
       }
-      if (EIG) {
-        do_rot = G != 0.f && fabsf(G) > (float)tol * sqrtf(fabsf(A * B)) + thr_abs;
-      } else {
-        const float sa = sqrtf(A), sb = sqrtf(B);
-        do_rot = G != 0.f && A != 0.f && B != 0.f && fabsf(G) > (float)tol * sa * sb + thr_abs * (sa + sb);
-      }
+      do_rot = G != 0.f && fabsf(G) > (float)tol * sqrtf(fabsf(A * B)) + thr_abs;
       if (do_rot) {
         const float zeta = (B - A) / (2.f * G);
         const float t =
@@ -455,19 +444,18 @@ inline int jacobi_block_tp(int64_t m, int64_t n) {
   return 64;
 }
 
-template <bool EIG>
 void jacobi_block_launch(tnad_ctx* c, float* W, float* V, int64_t m, int64_t n, int tp, int NB, int r, double tol,
                          double ae, const double* fro2, int* flag) {
   static std::atomic<bool> attr{false};
   if (!attr) {
-    TNAD_CK(cudaFuncSetAttribute(k_jacobi_block<EIG, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+    TNAD_CK(cudaFuncSetAttribute(k_jacobi_block<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     attr = true;
   }
   (void)tp;  // 64 threads per pair (jacobi_block_tp)
   const size_t sm = (size_t)2 * kJB * (m + n) * sizeof(float);
   // bulk copies need 16-byte aligned columns: m, n multiples of 4 and aligned bases
   const int bulk = (m % 4 == 0 && n % 4 == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)V & 15) == 0) ? 1 : 0;
-  k_jacobi_block<EIG, 64><<<(unsigned)(NB / 2), kJB * 64, sm, c->stream>>>(W, V, (int)m, (int)n, NB, r,
+  k_jacobi_block<64><<<(unsigned)(NB / 2), kJB * 64, sm, c->stream>>>(W, V, (int)m, (int)n, NB, r,
                                                                            r == 0 ? 1 : 0, tol, ae, fro2, flag, bulk,
                                                                            flag + 2);
 }
@@ -480,13 +468,13 @@ template <typename T, bool EIG = false>
 struct SweepGraph {
   cudaGraphExec_t exec = nullptr;
   double ae_ = -1.0;
-  int tp = 0;  // > 0 (FP32 only): block rounds (k_jacobi_block, tp threads per pair), NB − 1 launches a sweep
+  int tp = 0;  // > 0 (FP32 eigenvalue rule only): block rounds (k_jacobi_block, tp threads per pair), NB − 1 launches a sweep
   ~SweepGraph() {
     if (exec) cudaGraphExecDestroy(exec);
   }
   void run(tnad_ctx* c, const char* family, T* W, T* V, int64_t m, int64_t n, int NP, double tol, double ae,
            const double* fro2, int* flag, double round_flops) {
-    if constexpr (sizeof(T) == 4) {
+    if constexpr (sizeof(T) == 4 && EIG) {
       if (tp > 0) {
         run_blocks(c, family, W, V, m, n, tol, ae, fro2, flag, round_flops * (double)(NP - 1));
         return;
@@ -541,7 +529,7 @@ struct SweepGraph {
       TNAD_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), c->stream);
       for (int r = 0; r < NB - 1 && e == cudaSuccess; ++r) {
-        jacobi_block_launch<EIG>(c, W, V, m, n, tp, NB, r, tol, ae, fro2, flag);
+        jacobi_block_launch(c, W, V, m, n, tp, NB, r, tol, ae, fro2, flag);
         e = cudaGetLastError();
       }
       const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
@@ -767,6 +755,13 @@ __global__ void k_scatter_eig(const double* __restrict__ X, const double* __rest
 void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, double* S, double* V,
                 bool symmetric, int rel_sweeps) {
   TNAD_REQUIRE(m >= n && n >= 1, TNAD_ERR_SHAPE, "svd_jacobi: needs m >= n >= 1");
+  // symmetric A at LAPACK-level accuracy: below kPrecondMinN, and where the
+  // refinement below is not taken, QR-preconditioned sweeps (svd_qr.cu)
+  const bool qrj = symmetric && rel_sweeps == 0 && m == n && svd_qrj_fits(n, n);
+  if (qrj && (n < kPrecondMinN || !c->eig_refine)) {
+    svd_qrj(c, 1, &A, n, n, &U, &S, &V, true);
+    return;
+  }
   WsScope scope(c);
   double* W = ws_d(c, m * n);
   double* Vw = ws_d(c, n * n);
@@ -808,13 +803,18 @@ void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, d
     //
     // A size whose last refinement did not converge (a graded spectrum; the
     // plain path decomposes similar corners every step) skips the next
-    // kEigSkip attempts: those take the SVD-rule FP32 start, whose relative
-    // orthogonality suits the FP64 sweeps, and count as fallbacks.
+    // kEigSkip attempts, which count as fallbacks.  Up to 1024 columns the
+    // fallback is svd_qrj; larger matrices take the SVD-rule FP32 start, whose
+    // relative orthogonality suits the FP64 sweeps.
     bool refine = c->eig_refine && m == n && n <= 2048;
     if (refine && c->eig_skip_n == n && c->eig_skip_left > 0) {
       --c->eig_skip_left;
       ++c->eig_fallback;
       refine = false;
+      if (qrj) {
+        svd_qrj(c, 1, &A, n, n, &U, &S, &V, true);
+        return;
+      }
     }
     float* W32 = ws_f(c, m * n);
     float* V32 = ws_f(c, n * n);
@@ -827,7 +827,7 @@ void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, d
     // block rounds (b columns per block): 1/b of the launches and global passes
     SweepGraph<float> sweep32;
     SweepGraph<float, true> sweep32e;
-    if (c->jacobi_blocks) sweep32.tp = sweep32e.tp = jacobi_block_tp(m, n);
+    if (c->jacobi_blocks) sweep32e.tp = jacobi_block_tp(m, n);
     const double round_flops = (double)(n / 2) * (12.0 * (double)m + 6.0 * (double)n);
     for (int sweep = 0; sweep < kMaxSweeps32; ++sweep) {
       if (refine)
@@ -878,6 +878,10 @@ void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, d
       ++c->eig_fallback;
       c->eig_skip_n = n;
       c->eig_skip_left = kEigSkip;
+      if (qrj) {
+        svd_qrj(c, 1, &A, n, n, &U, &S, &V, true);
+        return;
+      }
     }
     gemm_f64(c, 'N', 'N', m, n, n, 1.0, A, m, Vw, n, 0.0, W, m);
   }

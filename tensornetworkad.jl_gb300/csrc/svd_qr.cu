@@ -1,0 +1,1384 @@
+// FP64 SVD at LAPACK-level accuracy (every triplet to ε·‖A‖) of matrices up to
+// 1024 rows: rank-revealing QR, then one-sided Jacobi on the triangular factor
+// (Drmač and Veselić, "New fast and accurate Jacobi SVD algorithm", SIAM J.
+// Matrix Anal. Appl. 29, 2008).  It serves the decompositions of src/trg.jl:36
+// and src/ctmrg.jl:136 that the product refinement (eig_refine.cu) does not.
+//
+//   A·P = Q·R          Householder QR with column pivoting, stopped at rank r
+//                      once every remaining column is below ½ε of the first
+//                      pivot (what is dropped is below the rounding of A)
+//   Rᵀ·P₂ = Q₂·R₂      a second one (general A, or r < n), r×r
+//   X·Vx = Wn·Σ        one-sided Jacobi, X = R₂ᵀ (or Rᵀ without the second QR)
+//
+// so that A = (Q·P₂·Wn)·Σ·(P·Q₂·Vx)ᵀ, completed by the trailing columns of Q
+// and P·Q₂ where r < n.  Symmetric A with r = n skips the second QR and the
+// accumulation of Vx: the eigenvectors are P·Wn.
+//
+// Why: GB300 issues one FP64 instruction per warp and SM quadrant every 64
+// clocks (76 with all four busy), so the sweeps are paid in instructions and in
+// rounds.  The corners and TRG splits are graded (singular values from 1 to
+// 1e-16): plain Jacobi sweeps took 9-36 of them there, on the triangular factor
+// it is 6-10, and the rank cut leaves ~250 of 400 columns of a χ = 20 split.
+// Each stage is one cooperative kernel (one launch instead of n − 1 per sweep).
+// Measured on one GB300 against FP64 element rounds (k_jacobi_round_cta): TRG at
+// χ = 20, 7 steps with gradient 704 → 28 ms; D=3, χ=36 energy and gradient (n =
+// 324) 349 → 65 ms; one n = 80 decomposition 4.9 → 1.4 ms, n = 255 26.7 → 5.9 ms.
+// At n = 324 the first QR takes 2.0 ms, the FP32 sweeps 3.4, the FP64 ones 2.6.
+#include <algorithm>
+#include <atomic>
+#include <cfloat>
+#include <climits>
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+
+#include "tc_common.cuh"
+#include "tnad_internal.h"
+
+namespace tnad {
+
+namespace {
+
+constexpr int kMaxSvdRows = 1024;
+constexpr int kSvdSweeps = 60;
+constexpr int kPreMin = 24;         // columns from which FP32 sweeps precede the FP64 ones
+constexpr int kPreSweeps = 20;
+constexpr float kPreCos = 1e-3f;    // a sweep that rotated no larger |cos| leaves ~1e-6: hand over
+constexpr int kScaleExp = 40;  // the largest |entry| is scaled to 2^40: squared norms of
+                               // columns down to ½ε of it stay inside the FP32 range
+
+// Per-problem counters (ints): rank, non-finite input, converged sweep count
+// (0: none), barrier counter of each of the three kernels, rotations per sweep
+// and the largest |cos| of a rotated pair per sweep (float bits).
+enum { kiRank = 0, kiBad = 1, kiSweeps = 2, kiExp = 3, kiErr = 4, kiPre = 5, kiBar = 8, kiRot = 16, kiCos = 16 + kSvdSweeps,
+       kiTan = 16 + 2 * kSvdSweeps, kiRot32 = 16 + 3 * kSvdSweeps, kiCos32 = kiRot32 + kPreSweeps, kiCount = kiCos32 + kPreSweeps };
+
+struct SvdProb {
+  const double* A;
+  double *X, *X2, *Vx;    // Rᵀ (n×n), R₂ᵀ and the accumulated rotations; leading dimension ldx
+  double *H, *H2;         // Householder vectors of the two factorisations, m×n and n×n
+  double *hinv, *hinv2;   // 2/vᵀv of each
+  int *perm, *perm2;      // perm[k]: column at pivot position k
+  double *cand;           // 2 × G × ldc candidate columns
+  unsigned long long* key;  // 2 × G candidate keys, and G column maxima
+  float *W32, *V32;       // FP32 copies of X and of the rotations; leading dimension ld32
+  double *W, *Wbuf;       // X·V after the FP32 sweeps (W null: none)
+  double *nrm, *sv;       // squared column norms, singular values (unsorted)
+  double *U, *S, *V;
+  int* info;
+};
+
+struct SvdArgs {
+  SvdProb p[2];
+  int m, n, ldx, ldc, ld32;
+  int second;      // run the second QR also when r = n
+  float trunc;     // rank cut relative to the first pivot
+  double tol;      // Jacobi: |cos| above which a pair rotates (FP64 and FP32 sweeps)
+  float tol32;
+  int max_sweeps;
+};
+
+__device__ __forceinline__ double wsum_d(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+__device__ __forceinline__ float wsum_f(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// FP64 ↔ FP32 by integer operations: the conversion instructions take ~95
+// clocks of the FP64 pipe each, these about 20 and 11 (truncation; values below
+// the FP32 normal range become 0, above it are not expected: everything is
+// scaled to [2^-60, 2^100])
+__device__ __forceinline__ float d2f(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d), a = hi & 0x7fffffffu;
+  const unsigned r = a < (897u << 20) ? 0u : (((a - (896u << 20)) << 3) | (lo >> 29));
+  return __uint_as_float(r | (hi & 0x80000000u));
+}
+
+__device__ __forceinline__ double f2d(float f) {
+  const unsigned b = __float_as_uint(f), a = b & 0x7fffffffu;
+  const unsigned hi = a ? (a >> 3) + (896u << 20) : 0u;
+  return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)(b << 29));
+}
+
+// FP32 quotient and square root to 1-2 ulp (they start Newton steps or only
+// decide angles): ~30 clocks instead of ~150 for the rounded ones
+__device__ __forceinline__ float fsqrt_ap(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// tan of the rotation that diagonalises [[a, g], [g, b]] with df = b − a, g2 = 2g (FP32)
+__device__ __forceinline__ float jacobi_tan(float df, float g2) {
+  if (fabsf(df) >= fabsf(g2)) {
+    const float w = __fdividef(g2, df);
+    return __fdividef(w, 1.f + fsqrt_ap(fmaf(w, w, 1.f)));
+  }
+  const float w = __fdividef(df, g2);
+  return __fdividef(copysignf(1.f, w), fabsf(w) + fsqrt_ap(fmaf(w, w, 1.f)));
+}
+
+// 1/√x by one cubic Newton (Halley) step from the FP32 value: relative error
+// (5/16)·e³ with e ~ 2e-7.  x inside the FP32 normal range.  Six FP64
+// instructions; sqrt() and a division take about 1300 clocks of the FP64 pipe.
+__device__ __forceinline__ double rsqrt_fast(double x) {
+  const double y = f2d(rsqrtf(d2f(x)));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// 1/x by two Newton steps from the FP32 value
+__device__ __forceinline__ double rcp_fast(double x) {
+  double y = f2d(__fdividef(1.f, d2f(x)));
+  y = fma(fma(-x, y, 1.0), y, y);
+  return fma(fma(-x, y, 1.0), y, y);
+}
+
+// Barrier over the CTAs of one problem.  CL: they form one thread-block cluster
+// (hardware barrier, 0.24 µs).  Otherwise a counter in global memory (1.1 µs
+// for 16 to 152 CTAs): the wait is bounded (2 s of %globaltimer); a CTA that
+// gives up sets *err, which the others see, and all of them return.
+template <bool CL>
+struct GridBar {
+  unsigned* cnt;
+  unsigned tgt, G;
+  int* err;
+  int* dead;  // shared: 1 once a wait gave up
+  __device__ bool sync() {
+    if (CL) {
+      asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+      return true;
+    }
+    __syncthreads();
+    tgt += G;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+      unsigned v, spins = 0;
+      const uint64_t t0 = tc::gtime();
+      while (true) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
+        if ((int)(v - tgt) >= 0) break;
+        if ((++spins & 255u) == 0 && (tc::gtime() - t0 > 2000000000ull || atomicAdd(err, 0) != 0)) {
+          atomicExch(err, 1);
+          *dead = 1;
+          break;
+        }
+      }
+      __threadfence();
+    }
+    __syncthreads();
+    return *dead == 0;
+  }
+};
+
+// ---------------------------------------------------------------------------
+// Householder QR with column pivoting.  One warp per column, the column in
+// registers (R chunks of 32 rows); CTA b holds the columns b, b + G, b + 2G...
+// Step k: every CTA has published its longest remaining column with its norm;
+// one barrier; every warp finds the longest of all (ties: smallest index),
+// reads that column from L2, forms its Householder vector (the same arithmetic
+// in every warp) and updates its own column.  One barrier and two dependent L2
+// reads a step; the norms that only choose pivots are FP32 sums of squares.
+// STAGE 0: A (m×n, scaled by a power of two) → H, hinv, perm, rank, X = Rᵀ in
+// pivot order.  STAGE 1: the r columns of X → H2, hinv2, perm2, X2 = R₂ᵀ.
+// ---------------------------------------------------------------------------
+template <int R, bool CL, int STAGE>
+__global__ void __launch_bounds__(256) k_qrcp(SvdArgs a) {
+  const SvdProb& q = a.p[blockIdx.y];
+  const int G = gridDim.x, cta = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+  int m, n;
+  if (STAGE == 0) {
+    m = a.m;
+    n = a.n;
+  } else {
+    m = a.n;
+    n = q.info[kiRank];
+    if (q.info[kiErr] || n == 0 || (!a.second && n == a.n)) return;  // uniform over the problem's CTAs
+  }
+  double* H = STAGE == 0 ? q.H : q.H2;
+  double* hinv = STAGE == 0 ? q.hinv : q.hinv2;
+  int* perm = STAGE == 0 ? q.perm : q.perm2;
+  double* X = STAGE == 0 ? q.X : q.X2;
+  __shared__ unsigned long long wkey[8];
+  __shared__ unsigned picked_mask[kMaxSvdRows / 32];
+  __shared__ int dead;
+  if (threadIdx.x == 0) dead = 0;
+  for (int i = threadIdx.x; i < kMaxSvdRows / 32; i += blockDim.x) picked_mask[i] = 0u;
+  __syncthreads();
+  GridBar<CL> bar{reinterpret_cast<unsigned*>(q.info + kiBar + STAGE), 0u, (unsigned)G, q.info + kiErr, &dead};
+
+  const int col = warp * G + cta;
+  const bool have = col < n;
+  double c[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int row = lane + 32 * i;
+    c[i] = (have && row < m) ? (STAGE == 0 ? q.A[row + (int64_t)col * m] : __ldcg(&q.X[row + (int64_t)col * a.ldx]))
+                             : 0.0;
+  }
+  if (STAGE == 0) {
+    // scale so that the largest |entry| lies in [2^40, 2^41): exact, undone on S
+    unsigned long long mx = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(c[i]));
+      mx = b > mx ? b : mx;  // NaN and infinities order above every finite value
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long b = __shfl_xor_sync(0xffffffffu, mx, o);
+      mx = b > mx ? b : mx;
+    }
+    if (lane == 0) wkey[warp] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < nwarp; ++w) mx = wkey[w] > mx ? wkey[w] : mx;
+      __stcg(&q.key[2 * G + cta], mx);
+    }
+    if (!bar.sync()) return;
+    mx = 0;
+    for (int g = lane; g < G; g += 32) {
+      const unsigned long long b = __ldcg(&q.key[2 * G + g]);
+      mx = b > mx ? b : mx;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long b = __shfl_xor_sync(0xffffffffu, mx, o);
+      mx = b > mx ? b : mx;
+    }
+    const double amax = __longlong_as_double((long long)mx);
+    if (!(amax > 0.0) || !isfinite(amax)) {  // zero or non-finite A (uniform)
+      if (cta == 0 && threadIdx.x == 0) {
+        q.info[kiRank] = 0;
+        q.info[kiBad] = amax == 0.0 ? 0 : 1;
+      }
+      for (int j = cta * blockDim.x + threadIdx.x; j < n; j += G * blockDim.x) perm[j] = j;
+      return;
+    }
+    const int e = ilogb(amax) - kScaleExp;
+#pragma unroll
+    for (int i = 0; i < R; ++i) c[i] = scalbn(c[i], -e);
+    if (cta == 0 && threadIdx.x == 0) q.info[kiExp] = e;
+  }
+  float nr = 0.f;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const float f = d2f(c[i]);
+    nr = fmaf(f, f, nr);
+  }
+  nr = wsum_f(nr);
+  int pos = -1;
+  float thr2 = 0.f;
+  const int kmax = min(m, n);
+  int k = 0;
+  for (; k < kmax; ++k) {
+    // this CTA's longest remaining column
+    const unsigned long long mykey =
+        (have && pos < 0) ? (((unsigned long long)__float_as_uint(nr) << 32) | (0xffffffffu - (unsigned)col)) : 0ull;
+    if (lane == 0) wkey[warp] = mykey;
+    __syncthreads();
+    unsigned long long best = 0;
+    for (int w = 0; w < nwarp; ++w) best = wkey[w] > best ? wkey[w] : best;
+    double* mine = q.cand + ((int64_t)(k & 1) * G + cta) * a.ldc;
+    if (best != 0 && best == mykey) {
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (32 * i < m && 32 * i + 31 >= k && lane + 32 * i < m) __stcg(&mine[lane + 32 * i], c[i]);
+    }
+    if (threadIdx.x == 0) __stcg(&q.key[(k & 1) * G + cta], best);
+    if (!bar.sync()) return;
+    best = 0;
+    for (int g = lane; g < G; g += 32) {
+      const unsigned long long b = __ldcg(&q.key[(k & 1) * G + g]);
+      best = b > best ? b : best;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long b = __shfl_xor_sync(0xffffffffu, best, o);
+      best = b > best ? b : best;
+    }
+    const float n2 = __uint_as_float((unsigned)(best >> 32));
+    const int wj = (int)(0xffffffffu - (unsigned)best);
+    if (STAGE == 0) {
+      if (k == 0) thr2 = a.trunc * a.trunc * n2;
+      if (n2 <= thr2) break;  // the rest is below the rounding of A
+    }
+    if (threadIdx.x == 0) picked_mask[wj >> 5] |= 1u << (wj & 31);
+    const double* win = q.cand + ((int64_t)(k & 1) * G + (wj % G)) * a.ldc;
+    double x[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int row = lane + 32 * i;
+      x[i] = (32 * i + 31 >= k && row >= k && row < m) ? __ldcg(&win[row]) : 0.0;
+    }
+    // v = x − β·e_k, β = −sign(α)·‖x‖, H = I − hk·v·vᵀ with hk = 2/vᵀv = 1/(‖x‖² + |α|‖x‖)
+    double s2 = 0.0, al = 0.0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (32 * i < m && 32 * i + 31 >= k) s2 = fma(x[i], x[i], s2);
+      if (i == (k >> 5)) al = x[i];
+    }
+    s2 = wsum_d(s2);
+    al = __shfl_sync(0xffffffffu, al, k & 31);
+    double beta = 0.0, hk = 0.0;
+    if (s2 > 1e-30) {
+      const double y = rsqrt_fast(s2);
+      double sg = s2 * y;
+      sg = fma(0.5 * y, fma(-sg, sg, s2), sg);
+      beta = al >= 0.0 ? -sg : sg;
+      hk = rcp_fast(fma(fabs(al), sg, s2));
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (i == (k >> 5) && lane == (k & 31)) x[i] = al - beta;
+    } else {
+#pragma unroll
+      for (int i = 0; i < R; ++i) x[i] = 0.0;
+    }
+    if (cta == 0 && warp == 0) {
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (lane + 32 * i < m) H[lane + 32 * i + (int64_t)k * m] = x[i];
+      if (lane == 0) {
+        hinv[k] = hk;
+        perm[k] = wj;
+      }
+    }
+    if (have && pos < 0) {
+      if (col == wj) {
+        pos = k;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          const int row = lane + 32 * i;
+          c[i] = row < k ? c[i] : (row == k ? beta : 0.0);
+        }
+      } else {
+        double d = 0.0;
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if (32 * i < m && 32 * i + 31 >= k) d = fma(x[i], c[i], d);
+        d = wsum_d(d) * hk;
+        nr = 0.f;
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if (32 * i < m && 32 * i + 31 >= k) {
+            c[i] = fma(-d, x[i], c[i]);
+            const float f = lane + 32 * i > k ? d2f(c[i]) : 0.f;
+            nr = fmaf(f, f, nr);
+          }
+        nr = wsum_f(nr);
+      }
+    }
+  }
+  const int r = k;  // rank (STAGE 0: k < kmax when the rest was cut)
+  __syncthreads();
+  if (have && pos < 0) {  // columns that were never a pivot follow in index order
+    int u = 0;
+    for (int w = 0; w < (col >> 5); ++w) u += 32 - __popc(picked_mask[w]);
+    u += (col & 31) - __popc(picked_mask[col >> 5] & ((1u << (col & 31)) - 1u));
+    pos = r + u;
+    if (lane == 0) perm[pos] = col;
+  }
+  if (have) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int row = lane + 32 * i;
+      if (row < r) X[pos + (int64_t)row * a.ldx] = c[i];
+    }
+  }
+  if (STAGE == 0 && cta == 0 && threadIdx.x == 0) q.info[kiRank] = r;
+}
+
+// ---------------------------------------------------------------------------
+// One-sided Jacobi sweeps on the rc columns of X (mx rows), one launch.
+// Columns are grouped in blocks of two; a round of the circle method pairs the
+// blocks and CTA k takes the block pair (P, Q): its 4 columns come from L2 to
+// shared memory (16-byte cp.async), the cross pairs are rotated in two inner
+// rounds of two disjoint pairs (in a sweep's first round the pairs inside P and
+// Q first), 64 threads per pair, and the columns go back; one barrier a round.
+// Blocks of two halve the barriers of single columns and leave one pair per two
+// SM quadrants; blocks of four leave half of the SMs without work.
+//
+// FP64 instructions are what a round costs, so the squared norms are carried
+// (a ← a − tγ, b ← b + tγ; formed anew at each sweep's start), the angle starts
+// in FP32 and takes one Newton step in FP64, and cos comes from rsqrt_fast: 14
+// instructions where the quotients and square roots took ~4000 clocks.
+// Sweeps end when no pair rotates, or when the largest |cos| that a sweep rotated
+// times its largest |tan| is below half of tol: a rotation by t changes the
+// |cos| of its columns with the others, zeroed before it, by t times theirs (not
+// by the square where two singular values are close and t is large).
+// ---------------------------------------------------------------------------
+template <int RJ, bool ACCV, bool CL>
+__global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  const SvdProb& q = a.p[blockIdx.y];
+  const int rc = q.info[kiRank];
+  const bool two = a.second || rc < a.n;
+  const int mx = two ? rc : a.n;
+  const int nreal = (rc + 1) >> 1, NB = nreal + (nreal & 1);
+  const int active = NB >> 1, cta = blockIdx.x;
+  if (!CL && cta >= max(active, 1)) return;
+  if (q.info[kiErr]) return;
+  double* W = q.W ? q.W : (two ? q.X2 : q.X);
+  double* V = q.Vx;
+  const int ldx = a.ldx;
+  const int ldw = (mx + 1) & ~1, ldv = ACCV ? (rc + 1) & ~1 : 0, cst = ldw + ldv;
+  double* sm = reinterpret_cast<double*>(sm_raw);  // 4 columns of cst doubles: W rows, then V rows
+  __shared__ double nrm4[4], red[2][2];
+  __shared__ int dead, nrot, cosmax, tanmax;
+  if (threadIdx.x == 0) dead = nrot = cosmax = tanmax = 0;
+  __syncthreads();
+  GridBar<CL> bar{reinterpret_cast<unsigned*>(q.info + kiBar + 2), 0u, (unsigned)max(active, 1), q.info + kiErr,
+                  &dead};
+  if (ACCV && !q.W) {  // Vx = I (each CTA its own share of the columns)
+    const int nc = CL ? (int)gridDim.x : max(active, 1);
+    for (int j = cta; j < rc; j += nc)
+      for (int i = threadIdx.x; i < rc; i += blockDim.x) __stcg(&V[i + (int64_t)j * ldx], i == j ? 1.0 : 0.0);
+    if (!bar.sync()) return;
+  }
+  const int grp = threadIdx.x >> 6, lt = threadIdx.x & 63, wip = (threadIdx.x >> 5) & 1, lane = threadIdx.x & 31;
+  const float tolf = (float)a.tol;
+
+  // rotate local columns x < y (in global order) of this thread group; their W
+  // rows stay in registers between the dot product and the rotation
+  auto process = [&](int x, int y, bool present) {
+    double g = 0.0, u[RJ], v[RJ];
+    double* wx = sm + (int64_t)x * cst;
+    double* wy = sm + (int64_t)y * cst;
+    if (present) {
+#pragma unroll
+      for (int e = 0; e < RJ; ++e) {
+        const int i = lt + 64 * e;
+        u[e] = i < mx ? wx[i] : 0.0;
+        v[e] = i < mx ? wy[i] : 0.0;
+      }
+#pragma unroll
+      for (int e = 0; e < RJ; ++e)
+        if (64 * e < mx) g = fma(u[e], v[e], g);
+      g = wsum_d(g);
+      if (lane == 0) red[grp][wip] = g;
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(grp + 1) : "memory");
+    if (present) {
+      g = red[grp][0] + red[grp][1];
+      const double na = nrm4[x], nb = nrm4[y];
+      const float gf = d2f(g), cs2 = fsqrt_ap(d2f(na)) * fsqrt_ap(d2f(nb));
+      if (fabsf(gf) > tolf * cs2) {
+        const double dl = nb - na;
+        const float df = d2f(dl), g2 = 2.f * gf;
+        const float t0 = jacobi_tan(df, g2);
+        // one Newton step on γt² + (b − a)t − γ = 0
+        const double td = f2d(t0);
+        const double fr = fma(fma(g, td, dl), td, -g);
+        const double t = fma(-fr, f2d(__fdividef(1.f, fmaf(g2, t0, df))), td);
+        const double cs = rsqrt_fast(fma(t, t, 1.0)), sn = cs * t;
+#pragma unroll
+        for (int e = 0; e < RJ; ++e) {
+          const int i = lt + 64 * e;
+          if (i < mx) {
+            wx[i] = cs * u[e] - sn * v[e];
+            wy[i] = sn * u[e] + cs * v[e];
+          }
+        }
+        if (ACCV) {
+          double* vx = wx + ldw;
+          double* vy = wy + ldw;
+#pragma unroll
+          for (int e = 0; e < RJ; ++e) {
+            const int i = lt + 64 * e;
+            u[e] = i < rc ? vx[i] : 0.0;
+            v[e] = i < rc ? vy[i] : 0.0;
+          }
+#pragma unroll
+          for (int e = 0; e < RJ; ++e) {
+            const int i = lt + 64 * e;
+            if (i < rc) {
+              vx[i] = cs * u[e] - sn * v[e];
+              vy[i] = sn * u[e] + cs * v[e];
+            }
+          }
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(grp + 1) : "memory");  // norms read by all of the group
+        if (lt == 0) {
+          const double tg = t * g;
+          nrm4[x] = na - tg;
+          nrm4[y] = nb + tg;
+          atomicAdd(&nrot, 1);
+          atomicMax(&cosmax, __float_as_int(cs2 > 0.f ? fminf(__fdividef(fabsf(gf), cs2), 1.f) : 1.f));
+          atomicMax(&tanmax, __float_as_int(fabsf(t0)));
+        }
+      }
+    }
+  };
+
+  const int rounds = NB - 1;
+  int sweep = 0;
+  bool done = rc < 2;
+  for (; sweep < a.max_sweeps && !done; ++sweep) {
+    for (int r = 0; r < rounds; ++r) {
+      if (cta < active) {
+        int P, Q;
+        if (cta == 0) {
+          P = r;
+          Q = NB - 1;
+        } else {
+          P = (r + cta) % (NB - 1);
+          Q = (r - cta + (NB - 1)) % (NB - 1);
+        }
+        if (P > Q) {
+          const int t = P;
+          P = Q;
+          Q = t;
+        }
+        const int gc[4] = {2 * P, 2 * P + 1, 2 * Q, 2 * Q + 1};
+        // 4 columns of W and V to shared memory
+        for (int l = 0; l < 4; ++l) {
+          if (gc[l] >= rc) continue;
+          const double* ws = W + (int64_t)gc[l] * ldx;
+          const uint32_t dst = tc::su32(sm + (int64_t)l * cst);
+          for (int i = threadIdx.x; i < (ldw >> 1); i += blockDim.x)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(ws + 2 * i) : "memory");
+          if (ACCV) {
+            const double* vs = V + (int64_t)gc[l] * ldx;
+            for (int i = threadIdx.x; i < (ldv >> 1); i += blockDim.x)
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 8u * ldw + 16u * i), "l"(vs + 2 * i)
+                           : "memory");
+          }
+        }
+        if (r > 0 && threadIdx.x < 4 && gc[threadIdx.x] < rc) nrm4[threadIdx.x] = __ldcg(&q.nrm[gc[threadIdx.x]]);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        const int rot0 = nrot;
+        if (r == 0) {  // norms anew: warp w takes column w
+          const int w = threadIdx.x >> 5;
+          double s = 0.0;
+          if (gc[w] < rc) {
+            const double* wc = sm + (int64_t)w * cst;
+#pragma unroll 4
+            for (int i = lane; i < mx; i += 32) s = fma(wc[i], wc[i], s);
+            s = wsum_d(s);
+            if (lane == 0) nrm4[w] = s;
+          }
+          __syncthreads();
+          process(2 * grp, 2 * grp + 1, gc[2 * grp + 1] < rc);
+          __syncthreads();
+        }
+        process(grp, 2 + grp, gc[grp] < rc && gc[2 + grp] < rc);
+        __syncthreads();
+        process(grp, 3 - grp, gc[grp] < rc && gc[3 - grp] < rc);
+        __syncthreads();
+        if (nrot != rot0 || r == 0) {
+          for (int l = 0; l < 4; ++l) {
+            if (gc[l] >= rc) continue;
+            double2* wd = reinterpret_cast<double2*>(W + (int64_t)gc[l] * ldx);
+            const double2* s2 = reinterpret_cast<const double2*>(sm + (int64_t)l * cst);
+            for (int i = threadIdx.x; i < (ldw >> 1); i += blockDim.x) __stcg(&wd[i], s2[i]);
+            if (ACCV) {
+              double2* vd = reinterpret_cast<double2*>(V + (int64_t)gc[l] * ldx);
+              for (int i = threadIdx.x; i < (ldv >> 1); i += blockDim.x) __stcg(&vd[i], s2[(ldw >> 1) + i]);
+            }
+          }
+          if (threadIdx.x < 4 && gc[threadIdx.x] < rc) __stcg(&q.nrm[gc[threadIdx.x]], nrm4[threadIdx.x]);
+        }
+      }
+      if (r == rounds - 1) {
+        __syncthreads();  // every thread has compared nrot with rot0
+        if (threadIdx.x == 0 && nrot) {
+          atomicAdd(&q.info[kiRot + sweep], nrot);
+          atomicMax(&q.info[kiCos + sweep], cosmax);
+          atomicMax(&q.info[kiTan + sweep], tanmax);
+          nrot = cosmax = tanmax = 0;
+        }
+      }
+      if (!bar.sync()) return;
+    }
+    const int rot = __ldcg(&q.info[kiRot + sweep]);
+    const float cm = __int_as_float(__ldcg(&q.info[kiCos + sweep]));
+    const float tm = __int_as_float(__ldcg(&q.info[kiTan + sweep]));
+    done = rot == 0 || cm * tm < 0.5f * tolf;
+  }
+  if (cta == 0 && threadIdx.x == 0) q.info[kiSweeps] = done ? max(sweep, 1) : 0;
+}
+
+// ---------------------------------------------------------------------------
+// FP32 sweeps that precede the FP64 ones (n ≥ kPreMin): the same tournament on
+// an FP32 copy of X with blocks of four columns (two cross barriers fewer per
+// column pair than blocks of two; FP32 arithmetic is 64 times as wide, so a
+// round is barrier and L2 latency either way).  One-sided rotations keep the
+// relative accuracy of graded columns in FP32 too, so X·V comes out with
+// |cos| ~ 1e-6 between all columns, small ones included.
+// ---------------------------------------------------------------------------
+template <int RJ>
+__global__ void __launch_bounds__(256) k_svd_sweeps32(SvdArgs a) {
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  const SvdProb& q = a.p[blockIdx.y];
+  const int rc = q.info[kiRank];
+  const bool two = a.second || rc < a.n;
+  const int mx = two ? rc : a.n;
+  const int nreal = (rc + 3) >> 2, NB = nreal + (nreal & 1);
+  const int active = NB >> 1, cta = blockIdx.x;
+  if (cta >= active || q.info[kiErr]) return;
+  float* W = q.W32;
+  float* V = q.V32;
+  const int ld = a.ld32;
+  const int ldw = (mx + 3) & ~3, ldv = (rc + 3) & ~3, cst = ldw + ldv;
+  float* sm = reinterpret_cast<float*>(sm_raw);  // 8 columns: W rows, then V rows
+  __shared__ float red[4][2][3];
+  __shared__ int dead, nrot, cosmax;
+  if (threadIdx.x == 0) dead = nrot = cosmax = 0;
+  __syncthreads();
+  GridBar<false> bar{reinterpret_cast<unsigned*>(q.info + kiBar + 3), 0u, (unsigned)active, q.info + kiErr, &dead};
+  const double* X = two ? q.X2 : q.X;
+  for (int j = cta; j < rc; j += active) {
+    for (int i = threadIdx.x; i < mx; i += blockDim.x)
+      __stcg(&W[i + (int64_t)j * ld], d2f(X[i + (int64_t)j * a.ldx]));
+    for (int i = threadIdx.x; i < rc; i += blockDim.x) __stcg(&V[i + (int64_t)j * ld], i == j ? 1.f : 0.f);
+  }
+  if (!bar.sync()) return;
+  const int grp = threadIdx.x >> 6, lt = threadIdx.x & 63, wip = (threadIdx.x >> 5) & 1, lane = threadIdx.x & 31;
+
+  auto process = [&](int x, int y, bool present) {
+    float* wx = sm + (int64_t)x * cst;
+    float* wy = sm + (int64_t)y * cst;
+    float u[RJ], v[RJ];
+    if (present) {
+      float na = 0.f, nb = 0.f, g = 0.f;
+#pragma unroll
+      for (int e = 0; e < RJ; ++e) {
+        const int i = lt + 64 * e;
+        u[e] = i < mx ? wx[i] : 0.f;
+        v[e] = i < mx ? wy[i] : 0.f;
+      }
+#pragma unroll
+      for (int e = 0; e < RJ; ++e) {
+        na = fmaf(u[e], u[e], na);
+        nb = fmaf(v[e], v[e], nb);
+        g = fmaf(u[e], v[e], g);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        na += __shfl_xor_sync(0xffffffffu, na, o);
+        nb += __shfl_xor_sync(0xffffffffu, nb, o);
+        g += __shfl_xor_sync(0xffffffffu, g, o);
+      }
+      if (lane == 0) {
+        red[grp][wip][0] = na;
+        red[grp][wip][1] = nb;
+        red[grp][wip][2] = g;
+      }
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(grp + 1) : "memory");
+    if (present) {
+      const float na = red[grp][0][0] + red[grp][1][0], nb = red[grp][0][1] + red[grp][1][1];
+      const float g = red[grp][0][2] + red[grp][1][2];
+      const float nn = fsqrt_ap(na) * fsqrt_ap(nb);
+      if (fabsf(g) > a.tol32 * nn) {
+        const float t = jacobi_tan(nb - na, 2.f * g);
+        const float cs = rsqrtf(fmaf(t, t, 1.f)), sn = cs * t;
+#pragma unroll
+        for (int e = 0; e < RJ; ++e) {
+          const int i = lt + 64 * e;
+          if (i < mx) {
+            wx[i] = cs * u[e] - sn * v[e];
+            wy[i] = sn * u[e] + cs * v[e];
+          }
+        }
+        float* vx = wx + ldw;
+        float* vy = wy + ldw;
+#pragma unroll
+        for (int e = 0; e < RJ; ++e) {
+          const int i = lt + 64 * e;
+          u[e] = i < rc ? vx[i] : 0.f;
+          v[e] = i < rc ? vy[i] : 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < RJ; ++e) {
+          const int i = lt + 64 * e;
+          if (i < rc) {
+            vx[i] = cs * u[e] - sn * v[e];
+            vy[i] = sn * u[e] + cs * v[e];
+          }
+        }
+        if (lt == 0) {
+          atomicAdd(&nrot, 1);
+          atomicMax(&cosmax, __float_as_int(nn > 0.f ? fminf(__fdividef(fabsf(g), nn), 1.f) : 1.f));
+        }
+      }
+    }
+    __syncthreads();  // columns change hands; red is free again
+  };
+
+  const int rounds = NB - 1;
+  bool done = rc < 2;
+  for (int sweep = 0; sweep < kPreSweeps && !done; ++sweep) {
+    for (int r = 0; r < rounds; ++r) {
+      int P, Q;
+      if (cta == 0) {
+        P = r;
+        Q = NB - 1;
+      } else {
+        P = (r + cta) % (NB - 1);
+        Q = (r - cta + (NB - 1)) % (NB - 1);
+      }
+      if (P > Q) {
+        const int t = P;
+        P = Q;
+        Q = t;
+      }
+      auto gcol = [&](int l) { return l < 4 ? 4 * P + l : 4 * Q + l - 4; };
+      for (int l = 0; l < 8; ++l) {
+        const int g = gcol(l);
+        if (g >= rc) continue;
+        const float* ws = W + (int64_t)g * ld;
+        const float* vs = V + (int64_t)g * ld;
+        const uint32_t dst = tc::su32(sm + (int64_t)l * cst);
+        for (int i = threadIdx.x; i < (ldw >> 2); i += blockDim.x)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(ws + 4 * i) : "memory");
+        for (int i = threadIdx.x; i < (ldv >> 2); i += blockDim.x)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4u * ldw + 16u * i), "l"(vs + 4 * i)
+                       : "memory");
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      if (r == 0) {  // pairs inside P (groups 0, 1) and inside Q (groups 2, 3)
+        for (int ir = 0; ir < 3; ++ir) {
+          int x, y;
+          if ((grp & 1) == 0) {
+            x = ir;
+            y = 3;
+          } else {
+            x = min((ir + 1) % 3, (ir + 2) % 3);
+            y = max((ir + 1) % 3, (ir + 2) % 3);
+          }
+          x += (grp >> 1) * 4;
+          y += (grp >> 1) * 4;
+          process(x, y, gcol(x) < rc && gcol(y) < rc);
+        }
+      }
+      for (int ir = 0; ir < 4; ++ir) {
+        const int y = 4 + ((grp + ir) & 3);
+        process(grp, y, gcol(grp) < rc && gcol(y) < rc);
+      }
+      for (int l = 0; l < 8; ++l) {
+        const int g = gcol(l);
+        if (g >= rc) continue;
+        float4* wd = reinterpret_cast<float4*>(W + (int64_t)g * ld);
+        float4* vd = reinterpret_cast<float4*>(V + (int64_t)g * ld);
+        const float4* s4 = reinterpret_cast<const float4*>(sm + (int64_t)l * cst);
+        for (int i = threadIdx.x; i < (ldw >> 2); i += blockDim.x) __stcg(&wd[i], s4[i]);
+        for (int i = threadIdx.x; i < (ldv >> 2); i += blockDim.x) __stcg(&vd[i], s4[(ldw >> 2) + i]);
+      }
+      if (r == rounds - 1 && threadIdx.x == 0 && nrot) {
+        atomicAdd(&q.info[kiRot32 + sweep], nrot);
+        atomicMax(&q.info[kiCos32 + sweep], cosmax);
+        nrot = 0;
+        cosmax = 0;
+      }
+      if (!bar.sync()) return;
+    }
+    done = __ldcg(&q.info[kiRot32 + sweep]) == 0 || __int_as_float(__ldcg(&q.info[kiCos32 + sweep])) < kPreCos;
+    if (done && cta == 0 && threadIdx.x == 0) q.info[kiPre] = sweep + 1;
+  }
+  // V in FP64
+  for (int j = cta; j < rc; j += active)
+    for (int i = threadIdx.x; i < rc; i += blockDim.x)
+      q.Vx[i + (int64_t)j * a.ldx] = f2d(__ldcg(&V[i + (int64_t)j * ld]));
+}
+
+// The same sweeps by one thread-block cluster (n ≤ 512; C = 1, 2, 4, 8 or 16
+// CTAs, at most 16 columns a block): its hardware barrier takes 0.24 µs where
+// the grid barrier takes 1.1, and with blocks this long a sweep has 2C − 1
+// exchanges through L2 instead of n/4.  One warp per column pair, B inner
+// rounds of B disjoint pairs with a CTA barrier each.  n = 324: 3.4 ms (grid
+// variant 3.75); n = 64: 0.98 ms for the whole decomposition (1.17).
+template <int RJ>
+__global__ void __launch_bounds__(512) k_svd_sweeps32_cl(SvdArgs a) {
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  const SvdProb& q = a.p[blockIdx.y];
+  const int rc = q.info[kiRank];
+  if (q.info[kiErr]) return;
+  const bool two = a.second || rc < a.n;
+  const int mx = two ? rc : a.n;
+  const int C = gridDim.x, cta = blockIdx.x, NB = 2 * C;
+  const int B = (rc + NB - 1) / NB;  // columns per block (the last blocks may be short or empty)
+  float* W = q.W32;
+  float* V = q.V32;
+  const int ld = a.ld32;
+  const int ldw = (mx + 3) & ~3, ldv = (rc + 3) & ~3, cst = ldw + ldv;
+  float* sm = reinterpret_cast<float*>(sm_raw);  // 2B columns: W rows, then V rows
+  __shared__ int nrot, cosmax;
+  if (threadIdx.x == 0) nrot = cosmax = 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double* X = two ? q.X2 : q.X;
+  for (int j = cta; j < rc; j += C) {
+    for (int i = threadIdx.x; i < mx; i += blockDim.x)
+      __stcg(&W[i + (int64_t)j * ld], d2f(X[i + (int64_t)j * a.ldx]));
+    for (int i = threadIdx.x; i < rc; i += blockDim.x) __stcg(&V[i + (int64_t)j * ld], i == j ? 1.f : 0.f);
+  }
+  GridBar<true> bar{nullptr, 0u, 0u, nullptr, nullptr};
+  bar.sync();
+
+  auto process = [&](int x, int y) {  // local columns, x before y in global order
+    float* wx = sm + (int64_t)x * cst;
+    float* wy = sm + (int64_t)y * cst;
+    float u[RJ], v[RJ];
+    float na = 0.f, nb = 0.f, g = 0.f;
+#pragma unroll
+    for (int e = 0; e < RJ; ++e) {
+      const int i = lane + 32 * e;
+      u[e] = i < mx ? wx[i] : 0.f;
+      v[e] = i < mx ? wy[i] : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < RJ; ++e) {
+      na = fmaf(u[e], u[e], na);
+      nb = fmaf(v[e], v[e], nb);
+      g = fmaf(u[e], v[e], g);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      na += __shfl_xor_sync(0xffffffffu, na, o);
+      nb += __shfl_xor_sync(0xffffffffu, nb, o);
+      g += __shfl_xor_sync(0xffffffffu, g, o);
+    }
+    const float nn = fsqrt_ap(na) * fsqrt_ap(nb);
+    if (!(fabsf(g) > a.tol32 * nn)) return;
+    const float t = jacobi_tan(nb - na, 2.f * g);
+    const float cs = rsqrtf(fmaf(t, t, 1.f)), sn = cs * t;
+#pragma unroll
+    for (int e = 0; e < RJ; ++e) {
+      const int i = lane + 32 * e;
+      if (i < mx) {
+        wx[i] = cs * u[e] - sn * v[e];
+        wy[i] = sn * u[e] + cs * v[e];
+      }
+    }
+    float* vx = wx + ldw;
+    float* vy = wy + ldw;
+#pragma unroll
+    for (int e = 0; e < RJ; ++e) {
+      const int i = lane + 32 * e;
+      u[e] = i < rc ? vx[i] : 0.f;
+      v[e] = i < rc ? vy[i] : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < RJ; ++e) {
+      const int i = lane + 32 * e;
+      if (i < rc) {
+        vx[i] = cs * u[e] - sn * v[e];
+        vy[i] = sn * u[e] + cs * v[e];
+      }
+    }
+    if (lane == 0) {
+      atomicAdd(&nrot, 1);
+      atomicMax(&cosmax, __float_as_int(nn > 0.f ? fminf(__fdividef(fabsf(g), nn), 1.f) : 1.f));
+    }
+  };
+
+  bool done = rc < 2;
+  for (int sweep = 0; sweep < kPreSweeps && !done; ++sweep) {
+    for (int r = 0; r < NB - 1; ++r) {
+      int P, Q;
+      if (cta == 0) {
+        P = r;
+        Q = NB - 1;
+      } else {
+        P = (r + cta) % (NB - 1);
+        Q = (r - cta + (NB - 1)) % (NB - 1);
+      }
+      if (P > Q) {
+        const int t = P;
+        P = Q;
+        Q = t;
+      }
+      auto gcol = [&](int l) { return l < B ? P * B + l : Q * B + l - B; };
+      for (int l = warp; l < 2 * B; l += 16) {  // one warp per column
+        const int g = gcol(l);
+        if (g >= rc) continue;
+        const float* ws = W + (int64_t)g * ld;
+        const float* vs = V + (int64_t)g * ld;
+        const uint32_t dst = tc::su32(sm + (int64_t)l * cst);
+        for (int i = lane; i < (ldw >> 2); i += 32)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(ws + 4 * i) : "memory");
+        for (int i = lane; i < (ldv >> 2); i += 32)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4u * ldw + 16u * i), "l"(vs + 4 * i)
+                       : "memory");
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      if (r == 0 && B > 1) {  // pairs inside P and inside Q: circle method over B (even: BE) columns
+        const int BE = B + (B & 1);
+        for (int ir = 0; ir < BE - 1; ++ir) {
+          for (int s = warp; s < BE; s += 16) {  // BE/2 slots for P, BE/2 for Q
+            const int k = s >= BE / 2 ? s - BE / 2 : s, off = s >= BE / 2 ? B : 0;
+            int x = k == 0 ? BE - 1 : (ir + k) % (BE - 1);
+            int y = k == 0 ? ir : (ir - k + (BE - 1)) % (BE - 1);
+            if (x > y) {
+              const int t = x;
+              x = y;
+              y = t;
+            }
+            if (y < B && gcol(off + y) < rc) process(off + x, off + y);
+          }
+          __syncthreads();
+        }
+      }
+      for (int ir = 0; ir < B; ++ir) {
+        for (int s = warp; s < B; s += 16) {
+          const int y = B + (s + ir < B ? s + ir : s + ir - B);
+          if (gcol(s) < rc && gcol(y) < rc) process(s, y);
+        }
+        __syncthreads();
+      }
+      for (int l = warp; l < 2 * B; l += 16) {
+        const int g = gcol(l);
+        if (g >= rc) continue;
+        float4* wd = reinterpret_cast<float4*>(W + (int64_t)g * ld);
+        float4* vd = reinterpret_cast<float4*>(V + (int64_t)g * ld);
+        const float4* s4 = reinterpret_cast<const float4*>(sm + (int64_t)l * cst);
+        for (int i = lane; i < (ldw >> 2); i += 32) __stcg(&wd[i], s4[i]);
+        for (int i = lane; i < (ldv >> 2); i += 32) __stcg(&vd[i], s4[(ldw >> 2) + i]);
+      }
+      if (r == NB - 2 && threadIdx.x == 0 && nrot) {
+        atomicAdd(&q.info[kiRot32 + sweep], nrot);
+        atomicMax(&q.info[kiCos32 + sweep], cosmax);
+        nrot = 0;
+        cosmax = 0;
+      }
+      bar.sync();
+    }
+    done = __ldcg(&q.info[kiRot32 + sweep]) == 0 || __int_as_float(__ldcg(&q.info[kiCos32 + sweep])) < kPreCos;
+    if (done && cta == 0 && threadIdx.x == 0) q.info[kiPre] = sweep + 1;
+  }
+  for (int j = cta; j < rc; j += C)  // V in FP64
+    for (int i = threadIdx.x; i < rc; i += blockDim.x)
+      q.Vx[i + (int64_t)j * a.ldx] = f2d(__ldcg(&V[i + (int64_t)j * ld]));
+}
+
+// F = VᵀV − I (r×r) → the factor of V ← V·(I − T): T_qp = F_qp below the
+// diagonal, F_pp/2 on it.  A column is cleared of the later (smaller) ones
+// only: the small columns of V carry their relative accuracy in tiny entries,
+// which a symmetric correction would fill with rounding of the large ones.
+__global__ void k_svd_tri(double* __restrict__ F, int r) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < r * r; e += gridDim.x * blockDim.x) {
+    const int i = e % r, j = e / r;
+    const double f = F[e];
+    F[e] = i > j ? f : (i == j ? 0.5 * (f - 1.0) : 0.0);
+  }
+}
+
+// σ_j = ‖W_j‖ (unsorted, still scaled); one warp per column
+__global__ void k_svd_norms(SvdArgs a) {
+  const SvdProb& q = a.p[blockIdx.y];
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int rc = q.info[kiRank];
+  if (j >= a.n) return;
+  double s = 0.0;
+  if (j < rc) {
+    const bool two = a.second || rc < a.n;
+    const int mx = two ? rc : a.n;
+    const double* w = (q.W ? q.W : (two ? q.X2 : q.X)) + (int64_t)j * a.ldx;
+    for (int i = lane; i < mx; i += 32) s = fma(w[i], w[i], s);
+    s = sqrt(wsum_d(s));
+  }
+  if (lane == 0) q.sv[j] = s;
+}
+
+// One CTA per column j: its rank among the σ (descending, ties by index; the
+// cut columns follow) and the column in its sorted place:
+//   U[:, rank] = P₂·Wn_j (to be multiplied by Q), V[:, rank] = Vx_j (by P·Q₂),
+//   or V[:, rank] = P·Wn_j where the second QR was skipped (symmetric, r = n);
+//   symmetric: only V is formed, from P₂·Wn_j.
+template <bool SYM>
+__global__ void __launch_bounds__(128) k_svd_place(SvdArgs a) {
+  const SvdProb& q = a.p[blockIdx.y];
+  const int j = blockIdx.x, m = a.m, n = a.n;
+  const int rc = q.info[kiRank];
+  const bool two = a.second || rc < n;
+  const double sj = q.sv[j];
+  int rk = j;
+  if (j < rc) {
+    int cnt = 0;
+    for (int i = threadIdx.x; i < rc; i += blockDim.x) {
+      const double si = q.sv[i];
+      cnt += (si > sj || (si == sj && i < j)) ? 1 : 0;
+    }
+    __shared__ int part[4];
+    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = cnt;
+    __syncthreads();
+    rk = part[0] + part[1] + part[2] + part[3];
+  }
+  double* u = SYM ? nullptr : q.U + (int64_t)rk * m;
+  double* v = q.V + (int64_t)rk * n;
+  if (q.info[kiBad]) {
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    if (!SYM)
+      for (int i = threadIdx.x; i < m; i += blockDim.x) u[i] = nan;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = nan;
+    if (threadIdx.x == 0) q.S[rk] = nan;
+    return;
+  }
+  if (threadIdx.x == 0) q.S[rk] = scalbn(sj, q.info[kiExp]);
+  if (j >= rc) {
+    if (!SYM)
+      for (int i = threadIdx.x; i < m; i += blockDim.x) u[i] = i == j ? 1.0 : 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = i == j ? 1.0 : 0.0;
+    return;
+  }
+  const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
+  if (SYM && !two) {
+    const double* w = (q.W ? q.W : q.X) + (int64_t)j * a.ldx;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) v[q.perm[i]] = w[i] * inv;
+    return;
+  }
+  const double* w = (q.W ? q.W : q.X2) + (int64_t)j * a.ldx;
+  double* o = SYM ? v : u;
+  const int mo = SYM ? n : m;
+  for (int i = rc + threadIdx.x; i < mo; i += blockDim.x) o[i] = 0.0;
+  for (int i = threadIdx.x; i < rc; i += blockDim.x) o[q.perm2[i]] = w[i] * inv;
+  if (!SYM) {
+    const double* x = q.Vx + (int64_t)j * a.ldx;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = i < rc ? x[i] : 0.0;
+  }
+}
+
+// B ← Q·B, Q = H_0·H_1···H_{r−1}: one warp per column of B, which it holds in
+// registers; the reflectors are read through L1/L2, the next one prefetched
+// while the current one is applied.  STAGE 0: Q of A on U (symmetric: on V);
+// STAGE 1: Q₂ on V, rows then permuted by P.
+template <int R, bool SYM, int STAGE>
+__global__ void __launch_bounds__(128) k_svd_apply_q(SvdArgs a) {
+  const SvdProb& q = a.p[blockIdx.y];
+  const int rc = q.info[kiRank], n = a.n;
+  if (q.info[kiErr] || q.info[kiBad]) return;
+  if (SYM && rc == n) return;  // the eigenvectors are in place
+  const int rows = STAGE == 0 ? a.m : n;
+  const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (col >= n) return;
+  const double* H = STAGE == 0 ? q.H : q.H2;
+  const double* hinv = STAGE == 0 ? q.hinv : q.hinv2;
+  double* B = ((STAGE == 0 && !SYM) ? q.U : q.V) + (int64_t)col * rows;
+  double c[R], x[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int row = lane + 32 * i;
+    c[i] = row < rows ? B[row] : 0.0;
+    x[i] = (row < rows && rc > 0) ? H[row + (int64_t)(rc - 1) * rows] : 0.0;
+  }
+  for (int k = rc - 1; k >= 0; --k) {
+    double d = 0.0;
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if (32 * i < rows && 32 * i + 31 >= k) d = fma(x[i], c[i], d);
+    double xn[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int row = lane + 32 * i;
+      xn[i] = (k > 0 && 32 * i + 31 >= k - 1 && row < rows) ? H[row + (int64_t)(k - 1) * rows] : 0.0;
+    }
+    d = wsum_d(d) * hinv[k];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (32 * i < rows && 32 * i + 31 >= k) c[i] = fma(-d, x[i], c[i]);
+      x[i] = xn[i];
+    }
+  }
+  __syncwarp();  // every lane has read its rows of the column
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int row = lane + 32 * i;
+    if (row < rows) B[STAGE == 1 ? q.perm[row] : row] = c[i];
+  }
+}
+
+// Left vectors of a symmetric A from its right ones: U_j = sign(λ_j)·V_j with
+// λ_j = v_j·(A·v_j).  Where σ_j is shared (to 1e-8) and above 1e-8·σ_1, V only
+// spans the singular subspace (a ±λ pair may come out mixed) and U follows
+// from A·V: a pair takes the 2×2 block h = VᵀAV/σ of its subspace, which is a
+// reflection [[c, s], [s, −c]] for ±λ (or ±I), normalised so that U stays
+// orthonormal to rounding; larger groups take A·v/σ.  One CTA per column.
+__global__ void __launch_bounds__(128) k_svd_sym_left(int n, const double* __restrict__ V,
+                                                      const double* __restrict__ AV, const double* __restrict__ S,
+                                                      double* __restrict__ U) {
+  const int j = blockIdx.x;
+  __shared__ double red[4][4];
+  const double sj = S[j];
+  auto near = [&](int x, int y) { return fabs(S[x] - S[y]) <= 1e-8 * S[y]; };
+  int lo = j, hi = j;
+  if (sj > 1e-8 * S[0]) {
+    while (lo > 0 && j - lo < 2 && near(lo - 1, lo)) --lo;
+    while (hi + 1 < n && hi - j < 2 && near(hi, hi + 1)) ++hi;
+  }
+  const int o = hi - lo == 1 ? (j == lo ? hi : lo) : j;  // partner of a pair
+  double h[4] = {0.0, 0.0, 0.0, 0.0};  // v_j·Av_j, v_o·Av_o, v_o·Av_j, v_j·Av_o
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double vj = V[i + (int64_t)j * n], wj = AV[i + (int64_t)j * n];
+    h[0] = fma(vj, wj, h[0]);
+    if (o != j) {
+      const double vo = V[i + (int64_t)o * n], wo = AV[i + (int64_t)o * n];
+      h[1] = fma(vo, wo, h[1]);
+      h[2] = fma(vo, wj, h[2]);
+      h[3] = fma(vj, wo, h[3]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const double t = wsum_d(h[e]);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][e] = t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    h[e] = red[0][e] + red[1][e] + red[2][e] + red[3][e];
+    if (sj > 0.0) h[e] /= sj;
+  }
+  double cj = h[0] < 0.0 ? -1.0 : 1.0, co = 0.0;
+  const bool from_av = hi - lo > 1;
+  const double b = 0.5 * (h[2] + h[3]);  // the same bits for both columns of the pair
+  if (o != j && (h[0] * h[1] < 0.0 || fabs(b) > 0.5)) {  // a ±λ pair: U_j = c·V_j + s·V_o
+    const double c0 = 0.5 * (h[0] - h[1]), r = 1.0 / sqrt(c0 * c0 + b * b);
+    cj = c0 * r;
+    co = b * r;
+  }
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    double u;
+    if (from_av)
+      u = AV[i + (int64_t)j * n] / sj;
+    else
+      u = co == 0.0 ? cj * V[i + (int64_t)j * n] : cj * V[i + (int64_t)j * n] + co * V[i + (int64_t)o * n];
+    U[i + (int64_t)j * n] = u;
+  }
+}
+
+template <typename F>
+void launch_grid(tnad_ctx* c, F* f, bool cluster, int G, int np, int threads, size_t smem, SvdArgs& a) {
+  cudaLaunchConfig_t cf = {};
+  cf.gridDim = dim3((unsigned)G, (unsigned)np);
+  cf.blockDim = dim3((unsigned)threads);
+  cf.dynamicSmemBytes = smem;
+  cf.stream = c->stream;
+  cudaLaunchAttribute at[1];
+  if (cluster) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)G;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeCooperative;  // the CTAs wait on one another: all resident or none
+    at[0].val.cooperative = 1;
+  }
+  cf.attrs = at;
+  cf.numAttrs = 1;
+  TNAD_CK(cudaLaunchKernelEx(&cf, f, a));
+  count_launch(c);
+}
+
+template <int R, int STAGE>
+void launch_qrcp(tnad_ctx* c, int np, int cols, SvdArgs& a) {
+  // up to 64 columns fit a cluster of 8 CTAs of 8 warps; beyond, as many CTAs
+  // as SMs (both problems together resident)
+  if (cols <= 64) {
+    const int G = std::min(8, cols);
+    launch_grid(c, k_qrcp<R, true, STAGE>, true, G, np, 32 * ((cols + G - 1) / G), 0, a);
+  } else {
+    const int G = std::min(cols, c->sm_count / np);
+    launch_grid(c, k_qrcp<R, false, STAGE>, false, G, np, 32 * ((cols + G - 1) / G), 0, a);
+  }
+}
+
+template <int RJ, bool ACCV>
+void launch_sweeps(tnad_ctx* c, int np, SvdArgs& a) {
+  const int nreal = (a.n + 1) / 2, G = std::max(1, (nreal + (nreal & 1)) / 2);
+  const size_t smem = (size_t)4 * ((a.n + 1) & ~1) * (ACCV ? 2 : 1) * sizeof(double);
+  if (G <= 8) {
+    launch_grid(c, k_svd_sweeps<RJ, ACCV, true>, true, G, np, 128, smem, a);
+  } else {
+    static std::atomic<bool> attr{false};
+    if (!attr) {
+      TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps<RJ, ACCV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   4 * kMaxSvdRows * 2 * 8));
+      attr = true;
+    }
+    launch_grid(c, k_svd_sweeps<RJ, ACCV, false>, false, G, np, 128, smem, a);
+  }
+}
+
+// FP32 sweeps, then V orthogonal to FP64 rounding (two first-order triangular
+// corrections: 1e-6 → 1e-12 → 1e-24) and W = X·V, all in DFMA products: the
+// tensor-core ones are accurate to the row and column scales only, not to the
+// small columns of graded operands.
+template <int RJ>
+void pre_sweeps(tnad_ctx* c, int np, SvdArgs& a, int* info_host) {
+  static std::atomic<bool> attr{false};
+  if constexpr (RJ <= 8) {  // n ≤ 512
+    const int C = a.n <= 32 ? 1 : a.n <= 64 ? 2 : a.n <= 128 ? 4 : a.n <= 256 ? 8 : 16;
+    const int B = (a.n + 2 * C - 1) / (2 * C);
+    const size_t smem = (size_t)2 * B * 2 * a.ld32 * sizeof(float);
+    if (!attr) {
+      TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps32_cl<2 * RJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   2 * 16 * 2 * 512 * 4));
+      TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps32_cl<2 * RJ>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      attr = true;
+    }
+    launch_grid(c, k_svd_sweeps32_cl<2 * RJ>, true, C, np, 512, smem, a);
+  } else {
+    const int nreal = (a.n + 3) / 4, G = std::max(1, (nreal + (nreal & 1)) / 2);
+    const size_t smem = (size_t)8 * 2 * a.ld32 * sizeof(float);
+    if (!attr) {
+      TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps32<RJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   8 * 2 * kMaxSvdRows * 4));
+      attr = true;
+    }
+    launch_grid(c, k_svd_sweeps32<RJ>, false, G, np, 256, smem, a);
+  }
+  for (int p = 0; p < np; ++p)
+    TNAD_CK(cudaMemcpyAsync(info_host + p * kiBar, a.p[p].info, sizeof(int) * kiBar, cudaMemcpyDeviceToHost, c->stream));
+  TNAD_CK(cudaStreamSynchronize(c->stream));
+  for (int p = 0; p < np; ++p) {
+    SvdProb& q = a.p[p];
+    const int r = info_host[p * kiBar + kiRank];
+    const bool two = a.second || r < a.n;
+    const int mx = two ? r : a.n;
+    if (r < 2 || info_host[p * kiBar + kiErr]) continue;  // (q.W stays null: nothing to hand over)
+    WsScope scope(c);
+    double* F = ws_d(c, (int64_t)r * r);
+    double* V2 = ws_d(c, (int64_t)a.ldx * r);
+    double *from = q.Vx, *to = V2;
+    for (int it = 0; it < 2; ++it) {
+      gemm_f64(c, 'T', 'N', r, r, r, 1.0, from, a.ldx, from, a.ldx, 0.0, F, r);
+      k_svd_tri<<<(unsigned)std::min((r * r + 255) / 256, 4096), 256, 0, c->stream>>>(F, r);
+      count_launch(c);
+      copy_d2d(c, to, from, (int64_t)a.ldx * (r - 1) + r);
+      gemm_f64(c, 'N', 'N', r, r, r, -1.0, from, a.ldx, F, r, 1.0, to, a.ldx);
+      std::swap(from, to);
+    }
+    q.W = q.Wbuf;
+    gemm_f64(c, 'N', 'N', mx, r, r, 1.0, two ? q.X2 : q.X, a.ldx, q.Vx, a.ldx, 0.0, q.W, a.ldx);
+    check_launch(c, "svd_pre_sweeps");
+  }
+}
+
+template <int R>
+void svd_qrj_r(tnad_ctx* c, int np, bool symmetric, SvdArgs& a, int* info_host) {
+  launch_qrcp<R, 0>(c, np, a.n, a);
+  launch_qrcp<R, 1>(c, np, a.n, a);
+  if (a.n >= kPreMin) pre_sweeps<R / 2>(c, np, a, info_host);
+  if (symmetric)
+    launch_sweeps<R / 2, false>(c, np, a);
+  else
+    launch_sweeps<R / 2, true>(c, np, a);
+  const dim3 gw((unsigned)((a.n + 3) / 4), (unsigned)np), gc((unsigned)a.n, (unsigned)np);
+  k_svd_norms<<<gw, 128, 0, c->stream>>>(a);
+  if (symmetric) {
+    k_svd_place<true><<<gc, 128, 0, c->stream>>>(a);
+    k_svd_apply_q<R, true, 0><<<gw, 128, 0, c->stream>>>(a);
+    count_launch(c, 3);
+  } else {
+    k_svd_place<false><<<gc, 128, 0, c->stream>>>(a);
+    k_svd_apply_q<R, false, 0><<<gw, 128, 0, c->stream>>>(a);
+    k_svd_apply_q<R, false, 1><<<gw, 128, 0, c->stream>>>(a);
+    count_launch(c, 4);
+  }
+  check_launch(c, "svd_qrj");
+}
+
+}  // namespace
+
+bool svd_qrj_fits(int64_t m, int64_t n) { return m >= n && n >= 2 && m <= kMaxSvdRows; }
+
+void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, double* const* U, double* const* S,
+             double* const* V, bool symmetric) {
+  TNAD_REQUIRE(svd_qrj_fits(m, n) && (np == 1 || np == 2), TNAD_ERR_SHAPE, "svd_qrj: needs 1024 >= m >= n >= 2");
+  if (np == 2 && n > 8 * (int64_t)(c->sm_count / 2)) {  // a CTA of the QR holds at most 8 columns
+    svd_qrj(c, 1, A, m, n, U, S, V, symmetric);
+    svd_qrj(c, 1, A + 1, m, n, U + 1, S + 1, V + 1, symmetric);
+    return;
+  }
+  TNAD_REQUIRE(n <= 8 * (int64_t)(c->sm_count / np), TNAD_ERR_SHAPE, "svd_qrj: too many columns for this GPU");
+  WsScope scope(c);
+  SvdArgs a = {};
+  a.m = (int)m;
+  a.n = (int)n;
+  a.ldx = (int)((n + 1) & ~(int64_t)1);
+  a.ldc = (int)m;
+  a.ld32 = (int)((n + 3) & ~(int64_t)3);
+  a.second = symmetric ? 0 : 1;
+  a.trunc = 0.5f * (float)DBL_EPSILON;
+  a.tol = 2.0 * std::sqrt((double)std::max<int64_t>(m, 16)) * DBL_EPSILON;
+  a.tol32 = 4.0f * std::sqrt((float)m) * FLT_EPSILON;
+  a.max_sweeps = kSvdSweeps;
+  if (c->fault_once == kFaultJacobiCap) {  // failure-path test: one sweep only
+    a.max_sweeps = 1;
+    c->fault_once = kFaultNone;
+  }
+  const int64_t G = c->sm_count;
+  int* info = (int*)c->ws.alloc(sizeof(int) * 2 * kiCount);
+  for (int p = 0; p < np; ++p) {
+    SvdProb& q = a.p[p];
+    q.A = A[p];
+    q.X = ws_d(c, (int64_t)a.ldx * n);
+    q.X2 = ws_d(c, (int64_t)a.ldx * n);
+    const bool pre = n >= kPreMin;
+    q.Vx = symmetric && !pre ? nullptr : ws_d(c, (int64_t)a.ldx * n);
+    q.Wbuf = pre ? ws_d(c, (int64_t)a.ldx * n) : nullptr;
+    q.W32 = pre ? ws_f(c, (int64_t)a.ld32 * n) : nullptr;
+    q.V32 = pre ? ws_f(c, (int64_t)a.ld32 * n) : nullptr;
+    q.H = ws_d(c, m * n);
+    q.H2 = ws_d(c, n * n);
+    q.hinv = ws_d(c, 2 * n);
+    q.hinv2 = q.hinv + n;
+    q.perm = (int*)c->ws.alloc(sizeof(int) * 2 * n);
+    q.perm2 = q.perm + n;
+    q.cand = ws_d(c, 2 * G * a.ldc);
+    q.key = (unsigned long long*)ws_d(c, 3 * G);
+    q.nrm = ws_d(c, n);
+    q.sv = ws_d(c, n);
+    q.U = U[p];
+    q.S = S[p];
+    q.V = V[p];
+    q.info = info + p * kiCount;
+  }
+  TNAD_CK(cudaMemsetAsync(info, 0, sizeof(int) * 2 * kiCount, c->stream));
+  const double nn = (double)n;
+  int h[2 * kiBar];
+  {
+    KernelTimer kt(c, "svd_qrj", np * 9.0 * nn * nn * nn, 8);
+    if (m <= 64)
+      svd_qrj_r<2>(c, np, symmetric, a, h);
+    else if (m <= 128)
+      svd_qrj_r<4>(c, np, symmetric, a, h);
+    else if (m <= 256)
+      svd_qrj_r<8>(c, np, symmetric, a, h);
+    else if (m <= 512)
+      svd_qrj_r<16>(c, np, symmetric, a, h);
+    else
+      svd_qrj_r<32>(c, np, symmetric, a, h);
+  }
+  if (symmetric) {
+    for (int p = 0; p < np; ++p) {
+      WsScope inner(c);
+      double* AV = ws_d(c, n * n);
+      gemm(c, TNAD_PREC_FP64, 'N', 'N', n, n, n, 1.0, A[p], n, V[p], n, 0.0, AV, n);
+      k_svd_sym_left<<<(unsigned)n, 128, 0, c->stream>>>((int)n, V[p], AV, S[p], U[p]);
+      count_launch(c);
+      check_launch(c, "svd_sym_left");
+    }
+  }
+  for (int p = 0; p < np; ++p)
+    TNAD_CK(cudaMemcpyAsync(h + p * kiBar, a.p[p].info, sizeof(int) * kiBar, cudaMemcpyDeviceToHost, c->stream));
+  TNAD_CK(cudaStreamSynchronize(c->stream));
+  for (int p = 0; p < np; ++p) {
+    TNAD_REQUIRE(h[p * kiBar + kiErr] == 0, TNAD_ERR_TIMEOUT, "svd_qrj: a bounded barrier wait expired");
+    TNAD_REQUIRE(h[p * kiBar + kiSweeps] > 0, TNAD_ERR_NOT_CONVERGED, "svd_qrj: no convergence within the sweep cap");
+    if (std::getenv("TNAD_TRACE"))
+      std::fprintf(stderr, "[tnad trace] svd_qrj n=%lld rank %d sweeps %d (FP32 %d)\n", (long long)n,
+                   h[p * kiBar + kiRank], h[p * kiBar + kiSweeps], h[p * kiBar + kiPre]);
+  }
+}
+
+}  // namespace tnad

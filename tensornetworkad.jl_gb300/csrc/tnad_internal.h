@@ -248,6 +248,14 @@ Ten contract_shape(const Ten& A, const char* la, const Ten& B, const char* lb, c
 // √s of them is differentiated, as in TRG; 0 gives LAPACK-level accuracy).
 void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, double* S,
                 double* V, bool symmetric, int rel_sweeps = 20);
+// SVD to LAPACK-level accuracy (ε·‖A‖ on every triplet) of np (1 or 2) matrices
+// of the same shape m×n (svd_qrj_fits: 1024 ≥ m ≥ n ≥ 2): rank-revealing QR,
+// then Jacobi on the triangular factor, each one launch (svd_qr.cu).  Values
+// below the rounding of A come back as 0, their vectors as an orthonormal
+// completion.  symmetric: U = V·sign(λ) (±λ pairs: from A·V).
+bool svd_qrj_fits(int64_t m, int64_t n);
+void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, double* const* U, double* const* S,
+             double* const* V, bool symmetric);
 // Refines X (n×n, nearly orthonormal approximate eigenvectors of the symmetric
 // A, n ≤ 2048) to FP64 accuracy by matrix products; lam gets the eigenvalues
 // (column order of X).  fro2: ‖A‖²_F on the device.  false: no convergence

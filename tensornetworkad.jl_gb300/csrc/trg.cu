@@ -83,17 +83,20 @@ __global__ void k_maxnorm_bwd(int64_t n, const double* __restrict__ dan, double 
   }
 }
 
-static void svd_any(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, double* S, double* V) {
-  // thin SVD for any shape; U m×ns, V n×ns, ns = min(m,n)
-  if (m >= n) {
-    svd_jacobi(c, A, m, n, U, S, V, false);
-  } else {
+// thin SVD for any shape; U m×ns, V n×ns, ns = min(m,n).  lapack: accurate to
+// ε·‖A‖ (svd_qrj) instead of relative to every singular value
+static void svd_any(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, double* S, double* V, bool lapack) {
+  if (m < n) {
     WsScope scope(c);
     double* At = ws_d(c, m * n);
     Ten t = make_ten(const_cast<double*>(A), {m, n});
     int perm[2] = {1, 0};
     permute(c, t, perm, At);
-    svd_jacobi(c, At, n, m, V, S, U, false);  // Aᵀ = V S Uᵀ
+    svd_any(c, At, n, m, V, S, U, lapack);  // Aᵀ = V S Uᵀ
+  } else if (lapack && svd_qrj_fits(m, n)) {
+    svd_qrj(c, 1, &A, m, n, &U, &S, &V, false);
+  } else {
+    svd_jacobi(c, A, m, n, U, S, V, false);
   }
 }
 
@@ -111,7 +114,7 @@ static void svd_back_any(tnad_ctx* c, const double* U, const double* S, const do
   }
 }
 
-void trg_svd_fwd(tnad_ctx* c, const double* t, const int64_t dd[4], int chi, double tol, TrgSvd& s, DevPool* pool) {
+static void trg_svd_alloc(const int64_t dd[4], TrgSvd& s, DevPool* pool) {
   s.m = dd[0] * dd[1];
   s.n = dd[2] * dd[3];
   s.ns = std::min(s.m, s.n);
@@ -119,10 +122,10 @@ void trg_svd_fwd(tnad_ctx* c, const double* t, const int64_t dd[4], int chi, dou
   s.U = pool->d(s.m * s.ns);
   s.S = pool->d(s.ns);
   s.V = pool->d(s.n * s.ns);
-  svd_any(c, t, s.m, s.n, s.U, s.S, s.V);
-  std::vector<double> hs(s.ns);
-  TNAD_CK(cudaMemcpyAsync(hs.data(), s.S, s.ns * 8, cudaMemcpyDeviceToHost, c->stream));
-  TNAD_CK(cudaStreamSynchronize(c->stream));
+}
+
+// bond dimension, floor and the split itself; hs: the singular values on the host
+static void trg_svd_finish(tnad_ctx* c, int chi, double tol, std::vector<double>& hs, TrgSvd& s, DevPool* pool) {
   int64_t cnt = 0;
   for (double x : hs) cnt += (x > tol) ? 1 : 0;
   s.k = std::min<int64_t>(std::min<int64_t>(cnt + 1, chi), s.ns);
@@ -144,6 +147,38 @@ void trg_svd_fwd(tnad_ctx* c, const double* t, const int64_t dd[4], int chi, dou
   k_trg_split<<<nb(s.m * s.k + s.k * s.n), 256, 0, c->stream>>>(s.U, s.S, s.V, s.m, s.n, s.k, s.u, s.v);
   count_launch(c);
   check_launch(c, "trg_split");
+}
+
+void trg_svd_fwd(tnad_ctx* c, const double* t, const int64_t dd[4], int chi, double tol, TrgSvd& s, DevPool* pool) {
+  trg_svd_alloc(dd, s, pool);
+  svd_any(c, t, s.m, s.n, s.U, s.S, s.V, false);
+  std::vector<double> hs(s.ns);
+  TNAD_CK(cudaMemcpyAsync(hs.data(), s.S, s.ns * 8, cudaMemcpyDeviceToHost, c->stream));
+  TNAD_CK(cudaStreamSynchronize(c->stream));
+  trg_svd_finish(c, chi, tol, hs, s, pool);
+}
+
+// Both splits of a TRG step.  They are independent and of the same shape (the
+// two diagonals of one tensor), so one batch of svd_qrj decomposes both: its
+// sweeps are latency-bound and a 400×400 split alone leaves half of the SMs idle.
+static void trg_svd_pair(tnad_ctx* c, const double* t1, const int64_t d1[4], const double* t2, const int64_t d2[4],
+                         int chi, double tol, TrgSvd& s1, TrgSvd& s2, DevPool* pool) {
+  trg_svd_alloc(d1, s1, pool);
+  trg_svd_alloc(d2, s2, pool);
+  if (s1.m == s2.m && s1.n == s2.n && svd_qrj_fits(s1.m, s1.n)) {
+    const double* A[2] = {t1, t2};
+    double *U[2] = {s1.U, s2.U}, *S[2] = {s1.S, s2.S}, *V[2] = {s1.V, s2.V};
+    svd_qrj(c, 2, A, s1.m, s1.n, U, S, V, false);
+  } else {
+    svd_any(c, t1, s1.m, s1.n, s1.U, s1.S, s1.V, true);
+    svd_any(c, t2, s2.m, s2.n, s2.U, s2.S, s2.V, true);
+  }
+  std::vector<double> h1(s1.ns), h2(s2.ns);
+  TNAD_CK(cudaMemcpyAsync(h1.data(), s1.S, s1.ns * 8, cudaMemcpyDeviceToHost, c->stream));
+  TNAD_CK(cudaMemcpyAsync(h2.data(), s2.S, s2.ns * 8, cudaMemcpyDeviceToHost, c->stream));
+  TNAD_CK(cudaStreamSynchronize(c->stream));
+  trg_svd_finish(c, chi, tol, h1, s1, pool);
+  trg_svd_finish(c, chi, tol, h2, s2, pool);
 }
 
 void trg_svd_bwd(tnad_ctx* c, const TrgSvd& s, const double* du, const double* dv, double* dt) {
@@ -191,8 +226,7 @@ void trg_fwd(tnad_ctx* c, TrgTape& tp, const double* a0, int d, int chi, int nit
     permute(c, at, p2, ldru);
     int64_t d1[4] = {dims[2], dims[1], dims[0], dims[3]};
     int64_t d2[4] = {dims[3], dims[2], dims[1], dims[0]};
-    trg_svd_fwd(c, drul, d1, chi, tol, I.s1, &P);  // dr, ul
-    trg_svd_fwd(c, ldru, d2, chi, tol, I.s2, &P);  // ld, ru
+    trg_svd_pair(c, drul, d1, ldru, d2, chi, tol, I.s1, I.s2, &P);  // dr, ul and ld, ru
     // a = ein"npu,por,dom,lmn -> urdl"(dr, ld, ul, ru)   (:25)
     Ten dr = make_ten(I.s1.u, {d1[0], d1[1], I.s1.k});
     Ten ul = make_ten(I.s1.v, {I.s1.k, d1[2], d1[3]});
