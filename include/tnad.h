@@ -161,9 +161,10 @@ int tnad_svd(tnad_ctx* ctx, const double* A, int m, int n, double* U, double* S,
    corner cpmat of src/ctmrg.jl:134-136, decomposed there by LinearAlgebra.svd),
    through its eigendecomposition: S = |λ| descending, V the eigenvectors,
    U = V·sign(λ).  For n ≥ 256 FP32 Jacobi sweeps are polished to FP64 accuracy
-   by a refinement made of matrix products (FP64 Jacobi sweeps where that does
-   not converge); prec = TNAD_PREC_FP64 runs those products as DFMA tiles,
-   TNAD_PREC_FP64_TC on the tensor cores (TNAD_ERR_STATE without tcgen05).
+   by a refinement made of matrix products (FP64 Jacobi on a QR factor where
+   that does not converge); prec = TNAD_PREC_FP64 runs the products that the
+   result is taken from as DFMA tiles, TNAD_PREC_FP64_TC on the tensor cores
+   (TNAD_ERR_STATE without tcgen05).
    Host pointers. */
 int tnad_svd_sym(tnad_ctx* ctx, int prec, const double* A, int n, double* U, double* S, double* V);
 /* Diagnostics of the symmetric SVDs run on this context (no reference

@@ -21,8 +21,11 @@
 //          eigenvalues are solved once the error has dropped below them
 //   E_ij = (S_ij + λ_j R_ij)/(λ_j − λ_i) between groups, R_ij/2 inside one
 //          (and on the diagonal): X ← X·(I + E), then X ← X·(3I − XᵀX)/2
-// until max|S_ij|/‖A‖_F ≤ 1e-10 and max|R_ij| ≤ 1e-8 with no group to solve
-// (that update and its re-orthogonalisation are the last), then λ_j = x_jᵀAx_j.
+// until max|S_ij|/‖A‖_F ≤ 1e-10 and max|R_ij| ≤ 1e-8 with no group to solve; the
+// plain path then measures S and G once more by DFMA products and takes the last
+// correction and λ_j = S_jj/G_jj from those, its iterations before that run on
+// the tensor cores (D=4, χ=64 plain energy and gradient, 6 steps: 724 → 250 ms,
+// gradient error against 64 bits 1.4e-14 → 5e-15).
 // A group larger than kMaxGroup, or no convergence within kMaxIt iterations,
 // returns false and the caller polishes with FP64 Jacobi sweeps instead (graded
 // spectra, whose small eigenvalues FP32 cannot separate).
@@ -32,6 +35,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 
 #include "tnad_internal.h"
 
@@ -98,18 +102,24 @@ __global__ void k_ref_lam(const double* __restrict__ S, const double* __restrict
   if (j < n) lam[j] = S[j + (int64_t)j * n] / G[j + (int64_t)j * n];
 }
 
-// pos_j = #{i : |λ_i| > |λ_j| or (= and i < j)} (descending |λ|), perm[pos_j] = j
+// pos_j = #{i : |λ_i| > |λ_j| or (= and i < j)} (descending |λ|), perm[pos_j] = j;
+// one warp per column (one thread per column took 157 µs at n = 1024: n dependent
+// loads on four SMs).  Non-negative doubles compare as their bit patterns, off
+// the FP64 pipe.
 __global__ void k_ref_rank(const double* __restrict__ absl, int n, int* __restrict__ pos, int* __restrict__ perm) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (j >= n) return;
-  const double a = absl[j];
+  const long long a = __double_as_longlong(absl[j]);
   int r = 0;
-  for (int i = 0; i < n; ++i) {
-    const double b = absl[i];
+  for (int i = lane; i < n; i += 32) {
+    const long long b = __double_as_longlong(absl[i]);
     r += (b > a || (b == a && i < j)) ? 1 : 0;
   }
-  pos[j] = r;
-  perm[r] = j;
+  for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  if (lane == 0) {
+    pos[j] = r;
+    perm[r] = j;
+  }
 }
 
 // One warp per column i: the sorted positions spanned by i and its strongly
@@ -447,22 +457,46 @@ __global__ void __launch_bounds__(128) k_ref_rot_rows(double* __restrict__ M, in
 }
 
 // E_ij = (S_ij + λ_j R_ij)/(λ_j − λ_i) between groups; R_ij/2 inside a group
-// and on the diagonal (R = I − G)
-__global__ void k_ref_E(const double* __restrict__ S, const double* __restrict__ G, const double* __restrict__ lam,
-                        const int* __restrict__ gid, int n, double* __restrict__ E) {
-  const int64_t nn = (int64_t)n * n;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nn; e += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % n), j = (int)(e / n);
-    const double r = (i == j ? 1.0 : 0.0) - G[e];
-    double v;
-    if (i == j || gid[i] == gid[j]) {
-      v = 0.5 * r;
-    } else {
+// and on the diagonal (R = I − G).  S and R are taken symmetrised (the products
+// leave S_ij ≠ S_ji at rounding level, which a small λ_j − λ_i would magnify), so
+// that E + Eᵀ = R and X·(I + E) is orthogonal up to E².  32×32 tiles with their
+// mirror image through shared memory; emax: largest |E_ij| (float bits).
+__global__ void __launch_bounds__(256) k_ref_E(const double* __restrict__ S, const double* __restrict__ G,
+                                               const double* __restrict__ lam, const int* __restrict__ gid, int n,
+                                               double* __restrict__ E, int* __restrict__ emax) {
+  __shared__ double ts[32][33], tg[32][33];
+  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int r = ty; r < 32; r += 8) {  // the mirror tile: rows j0.., columns i0..
+    const int row = j0 + tx, col = i0 + r;
+    const bool in = row < n && col < n;
+    ts[r][tx] = in ? S[row + (int64_t)col * n] : 0.0;
+    tg[r][tx] = in ? G[row + (int64_t)col * n] : 0.0;
+  }
+  __syncthreads();
+  float mx = 0.f;
+  for (int r = ty; r < 32; r += 8) {
+    const int i = i0 + tx, j = j0 + r;
+    if (i >= n || j >= n) continue;
+    const int64_t e = i + (int64_t)j * n;
+    const double rr = (i == j ? 1.0 : 0.0) - 0.5 * (G[e] + tg[tx][r]);
+    double v = 0.5 * rr;
+    if (i != j && gid[i] != gid[j]) {
       const double den = lam[j] - lam[i];
-      v = den != 0.0 ? (S[e] + lam[j] * r) / den : 0.5 * r;
+      if (den != 0.0) v = (0.5 * (S[e] + ts[tx][r]) + lam[j] * rr) / den;
     }
     E[e] = v;
+    mx = fmaxf(mx, (float)fabs(v));
   }
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (tx == 0) atomicMax(emax, __float_as_int(mx));
+}
+
+// G ← (I − G)/2: the Newton–Schulz step X ← X·(3I − G)/2 as X + X·(I − G)/2,
+// whose product has only to be accurate relative to the small I − G
+__global__ void k_ref_ns(double* __restrict__ G, int n) {
+  const int64_t nn = (int64_t)n * n;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nn; e += (int64_t)gridDim.x * blockDim.x)
+    G[e] = 0.5 * ((e % n == e / n ? 1.0 : 0.0) - G[e]);
 }
 
 // lam_j = Σ_i X_ij·Y_ij (one warp per column)
@@ -541,16 +575,32 @@ bool eig_refine(tnad_ctx* c, const double* A, int64_t n64, double* X, double* la
   int* g_qoff = g_size + n;
   int* si = g_qoff + n;  // 4 ints
   const int64_t col_threads = (int64_t)n * 32;
-  bool done = false;
+  // The iteration is self-correcting, so every product but those of the last
+  // measurement may run on the tensor cores (errors ~1e-14 of the scales, far
+  // below what the step corrects): at n = 1024 one takes 0.3 ms there and 2.1 ms
+  // as DFMA tiles, which are at the FP64 pipe's limit.  Unless the call routes
+  // its FP64 products to the tensor cores anyway (c->fp64_tc), the converged X is
+  // measured once more by DFMA products, and its last correction and λ come from
+  // those.
+  const bool dfma_last = !c->fp64_tc;
+  auto product = [&](bool exact, char ta, const double* P, const double* Q, double alpha, double beta, double* out) {
+    if (exact || !c->tc_ok)
+      gemm_f64(c, ta, 'N', n, n, n, alpha, P, n, Q, n, beta, out, n);
+    else
+      gemm_fp64tc(c, ta, 'N', n, n, n, alpha, P, n, Q, n, beta, out, n);
+  };
+  bool done = false, last = false;
   double prev_off = 0.0;
-  for (int it = 0; it < kMaxIt && !done; ++it) {
-    KernelTimer kt(c, "eig_refine", 6.0 * 2.0 * (double)nn * n);
-    gemm(c, TNAD_PREC_FP64, 'N', 'N', n, n, n, 1.0, A, n, X, n, 0.0, AX, n);
-    gemm(c, TNAD_PREC_FP64, 'T', 'N', n, n, n, 1.0, X, n, AX, n, 0.0, S, n);
-    gemm(c, TNAD_PREC_FP64, 'T', 'N', n, n, n, 1.0, X, n, X, n, 0.0, G, n);
+  for (int it = 0; it < kMaxIt + 1 && !done; ++it) {
+    KernelTimer kt(c, "eig_refine", (last ? 4.0 : 6.0) * 2.0 * (double)nn * n);
+    const bool exact = last;
+    product(exact, 'N', A, X, 1.0, 0.0, AX);
+    product(exact, 'T', X, AX, 1.0, 0.0, S);
+    product(exact, 'T', X, X, 1.0, 0.0, G);
     k_ref_colstats<<<nblk(col_threads), 256, 0, c->stream>>>(S, G, n, lam, absl, cmo, cmr);
-    k_ref_rank<<<nblk(n), 256, 0, c->stream>>>(absl, n, pos, perm);
+    k_ref_rank<<<nblk(col_threads), 256, 0, c->stream>>>(absl, n, pos, perm);
     TNAD_CK(cudaMemsetAsync(cover, 0, sizeof(int) * (size_t)(n + 1), c->stream));
+    TNAD_CK(cudaMemsetAsync(si + 3, 0, sizeof(int), c->stream));
     k_ref_strong<<<nblk(col_threads), 256, 0, c->stream>>>(S, G, lam, pos, n, kEta, cover);
     k_ref_groups<<<1, 1024, 0, c->stream>>>(cover, perm, absl, cmo, cmr, n, fro2, gid, g_start, g_size, g_qoff, si,
                                             sd);
@@ -568,9 +618,19 @@ bool eig_refine(tnad_ctx* c, const double* A, int64_t n64, double* X, double* la
     // not an approximate eigendecomposition (the first measurement), growing
     // errors, non-finite entries or a group too large for one CTA: give up
     if (!std::isfinite(hd[0]) || !std::isfinite(hd[1]) || maxgroup > kMaxGroup) return false;
-    if ((it == 0 && hd[0] > kMaxStartOff) || (it > 0 && hd[0] > 4.0 * prev_off)) return false;
+    if ((it == 0 && hd[0] > kMaxStartOff) || (it > 0 && hd[0] > std::max(4.0 * prev_off, 1e-12))) return false;
     prev_off = hd[0];
-    done = it >= 1 && hd[0] <= 1e-10 && hd[1] <= 1e-8 && ngroups == 0;
+    if (last) {
+      done = true;
+    } else if (it >= 1 && hd[0] <= 1e-10 && hd[1] <= 1e-8 && ngroups == 0) {
+      if (dfma_last) {
+        last = true;  // X stays; the next pass measures it by DFMA products
+        continue;
+      }
+      done = true;
+    } else if (it >= kMaxIt - 1) {
+      return false;
+    }
     if (ngroups > 0) {
       // Rayleigh–Ritz inside the groups; S, G and X follow the block rotation
       const size_t rr_sm = (size_t)(maxgroup * (maxgroup + 1) + maxgroup * maxgroup) * 8;
@@ -586,22 +646,35 @@ bool eig_refine(tnad_ctx* c, const double* A, int64_t n64, double* X, double* la
       count_launch(c, 7);
       check_launch(c, "eig_refine_rr");
     }
-    k_ref_E<<<nblk(nn), 256, 0, c->stream>>>(S, G, lam, gid, n, E);
+    const dim3 ge((unsigned)((n + 31) / 32), (unsigned)((n + 31) / 32));
+    k_ref_E<<<ge, 256, 0, c->stream>>>(S, G, lam, gid, n, E, si + 3);
     count_launch(c);
     check_launch(c, "eig_refine_E");
-    // X ← X·(I + E), then one Newton–Schulz step X ← X·(3I − XᵀX)/2
+    // X ← X·(I + E), then one Newton–Schulz step X ← X·(3I − XᵀX)/2; not after
+    // the last correction where E² is below rounding (λ = S_jj/G_jj is then
+    // accurate to E² as well)
     copy_d2d(c, Xn, X, nn);
-    gemm(c, TNAD_PREC_FP64, 'N', 'N', n, n, n, 1.0, X, n, E, n, 1.0, Xn, n);
-    gemm(c, TNAD_PREC_FP64, 'T', 'N', n, n, n, 1.0, Xn, n, Xn, n, 0.0, G, n);
+    product(false, 'N', X, E, 1.0, 1.0, Xn);
     copy_d2d(c, X, Xn, nn);
-    gemm(c, TNAD_PREC_FP64, 'N', 'N', n, n, n, -0.5, Xn, n, G, n, 1.5, X, n);
+    if (done) {
+      TNAD_CK(cudaMemcpyAsync(hs + 3, si + 3, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+      TNAD_CK(cudaStreamSynchronize(c->stream));
+      float em;
+      std::memcpy(&em, hs + 3, sizeof(em));
+      if (em <= 1e-8f) break;
+    }
+    product(done && dfma_last, 'T', Xn, Xn, 1.0, 0.0, G);
+    k_ref_ns<<<nblk(nn), 256, 0, c->stream>>>(G, n);
+    count_launch(c);
+    product(false, 'N', Xn, G, 1.0, 1.0, X);
+    if (done) {  // the last correction was not small against 1e-8: λ_j = x_jᵀAx_j anew
+      product(dfma_last, 'N', A, X, 1.0, 0.0, AX);
+      k_ref_coldots<<<nblk(col_threads), 256, 0, c->stream>>>(X, AX, n, lam);
+      count_launch(c);
+      check_launch(c, "eig_refine_lam");
+    }
   }
-  if (!done) return false;
-  gemm(c, TNAD_PREC_FP64, 'N', 'N', n, n, n, 1.0, A, n, X, n, 0.0, AX, n);
-  k_ref_coldots<<<nblk(col_threads), 256, 0, c->stream>>>(X, AX, n, lam);
-  count_launch(c);
-  check_launch(c, "eig_refine_lam");
-  return true;
+  return done;
 }
 
 // Eigendecomposition H = W·diag(lam)·Wᵀ of a small symmetric p×p matrix
