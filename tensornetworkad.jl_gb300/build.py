@@ -31,7 +31,7 @@ def _nvcc() -> str:
 
 
 def _newest_header() -> float:
-    hs = list(CSRC.glob("*.h")) + list((ROOT / "include").glob("*.h"))
+    hs = [*CSRC.glob("*.h"), *CSRC.glob("*.cuh"), *(ROOT / "include").glob("*.h")]
     return max((h.stat().st_mtime for h in hs), default=0.0)
 
 

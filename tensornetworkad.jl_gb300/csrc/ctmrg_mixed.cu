@@ -28,7 +28,6 @@
 namespace tnad {
 
 void chol_inv_upper(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* dev_fail);
-void chol_inv_upper_f32(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* dev_fail);
 void randn(tnad_ctx* c, double* x, int64_t n, uint64_t seed, double scale, bool accumulate,
            const double* dev_sumsq = nullptr);
 
@@ -146,8 +145,8 @@ void align_polar(tnad_ctx* c, int prec, double* z, const double* zprev, int64_t 
 // subspaces: two CholeskyQR passes (Gram in FP64).  A tiny random component
 // (relative `jitter`) keeps Y full rank when M has fewer than p non-null
 // directions (the zero-padded raw environment of the first steps).  The
-// first factorisation stays in FP64: CholeskyQR in FP32 (even shifted, as in
-// CholeskyQR3) breaks down on these nearly rank-deficient blocks.
+// factorisations are FP64: CholeskyQR in FP32 (even shifted, as in CholeskyQR3)
+// breaks down on these nearly rank-deficient blocks.
 void cholqr2(tnad_ctx* c, int prec, const double* Y, int64_t n, int64_t p, double* Q, double jitter, uint64_t seed) {
   WsScope scope(c);
   double* G = ws_d(c, p * p);
@@ -163,12 +162,7 @@ void cholqr2(tnad_ctx* c, int prec, const double* Y, int64_t n, int64_t p, doubl
   const double* src = t;
   for (int pass = 0; pass < 2; ++pass) {
     gemm(c, TNAD_PREC_FP64, 'T', 'N', p, p, n, 1.0, src, n, src, n, 0.0, G, p);
-    // the second Gram matrix is I + O(κ(Y)²·ε64): at TF32X3 accuracy its
-    // factor is taken in FP32 (GB300's FP32 pipe is far wider than its FP64 one)
-    if (pass == 1 && prec != TNAD_PREC_FP64)
-      chol_inv_upper_f32(c, G, p, Ri, fail);
-    else
-      chol_inv_upper(c, G, p, Ri, fail);
+    chol_inv_upper(c, G, p, Ri, fail);
     gemm(c, prec, 'N', 'N', n, p, p, 1.0, src, n, Ri, p, 0.0, Q, n);
     if (pass == 0) {
       copy_d2d(c, t, Q, n * p);

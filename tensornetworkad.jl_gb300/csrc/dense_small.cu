@@ -1,135 +1,231 @@
-// Small dense kernels of the subspace eigensolver, each in one CTA:
+// Small dense kernels of the subspace eigensolver, in one CTA or one cluster:
 //  - Cholesky of a p×p Gram matrix and the inverse of its triangular factor
-//    (CholeskyQR of the n×p block: Q = Y·R⁻¹);
-//  - cyclic parallel Jacobi eigendecomposition of a symmetric p×p matrix held
-//    in shared memory (circle-method rounds of p/2 disjoint rotations), in
-//    FP32 while the contractions run at 3xTF32 accuracy and in FP64 for the
-//    polishing steps; eigenvectors accumulate in global memory;
+//    (CholeskyQR of the n×p block: Q = Y·R⁻¹), in one cluster of 16 CTAs;
+//  - parallel Jacobi eigendecompositions of a symmetric p×p matrix held in
+//    shared memory (circle-method rounds of p/2 disjoint rotations): FP32,
+//    one-sided (the Rayleigh–Ritz problems, refined by products where FP64 is
+//    wanted), and FP64, two-sided (the gauge-fixing problems; its eigenvectors
+//    accumulate in global memory);
 //  - a counter-based Gaussian generator for deterministic start blocks.
 #include <cfloat>
 #include <atomic>
 #include <cmath>
 
+#include "fp64_fast.cuh"
 #include "tnad_internal.h"
 
 namespace tnad {
 
 // ---------------------------------------------------------------- Cholesky
-// G (p×p, column-major, symmetric positive semi-definite) → R (p×p, upper
+// G (p×p, column-major, symmetric positive semi-definite) → R⁻¹ (p×p, upper
 // triangular, zeros below) with G + E = RᵀR and E ≥ 0 diagonal: a pivot below
 // kPivotFloor·max_k G_kk (a column numerically inside the span of the previous
 // ones, e.g. when the subspace is wider than the rank of the matrix it
 // iterates on) is raised to that floor, so the factor stays finite and the
 // column maps to a vector of norm ≲ 1.  *fail = 1 when G has no positive
-// finite diagonal.  One CTA, right-looking, the matrix in shared memory.
+// finite diagonal.
+//
+// One cluster of 16 CTAs.  GB300 retires 1.7 FP64 multiply-adds a clock and SM:
+// the p³/3 of factor and inverse alone take 85 µs in one SM at p = 96, and the
+// one-CTA factorisation with its quotient, square root and two barriers a
+// pivot took 260 µs, the inverse 89 more.  Here the columns of G = L·Lᵀ and of
+// Y = L⁻¹ (the right-hand sides of L·Y = I) are dealt to the CTAs in panels of
+// 4, right-looking: the owner factors a panel (one row per thread; every warp
+// carries a copy of the 4×4 diagonal block, so no barrier inside), one cluster
+// barrier, every CTA reads the panel from the owner's shared memory and
+// updates its own columns of both parts.  The owner of the next panel updates
+// and factors that one first and leaves its other columns for the time between
+// its arrival at the barrier and the others'.  R⁻¹ = Yᵀ.  Panels of 8 on 8 CTAs
+// without that order took 107 µs, this 86 (p = 96, factor and inverse).  Also replaces the FP32 factorisation that
+// the TF32 phase used for its second pass (156 µs).
 constexpr double kPivotFloor = 1e-14;
+constexpr int kCholC = 16;    // CTAs of the cluster
+constexpr int kCholNB = 4;    // columns of a panel
+constexpr int kCholMaxP = 160;
+constexpr int kCholLd = kCholMaxP + 1;  // column stride; slot kCholMaxP holds 1/L_kk
+constexpr int kCholPanels = (kCholMaxP / kCholNB + kCholC - 1) / kCholC;  // panels of one CTA
 
-template <typename T>
-__global__ void __launch_bounds__(512) k_chol_factor(const double* __restrict__ G, int p, double floor_rel,
-                                                     double* __restrict__ Rg, int* __restrict__ fail) {
-  extern __shared__ unsigned char sm_raw[];
-  T* A = reinterpret_cast<T*>(sm_raw);  // working copy of G (upper triangle), p × ld
-  const int ld = p + 1;                 // padded leading dimension
-  __shared__ T piv[2];                  // 1/d_k, sqrt(d_k) of the current step
-  __shared__ int bad;
-  __shared__ T floor_;
-  for (int e = threadIdx.x; e < p * p; e += blockDim.x) A[(e % p) + (e / p) * ld] = (T)G[e];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    T mx = 0;
-    for (int k = 0; k < p; ++k) mx = fmax(mx, A[k + k * ld]);
-    bad = (mx > (T)0 && isfinite(mx)) ? 0 : 1;
-    floor_ = bad ? (T)1e-30 : (T)floor_rel * mx;
-  }
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  // zeros below the diagonal of the output factor
-  for (int j = w; j < p; j += nw)
-    for (int i = j + 1 + lane; i < p; i += 32) Rg[i + (int64_t)j * p] = 0.0;
-  __syncthreads();
-  // right-looking, one barrier pair per pivot; warp w owns columns j ≡ w (mod nw)
-  // and its lanes the rows of each column:  R[k, j] = A[k, j]/√d_k and
-  // A[i, j] −= A[k, i]·A[k, j]/d_k for k < i ≤ j
-  for (int k = 0; k < p; ++k) {
-    if (threadIdx.x == 0) {
-      T d = A[k + k * ld];
-      if (!(d > floor_)) d = floor_;
-      piv[0] = (T)1 / d;
-      piv[1] = sqrt(d);
-    }
-    __syncthreads();
-    const T inv_d = piv[0], rkk = piv[1], inv_r = inv_d * rkk;  // 1/√d
-    for (int j = k + ((w - k) % nw + nw) % nw; j < p; j += nw) {
-      const T akj = A[k + j * ld];
-      if (lane == 0) Rg[k + (int64_t)j * p] = (double)(j == k ? rkk : akj * inv_r);
-      if (j == k) continue;
-      const T f = akj * inv_d;
-      for (int i = k + 1 + lane; i <= j; i += 32) A[i + j * ld] -= A[k + i * ld] * f;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0 && bad) *fail = 1;
-}
-
-// Rinv = R⁻¹ for upper-triangular R (p×p): one warp per column j solves
-// R·x = e_j by back substitution (lanes split each row's dot product), R in
-// shared memory with leading dimension p+1; 8 columns per CTA.
-template <typename T>
-__global__ void k_tri_inv(const double* __restrict__ Rg, int p, double* __restrict__ Rinv) {
-  extern __shared__ unsigned char sm_raw[];
-  T* R = reinterpret_cast<T*>(sm_raw);  // p × ld
-  const int ld = p + 1;
-  T* rd = R + p * ld;  // 1/R[i,i]
-  T* X = rd + p;       // 8 × p solution columns
-  for (int e = threadIdx.x; e < p * p; e += blockDim.x) {
-    const int i = e % p, j = e / p;
-    R[i + j * ld] = (T)Rg[e];
-  }
-  for (int i = threadIdx.x; i < p; i += blockDim.x) rd[i] = (T)1 / (T)Rg[i + (int64_t)i * p];
-  __syncthreads();
+__global__ void __launch_bounds__(256) k_chol_inv(const double* __restrict__ G, int p, double floor_rel,
+                                                  double* __restrict__ Rinv, int* __restrict__ fail) {
+  extern __shared__ __align__(16) double csm[];
+  double* A = csm;                                        // own columns of L, kCholPanels·8 × kCholLd
+  double* Y = A + kCholPanels * kCholNB * kCholLd;        // own columns of L⁻¹
+  double* Lp = Y + kCholPanels * kCholNB * kCholLd;       // the current panel, 8 × kCholLd
+  __shared__ double fl_sh;
+  const int rank = blockIdx.x;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = blockIdx.x * 8 + w;
-  if (j >= p) return;
-  T* x = X + w * p;
-  for (int i = j; i >= 0; --i) {
-    T s = 0;
-    for (int l = i + 1 + lane; l <= j; l += 32) s += R[i + l * ld] * x[l];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) x[i] = ((i == j ? (T)1 : (T)0) - s) * rd[i];
-    __syncwarp();
+  const int np = (p + kCholNB - 1) / kCholNB;
+  auto gcol = [&](int lc) { return ((lc / kCholNB) * kCholC + rank) * kCholNB + lc % kCholNB; };
+  for (int lc = w; lc < kCholPanels * kCholNB; lc += 8) {
+    const int j = gcol(lc);
+    if (j >= p) continue;
+    for (int i = lane; i < p; i += 32) {
+      A[lc * kCholLd + i] = G[i + (int64_t)j * p];
+      Y[lc * kCholLd + i] = i == j ? 1.0 : 0.0;
+    }
   }
-  for (int i = lane; i < p; i += 32) Rinv[i + (int64_t)j * p] = i <= j ? (double)x[i] : 0.0;
-}
-
-template <typename T>
-void chol_inv_t(tnad_ctx* c, const double* G, int64_t p, double floor_rel, double* Rinv, int* dev_fail) {
-  static std::atomic<bool> attr{false};
-  const size_t es = sizeof(T);
-  if (!attr) {
-    TNAD_CK(cudaFuncSetAttribute(k_chol_factor<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(160 * 161 * es)));
-    TNAD_CK(cudaFuncSetAttribute(k_tri_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)((160 * 161 + 9 * 160) * es)));
-    attr = true;
+  if (w == 0) {
+    double mx = 0.0;
+    for (int k = lane; k < p; k += 32) mx = fmax(mx, G[k + (int64_t)k * p]);
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) {
+      const bool ok = mx > 0.0 && isfinite(mx);
+      fl_sh = ok ? floor_rel * mx : 1e-30;
+      if (!ok && rank == 0) *fail = 1;
+    }
   }
-  WsScope scope(c);
-  double* R = ws_d(c, p * p);
-  KernelTimer kt(c, "chol", (double)p * p * p / 3.0);
-  k_chol_factor<T><<<1, 512, (size_t)p * (p + 1) * es, c->stream>>>(G, (int)p, floor_rel, R, dev_fail);
-  k_tri_inv<T><<<(unsigned)((p + 7) / 8), 256, (size_t)(p * (p + 1) + 9 * p) * es, c->stream>>>(R, (int)p, Rinv);
-  count_launch(c, 2);
-  check_launch(c, "chol_inv");
+  __syncthreads();
+  const double flo = fl_sh;
+  // Factor the panel J in its owner's shared memory: row k0 + tid in this thread,
+  // rows k0..k0+3 also in lanes 0..3 of every warp
+  auto factor = [&](int J) {
+    const int k0 = J * kCholNB, nc = min(kCholNB, p - k0);
+    double* Ap = A + (J / kCholC) * kCholNB * kCholLd;
+    const int i = k0 + (int)threadIdx.x, id = k0 + (lane & (kCholNB - 1));
+    double a[kCholNB], d[kCholNB];
+#pragma unroll
+    for (int c = 0; c < kCholNB; ++c) {
+      a[c] = (c < nc && i < p) ? Ap[c * kCholLd + i] : 0.0;
+      d[c] = (c < nc && id < p) ? Ap[c * kCholLd + id] : 0.0;
+    }
+    __syncthreads();  // every warp has its copy of the diagonal block
+    if ((int)(threadIdx.x & ~31u) >= p - k0) return;  // no row of the panel in this warp
+#pragma unroll
+    for (int c = 0; c < kCholNB; ++c) {
+      if (c < nc) {
+        double piv = __shfl_sync(0xffffffffu, d[c], c);
+        if (!(piv > flo)) piv = flo;
+        const double inv = rsqrt_any(piv);
+        a[c] = i == k0 + c ? piv * inv : a[c] * inv;
+        d[c] *= inv;
+#pragma unroll
+        for (int b = c + 1; b < kCholNB; ++b) {
+          if (b < nc) {
+            const double lb = __shfl_sync(0xffffffffu, d[c], b);
+            a[b] = fma(-a[c], lb, a[b]);
+            d[b] = fma(-d[c], lb, d[b]);
+          }
+        }
+        if (threadIdx.x == 0) Ap[c * kCholLd + kCholMaxP] = inv;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < kCholNB; ++c)
+      if (c < nc && i < p) Ap[c * kCholLd + i] = a[c];
+  };
+  // col[r] −= Σ_c f_c·L(r, k0 + c) for the rows r = r0 + lane, r0 + lane + step...
+  auto apply = [&](double* col, const double* f, int nc, int r0, int step, int from) {
+    for (int r = r0 + lane; r < p; r += step) {
+      if (r < from) continue;
+      double v = col[r];
+#pragma unroll
+      for (int c = 0; c < kCholNB; ++c)
+        if (c < nc) v = fma(-f[c], Lp[c * kCholLd + r], v);
+      col[r] = v;
+    }
+  };
+  if (rank == 0) factor(0);
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  for (int J = 0; J < np; ++J) {
+    const int k0 = J * kCholNB, nc = min(kCholNB, p - k0), owner = J % kCholC;
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    {  // the panel, rows k0.. and the 1/L_kk slot, from the owner's shared memory
+      const double* Ap = A + (J / kCholC) * kCholNB * kCholLd;
+      uint32_t remote;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                   : "=r"(remote)
+                   : "r"((uint32_t)__cvta_generic_to_shared(Ap)), "r"(owner));
+      const int nr = p - k0 + 1;
+      for (int c = w & (kCholNB - 1); c < nc; c += kCholNB)
+        for (int e = lane + 32 * (w / kCholNB); e < nr; e += 64) {
+          const int row = e < nr - 1 ? k0 + e : kCholMaxP;
+          double v;
+          asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(remote + (uint32_t)(c * kCholLd + row) * 8u));
+          Lp[c * kCholLd + row] = v;
+        }
+    }
+    __syncthreads();
+    const int k1 = k0 + nc;  // first column of the next panel
+    const bool next = J + 1 < np && rank == (J + 1) % kCholC;
+    if (next) {
+      const int c = w & (kCholNB - 1);
+      if (k1 + c < p) {
+        double f[kCholNB];
+#pragma unroll
+        for (int q = 0; q < kCholNB; ++q) f[q] = q < nc ? Lp[q * kCholLd + k1 + c] : 0.0;
+        apply(A + (((J + 1) / kCholC) * kCholNB + c) * kCholLd, f, nc, k1 + 32 * (w / kCholNB), 64, k1 + c);
+      }
+      __syncthreads();
+      factor(J + 1);
+    }
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    // own columns: L part beyond the panel (and the next one, done above), Y part
+    // up to the panel's last column
+    for (int lc = w; lc < 2 * kCholPanels * kCholNB; lc += 8) {
+      const bool yp = lc >= kCholPanels * kCholNB;
+      const int l = yp ? lc - kCholPanels * kCholNB : lc, j = gcol(l);
+      if (j >= p || (yp ? j >= k1 : j < (next ? k1 + kCholNB : k1))) continue;
+      double* col = (yp ? Y : A) + l * kCholLd;
+      double f[kCholNB];
+      if (!yp) {
+#pragma unroll
+        for (int c = 0; c < kCholNB; ++c) f[c] = c < nc ? Lp[c * kCholLd + j] : 0.0;
+      } else {
+        // forward substitution within the panel's rows, lane c holding row k0 + c
+        double v = lane < nc ? col[k0 + lane] : 0.0;
+#pragma unroll
+        for (int c = 0; c < kCholNB; ++c) {
+          f[c] = 0.0;
+          if (c < nc) {
+            f[c] = __shfl_sync(0xffffffffu, v, c) * Lp[c * kCholLd + kCholMaxP];
+            if (lane > c && lane < nc) v = fma(-f[c], Lp[c * kCholLd + k0 + lane], v);
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < kCholNB; ++c)
+          if (lane == c && c < nc) col[k0 + c] = f[c];
+      }
+      apply(col, f, nc, k1, 32, yp ? 0 : j);
+    }
+    __syncthreads();  // Lp is free, the own columns are up to date
+  }
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  // R⁻¹(j, i) = Y(i, j): column j of Y is row j of R⁻¹
+  for (int lc = w; lc < kCholPanels * kCholNB; lc += 8) {
+    const int j = gcol(lc);
+    if (j >= p) continue;
+    for (int i = lane; i < p; i += 32) Rinv[j + (int64_t)i * p] = i >= j ? Y[lc * kCholLd + i] : 0.0;
+  }
+  // no CTA leaves while another may still read its shared memory
+  asm volatile("barrier.cluster.arrive;\nbarrier.cluster.wait;" ::: "memory");
 }
 
 void chol_inv_upper(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* dev_fail) {
-  TNAD_REQUIRE(p >= 1 && p <= 160, TNAD_ERR_SHAPE, "chol_inv_upper: p must be in [1,160]");
-  chol_inv_t<double>(c, G, p, kPivotFloor, Rinv, dev_fail);
-}
-
-// FP32 factorisation (relative pivot floor 1e-7) for Gram matrices that are
-// already close to I: the second CholeskyQR pass while the contractions run
-// at TF32X3 accuracy.
-void chol_inv_upper_f32(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* dev_fail) {
-  TNAD_REQUIRE(p >= 1 && p <= 160, TNAD_ERR_SHAPE, "chol_inv_upper_f32: p must be in [1,160]");
-  chol_inv_t<float>(c, G, p, 1e-7, Rinv, dev_fail);
+  TNAD_REQUIRE(p >= 1 && p <= kCholMaxP, TNAD_ERR_SHAPE, "chol_inv_upper: p must be in [1,160]");
+  constexpr size_t smem = (size_t)(2 * kCholPanels + 1) * kCholNB * kCholLd * sizeof(double);
+  static std::atomic<bool> attr{false};
+  if (!attr) {
+    TNAD_CK(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TNAD_CK(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    attr = true;
+  }
+  KernelTimer kt(c, "chol", (double)p * p * p / 3.0);
+  cudaLaunchConfig_t cf = {};
+  cf.gridDim = dim3(kCholC);
+  cf.blockDim = dim3(256);
+  cf.dynamicSmemBytes = smem;
+  cf.stream = c->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kCholC;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cf.attrs = at;
+  cf.numAttrs = 1;
+  TNAD_CK(cudaLaunchKernelEx(&cf, k_chol_inv, G, (int)p, kPivotFloor, Rinv, dev_fail));
+  count_launch(c);
+  check_launch(c, "chol_inv");
 }
 
 // ---------------------------------------------------------------- Jacobi eigh
@@ -147,25 +243,24 @@ __device__ __forceinline__ void circle_pair(int r, int k, int NP, int* p, int* q
 // descending when by_value), W (p×p eigenvectors as columns, same order).
 // Z: p×p scratch for the unsorted vectors.  Sweeps until no rotation is needed
 // (or max_sweeps; the sweep count goes to info[0]).
-template <typename T>
 __global__ void k_eigh_jacobi(const double* __restrict__ A, int p, int max_sweeps, double* __restrict__ lam,
-                              double* __restrict__ W, T* __restrict__ Z, int* __restrict__ info, int by_value) {
+                              double* __restrict__ W, double* __restrict__ Z, int* __restrict__ info, int by_value) {
   extern __shared__ unsigned char smraw[];
-  T* H = reinterpret_cast<T*>(smraw);  // p×p, leading dimension ld = p+1 (bank-conflict free)
+  double* H = reinterpret_cast<double*>(smraw);  // p×p, leading dimension ld = p+1 (bank-conflict free)
   const int ld = p + 1;
-  __shared__ T cs_[128], sn_[128];
+  __shared__ double cs_[128], sn_[128];
   __shared__ int pp_[128], qq_[128];
   __shared__ int rotated;
   __shared__ double fro_part[32];
   const int NP = p + (p & 1);
-  const double eps_t = sizeof(T) == 8 ? DBL_EPSILON : FLT_EPSILON;
-  const T tol = (T)(4.0 * eps_t * sqrt((double)p));
+  const double eps_t = DBL_EPSILON;
+  const double tol = (double)(4.0 * eps_t * sqrt((double)p));
   double ss = 0.0;
   for (int e = threadIdx.x; e < p * p; e += blockDim.x) {
     const double v = A[e];
     ss += v * v;
-    H[(e % p) + (e / p) * ld] = (T)v;
-    Z[e] = (e % p == e / p) ? (T)1 : (T)0;
+    H[(e % p) + (e / p) * ld] = (double)v;
+    Z[e] = (e % p == e / p) ? 1.0 : (double)0;
   }
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if ((threadIdx.x & 31) == 0) fro_part[threadIdx.x >> 5] = ss;
@@ -175,7 +270,7 @@ __global__ void k_eigh_jacobi(const double* __restrict__ A, int p, int max_sweep
   // relative rule would keep rotating until the sweep cap.
   double fro2 = 0.0;
   for (int w = 0; w < (int)(blockDim.x >> 5); ++w) fro2 += fro_part[w];
-  const T absfl = (T)(2.0 * eps_t * sqrt((double)p) * sqrt(fro2));
+  const double absfl = (double)(2.0 * eps_t * sqrt((double)p) * sqrt(fro2));
   int sweep = 0;
   for (; sweep < max_sweeps; ++sweep) {
     if (threadIdx.x == 0) rotated = 0;
@@ -185,20 +280,18 @@ __global__ void k_eigh_jacobi(const double* __restrict__ A, int p, int max_sweep
       for (int k = threadIdx.x; k < NP / 2; k += blockDim.x) {
         int a, b;
         circle_pair(r, k, NP, &a, &b);
-        T c = 1, s = 0;
+        double c = 1, s = 0;
         if (a < p && b < p) {
           if (a > b) {
             int t = a;
             a = b;
             b = t;
           }
-          const T apq = H[a + b * ld], app = H[a + a * ld], aqq = H[b + b * ld];
-          // stop rule in the kernel's own precision (an FP64 test in the FP32
-          // kernel would run on GB300's narrow FP64 pipe)
-          if (apq != (T)0 && fabs(apq) > tol * sqrt(fabs(app)) * sqrt(fabs(aqq)) && fabs(apq) > absfl) {
-            const T tau = (aqq - app) / ((T)2 * apq);
-            const T t = (tau >= (T)0 ? (T)1 : (T)-1) / (fabs(tau) + sqrt((T)1 + tau * tau));
-            c = (T)1 / sqrt((T)1 + t * t);
+          const double apq = H[a + b * ld], app = H[a + a * ld], aqq = H[b + b * ld];
+          if (apq != (double)0 && fabs(apq) > tol * sqrt(fabs(app)) * sqrt(fabs(aqq)) && fabs(apq) > absfl) {
+            const double tau = (aqq - app) / (2.0 * apq);
+            const double t = (tau >= (double)0 ? 1.0 : -1.0) / (fabs(tau) + sqrt((double)1 + tau * tau));
+            c = (double)1 / sqrt((double)1 + t * t);
             s = t * c;
             rotated = 1;
           }
@@ -217,10 +310,10 @@ __global__ void k_eigh_jacobi(const double* __restrict__ A, int p, int max_sweep
       // rows: (row a, row b) ← (c·row a − s·row b, s·row a + c·row b)
       for (int k = wid; k < NP / 2; k += nwarp) {
         const int a = pp_[k], b = qq_[k];
-        if (a < 0 || sn_[k] == (T)0) continue;
-        const T c = cs_[k], s = sn_[k];
+        if (a < 0 || sn_[k] == (double)0) continue;
+        const double c = cs_[k], s = sn_[k];
         for (int col = lane; col < p; col += 32) {
-          const T x = H[a + col * ld], y = H[b + col * ld];
+          const double x = H[a + col * ld], y = H[b + col * ld];
           H[a + col * ld] = c * x - s * y;
           H[b + col * ld] = s * x + c * y;
         }
@@ -229,20 +322,20 @@ __global__ void k_eigh_jacobi(const double* __restrict__ A, int p, int max_sweep
       // columns of H and of Z; then the rotated pair's off-diagonal entry is 0
       for (int k = wid; k < NP / 2; k += nwarp) {
         const int a = pp_[k], b = qq_[k];
-        if (a < 0 || sn_[k] == (T)0) continue;
-        const T c = cs_[k], s = sn_[k];
+        if (a < 0 || sn_[k] == (double)0) continue;
+        const double c = cs_[k], s = sn_[k];
         for (int row = lane; row < p; row += 32) {
-          const T x = H[row + a * ld], y = H[row + b * ld];
+          const double x = H[row + a * ld], y = H[row + b * ld];
           H[row + a * ld] = c * x - s * y;
           H[row + b * ld] = s * x + c * y;
-          const T zx = Z[row + a * p], zy = Z[row + b * p];
+          const double zx = Z[row + a * p], zy = Z[row + b * p];
           Z[row + a * p] = c * zx - s * zy;
           Z[row + b * p] = s * zx + c * zy;
         }
         __syncwarp();
         if (lane == 0) {
-          H[a + b * ld] = (T)0;
-          H[b + a * ld] = (T)0;
+          H[a + b * ld] = (double)0;
+          H[b + a * ld] = (double)0;
         }
       }
       __syncthreads();
@@ -268,30 +361,200 @@ __global__ void k_eigh_jacobi(const double* __restrict__ A, int p, int max_sweep
   if (threadIdx.x == 0 && info) info[0] = sweep;
 }
 
+// The FP32 solve, one-sided: W = A·V and V in shared memory, the rotation of a
+// pair from the 2×2 block of VᵀAV (a = v_p·w_p, b = v_q·w_q, g = (v_p·w_q +
+// v_q·w_p)/2), so that ±λ pairs stay apart.  8 lanes per pair, their rows as
+// 16-byte shared loads and packed FP32 pairs (fma.rn.f32x2): all ⌈p/2⌉ pairs of
+// a round in ⌈p/8⌉ warps at once and one barrier a round, where the two-sided
+// form (k_eigh_jacobi) takes three and two passes over H.  Latency bound (one
+// CTA): p = 96 in 455 µs, two-sided 758.  Same stop rule.
+__device__ __forceinline__ uint64_t pk2(float a, float b) {
+  return ((uint64_t)__float_as_uint(b) << 32) | __float_as_uint(a);
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float hsum2(uint64_t a) {
+  return __uint_as_float((unsigned)a) + __uint_as_float((unsigned)(a >> 32));
+}
+
+constexpr int kEigh32MaxP = 160;  // W and V of FP32 in one CTA's shared memory
+
+template <int RV>  // 16-byte row chunks per lane: ⌈p/32⌉
+__global__ void __launch_bounds__(640) k_eigh32(const double* __restrict__ A, int p, int max_sweeps,
+                                                double* __restrict__ lam, double* __restrict__ Wout,
+                                                int* __restrict__ info, int by_value) {
+  extern __shared__ __align__(16) float esm[];
+  const int pr = (p + 3) & ~3, cs = 2 * pr, q4 = pr >> 2;  // column: W rows, then V rows
+  __shared__ float fro_part[20];
+  __shared__ int rotated;
+  __shared__ float lam_sh[kEigh32MaxP];
+  const int NP = p + (p & 1), nb = NP >> 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l8 = lane & 7;
+  float ss = 0.f;
+  for (int e = threadIdx.x; e < p * cs; e += blockDim.x) {
+    const int i = e % cs, j = e / cs;
+    float v;
+    if (i < pr) {
+      v = i < p ? (float)A[i + (int64_t)j * p] : 0.f;
+      ss = fmaf(v, v, ss);
+    } else {
+      v = i - pr == j ? 1.f : 0.f;
+    }
+    esm[e] = v;
+  }
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (lane == 0) fro_part[warp] = ss;
+  __syncthreads();
+  float fro2 = 0.f;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) fro2 += fro_part[w];
+  const float tol = 4.f * FLT_EPSILON * sqrtf((float)p);
+  const float absfl = 2.f * FLT_EPSILON * sqrtf((float)p) * sqrtf(fro2);
+  const int k = warp * 4 + (lane >> 3);  // this lane group's pair
+  int sweep = 0;
+  for (; sweep < max_sweeps; ++sweep) {
+    if (threadIdx.x == 0) rotated = 0;
+    __syncthreads();
+    for (int r = 0; r < NP - 1; ++r) {
+      int a = 0, b = 0;
+      bool on = k < nb;
+      if (on) {
+        circle_pair(r, k, NP, &a, &b);
+        on = a < p && b < p;
+        if (a > b) {
+          const int t = a;
+          a = b;
+          b = t;
+        }
+      }
+      ulonglong2* xa = reinterpret_cast<ulonglong2*>(esm + a * cs);
+      ulonglong2* xb = reinterpret_cast<ulonglong2*>(esm + b * cs);
+      ulonglong2 wx[RV], wy[RV], vx[RV], vy[RV];
+      uint64_t sa = 0, sb = 0, sg = 0;
+#pragma unroll
+      for (int e = 0; e < RV; ++e) {
+        const int i = l8 + 8 * e;
+        const bool in = on && i < q4;
+        const ulonglong2 z = make_ulonglong2(0, 0);
+        wx[e] = in ? xa[i] : z;
+        wy[e] = in ? xb[i] : z;
+        vx[e] = in ? xa[q4 + i] : z;
+        vy[e] = in ? xb[q4 + i] : z;
+      }
+#pragma unroll
+      for (int e = 0; e < RV; ++e) {
+        sa = fma2(vx[e].x, wx[e].x, sa);
+        sb = fma2(vy[e].x, wy[e].x, sb);
+        sg = fma2(vx[e].x, wy[e].x, sg);
+        sg = fma2(vy[e].x, wx[e].x, sg);
+        sa = fma2(vx[e].y, wx[e].y, sa);
+        sb = fma2(vy[e].y, wy[e].y, sb);
+        sg = fma2(vx[e].y, wy[e].y, sg);
+        sg = fma2(vy[e].y, wx[e].y, sg);
+      }
+      float fa = hsum2(sa), fb = hsum2(sb), g2 = hsum2(sg);  // g2 = 2g
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        fa += __shfl_xor_sync(0xffffffffu, fa, o);
+        fb += __shfl_xor_sync(0xffffffffu, fb, o);
+        g2 += __shfl_xor_sync(0xffffffffu, g2, o);
+      }
+      const float ag = 0.5f * fabsf(g2);
+      if (on && ag > tol * fsqrt_ap(fabsf(fa)) * fsqrt_ap(fabsf(fb)) && ag > absfl) {
+        const float t = jacobi_tan(fb - fa, g2);
+        const float c = rsqrtf(fmaf(t, t, 1.f)), sn = c * t;
+        const uint64_t c2 = pk2(c, c), s2 = pk2(sn, sn), n2 = pk2(-sn, -sn);
+#pragma unroll
+        for (int e = 0; e < RV; ++e) {
+          const int i = l8 + 8 * e;
+          if (i < q4) {
+            xa[i] = make_ulonglong2(fma2(c2, wx[e].x, mul2(n2, wy[e].x)), fma2(c2, wx[e].y, mul2(n2, wy[e].y)));
+            xb[i] = make_ulonglong2(fma2(c2, wy[e].x, mul2(s2, wx[e].x)), fma2(c2, wy[e].y, mul2(s2, wx[e].y)));
+            xa[q4 + i] = make_ulonglong2(fma2(c2, vx[e].x, mul2(n2, vy[e].x)), fma2(c2, vx[e].y, mul2(n2, vy[e].y)));
+            xb[q4 + i] = make_ulonglong2(fma2(c2, vy[e].x, mul2(s2, vx[e].x)), fma2(c2, vy[e].y, mul2(s2, vx[e].y)));
+          }
+        }
+        if (l8 == 0) rotated = 1;
+      }
+      __syncthreads();
+    }
+    const int done = (rotated == 0);
+    __syncthreads();
+    if (done) break;
+  }
+  // λ_j = v_j·w_j, columns sorted descending by |λ| (or λ), ties by index
+  const int nw = blockDim.x >> 5;
+  for (int j = warp; j < p; j += nw) {
+    float s = 0.f;
+    for (int i = lane; i < p; i += 32) s = fmaf(esm[j * cs + i], esm[j * cs + pr + i], s);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) lam_sh[j] = s;
+  }
+  __syncthreads();
+  for (int j = warp; j < p; j += nw) {
+    const float lj = lam_sh[j], kj = by_value ? lj : fabsf(lj);
+    int rk = 0;
+    for (int i = lane; i < p; i += 32) {
+      const float ki = by_value ? lam_sh[i] : fabsf(lam_sh[i]);
+      rk += (ki > kj || (ki == kj && i < j)) ? 1 : 0;
+    }
+    for (int o = 16; o > 0; o >>= 1) rk += __shfl_xor_sync(0xffffffffu, rk, o);
+    if (lane == 0) lam[rk] = (double)lj;
+    for (int i = lane; i < p; i += 32) Wout[i + (int64_t)rk * p] = (double)esm[j * cs + pr + i];
+  }
+  if (threadIdx.x == 0 && info) info[0] = sweep;
+}
+
+template <int RV>
+void eigh32_launch(tnad_ctx* c, const double* A, int p, int max_sweeps, double* lam, double* W, int* info, int by_value) {
+  static std::atomic<bool> attr{false};
+  if (!attr) {
+    TNAD_CK(cudaFuncSetAttribute(k_eigh32<RV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 2 * kEigh32MaxP * kEigh32MaxP * 4));
+    attr = true;
+  }
+  const int pr = (p + 3) & ~3, nb = (p + 1) / 2;
+  k_eigh32<RV><<<1, 32 * ((nb + 3) / 4), (size_t)p * 2 * pr * sizeof(float), c->stream>>>(A, p, max_sweeps, lam, W,
+                                                                                          info, by_value);
+}
+
 void eigh_small_prec(tnad_ctx* c, bool fp32, const double* A, int64_t p, double* W, double* lam, int max_sweeps,
                      int* dev_info, bool by_value) {
-  TNAD_REQUIRE(p >= 1 && p <= 256, TNAD_ERR_SHAPE, "eigh_small: p must be in [1,256]");
-  WsScope scope(c);
-  const size_t sm = (size_t)(p + 1) * p * (fp32 ? 4 : 8);
-  const size_t kMaxSm = 200 * 1024;
-  TNAD_REQUIRE(sm <= kMaxSm, TNAD_ERR_SHAPE, "eigh_small: matrix does not fit in shared memory");
-  static std::atomic<bool> attr32{false}, attr64{false};
-  // eigenvectors accumulate in global memory (L1-cached); H lives in shared memory
+  TNAD_REQUIRE(p >= 1 && p <= (fp32 ? kEigh32MaxP : 256), TNAD_ERR_SHAPE,
+               "eigh_small: p must be in [1,256] (FP32: [1,160])");
   KernelTimer kt(c, fp32 ? "eigh_f32" : "eigh_f64", 0.0);
   if (fp32) {
-    if (!attr32) {
-      TNAD_CK(cudaFuncSetAttribute(k_eigh_jacobi<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSm));
-      attr32 = true;
-    }
-    float* Z = ws_f(c, p * p);
-    k_eigh_jacobi<float><<<1, 512, sm, c->stream>>>(A, (int)p, max_sweeps, lam, W, Z, dev_info, by_value ? 1 : 0);
+    const int bv = by_value ? 1 : 0;
+    if (p <= 32)
+      eigh32_launch<1>(c, A, (int)p, max_sweeps, lam, W, dev_info, bv);
+    else if (p <= 64)
+      eigh32_launch<2>(c, A, (int)p, max_sweeps, lam, W, dev_info, bv);
+    else if (p <= 96)
+      eigh32_launch<3>(c, A, (int)p, max_sweeps, lam, W, dev_info, bv);
+    else if (p <= 128)
+      eigh32_launch<4>(c, A, (int)p, max_sweeps, lam, W, dev_info, bv);
+    else
+      eigh32_launch<5>(c, A, (int)p, max_sweeps, lam, W, dev_info, bv);
   } else {
+    WsScope scope(c);
+    const size_t sm = (size_t)(p + 1) * p * 8;
+    const size_t kMaxSm = 200 * 1024;
+    TNAD_REQUIRE(sm <= kMaxSm, TNAD_ERR_SHAPE, "eigh_small: matrix does not fit in shared memory");
+    static std::atomic<bool> attr64{false};
     if (!attr64) {
-      TNAD_CK(cudaFuncSetAttribute(k_eigh_jacobi<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSm));
+      TNAD_CK(cudaFuncSetAttribute(k_eigh_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSm));
       attr64 = true;
     }
+    // eigenvectors accumulate in global memory (L1-cached); H lives in shared memory
     double* Z = ws_d(c, p * p);
-    k_eigh_jacobi<double><<<1, 512, sm, c->stream>>>(A, (int)p, max_sweeps, lam, W, Z, dev_info, by_value ? 1 : 0);
+    k_eigh_jacobi<<<1, 512, sm, c->stream>>>(A, (int)p, max_sweeps, lam, W, Z, dev_info, by_value ? 1 : 0);
   }
   count_launch(c);
   check_launch(c, "eigh_small");
@@ -305,15 +568,21 @@ void eigh_small(tnad_ctx* c, const double* A, int64_t p, double* W, double* lam)
 // O = polar(X) for a χ×χ X (χ ≤ 128) by Newton–Schulz, O ← O·(3I − OᵀO)/2,
 // in FP32 in one CTA (the caller polishes in FP64); larger χ take polar_ns_gemm.  info[0] = 1 when the
 // result is orthogonal to 1e-4 (else the caller falls back to sign alignment).
-__global__ void k_polar_ns(const double* __restrict__ X, int m, int iters, double* __restrict__ O,
-                           int* __restrict__ info) {
-  extern __shared__ float psm[];
-  const int ld = m + 1;         // padded leading dimension (bank-conflict free)
-  float* A = psm;               // m×m current iterate
-  float* G = psm + m * ld;      // AᵀA
-  float* B = psm + 2 * m * ld;  // next iterate
+//
+// Each thread owns a 4×4 tile of the product (⌈m/4⌉² ≤ 1024 threads): two 16-byte
+// shared loads per 16 multiply-adds.  That needs the iterate in both layouts
+// (rows and columns contiguous) and uses that AᵀA is symmetric bit for bit; the
+// next iterate waits in registers until every tile has read the old one;
+// bound by the shared loads: 132 µs for m = 64 and 24 iterations (2×2 tiles with
+// 4-byte loads: 335 µs), the same sums in the same order.
+__global__ void __launch_bounds__(1024) k_polar_ns(const double* __restrict__ X, int m, int iters,
+                                                   double* __restrict__ O, int* __restrict__ info) {
+  extern __shared__ __align__(16) float psm[];
+  const int nt = (m + 3) >> 2, ld = 4 * nt + 4;  // 16-byte columns, one float4 of padding
+  float* A = psm;                                // A(i, k) at i + k·ld
+  float* At = psm + 4 * nt * ld;                 // A(k, i) at i + k·ld
+  float* G = psm + 8 * nt * ld;                  // AᵀA, symmetric
   __shared__ float red[32];
-  __shared__ int done;
   const int mm = m * m;
   // scale by 1/‖X‖_F·√m so that all singular values are ≤ 1 < √3
   float s = 0.f;
@@ -327,72 +596,90 @@ __global__ void k_polar_ns(const double* __restrict__ X, int m, int iters, doubl
     red[0] = t > 0.f ? sqrtf((float)m / t) : 1.f;
   }
   __syncthreads();
-  const float sc = fminf(red[0], 1.0f) * 0.999f;
-  for (int e = threadIdx.x; e < mm; e += blockDim.x) A[(e % m) + (e / m) * ld] = (float)X[e] * (red[0] > 1.f ? sc : 1.0f);
+  const float sc = red[0] > 1.f ? fminf(red[0], 1.0f) * 0.999f : 1.0f;
+  for (int e = threadIdx.x; e < 16 * nt * nt; e += blockDim.x) {
+    const int i = e % (4 * nt), k = e / (4 * nt);
+    const float v = (i < m && k < m) ? (float)X[i + k * m] * sc : 0.f;
+    A[i + k * ld] = v;
+    At[k + i * ld] = v;
+  }
   __syncthreads();
+  const bool act = (int)threadIdx.x < nt * nt;
+  const int i0 = 4 * ((int)threadIdx.x % nt), j0 = 4 * ((int)threadIdx.x / nt);
   float worst = 0.f;
   for (int it = 0; it <= iters; ++it) {
-    // G = AᵀA, and how far it is from I; each thread owns a 2×2 block of G
-    // (half the shared-memory loads per multiply-add of one element per thread)
+    // G = AᵀA, and how far it is from I
+    float g[4][4];
     float dev = 0.f;
-    const int mh = (m + 1) >> 1;
-    for (int e = threadIdx.x; e < mh * mh; e += blockDim.x) {
-      const int i0 = 2 * (e % mh), j0 = 2 * (e / mh);
-      const int i1 = min(i0 + 1, m - 1), j1 = min(j0 + 1, m - 1);
-      float g00 = 0.f, g01 = 0.f, g10 = 0.f, g11 = 0.f;
-      for (int k = 0; k < m; ++k) {
-        const float a0 = A[k + i0 * ld], a1 = A[k + i1 * ld], b0 = A[k + j0 * ld], b1 = A[k + j1 * ld];
-        g00 += a0 * b0;
-        g01 += a0 * b1;
-        g10 += a1 * b0;
-        g11 += a1 * b1;
+    if (act) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) g[a][b] = 0.f;
+#pragma unroll 4
+      for (int k = 0; k < 4 * nt; ++k) {  // rows beyond m are zero
+        const float4 x = *reinterpret_cast<const float4*>(&At[i0 + k * ld]);
+        const float4 y = *reinterpret_cast<const float4*>(&At[j0 + k * ld]);
+        const float xa[4] = {x.x, x.y, x.z, x.w}, ya[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) g[a][b] = fmaf(xa[a], ya[b], g[a][b]);
       }
-      G[i0 + j0 * ld] = g00;
-      G[i0 + j1 * ld] = g01;
-      G[i1 + j0 * ld] = g10;
-      G[i1 + j1 * ld] = g11;
-      dev = fmaxf(dev, fabsf(g00 - (i0 == j0 ? 1.f : 0.f)));
-      dev = fmaxf(dev, fabsf(g01 - (i0 == j1 ? 1.f : 0.f)));
-      dev = fmaxf(dev, fabsf(g10 - (i1 == j0 ? 1.f : 0.f)));
-      dev = fmaxf(dev, fabsf(g11 - (i1 == j1 ? 1.f : 0.f)));
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        *reinterpret_cast<float4*>(&G[i0 + (j0 + b) * ld]) = make_float4(g[0][b], g[1][b], g[2][b], g[3][b]);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+          if (i0 + a < m && j0 + b < m) dev = fmaxf(dev, fabsf(g[a][b] - (i0 + a == j0 + b ? 1.f : 0.f)));
+      }
     }
     for (int o = 16; o > 0; o >>= 1) dev = fmaxf(dev, __shfl_xor_sync(0xffffffffu, dev, o));
-    __syncthreads();
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dev;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      float t = 0.f;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = fmaxf(t, red[w]);
-      red[0] = t;
-      // all iterations run: stopping once AᵀA is at FP32 rounding (and polishing
-      // in FP64) changed the converged gauge enough to make the fixed-point
-      // adjoint's GMRES several times slower
-      done = it == iters ? 1 : 0;
+    // all iterations run: stopping once AᵀA is at FP32 rounding (and polishing
+    // in FP64) changed the converged gauge enough to make the fixed-point
+    // adjoint's GMRES several times slower
+    if (it == iters) {
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) worst = fmaxf(worst, red[w]);
+      break;
     }
-    __syncthreads();
-    worst = red[0];
-    if (done) break;
-    // B = A·(1.5 I − 0.5 G), 2×2 blocks per thread
-    for (int e = threadIdx.x; e < mh * mh; e += blockDim.x) {
-      const int i0 = 2 * (e % mh), j0 = 2 * (e / mh);
-      const int i1 = min(i0 + 1, m - 1), j1 = min(j0 + 1, m - 1);
-      float b00 = 0.f, b01 = 0.f, b10 = 0.f, b11 = 0.f;
-      for (int k = 0; k < m; ++k) {
-        const float a0 = A[i0 + k * ld], a1 = A[i1 + k * ld], g0 = G[k + j0 * ld], g1 = G[k + j1 * ld];
-        b00 += a0 * g0;
-        b01 += a0 * g1;
-        b10 += a1 * g0;
-        b11 += a1 * g1;
+    // A ← A·(1.5 I − 0.5 G)
+    float v[4][4];
+    if (act) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) g[a][b] = 0.f;
+#pragma unroll 4
+      for (int k = 0; k < 4 * nt; ++k) {
+        const float4 x = *reinterpret_cast<const float4*>(&A[i0 + k * ld]);
+        const float4 y = *reinterpret_cast<const float4*>(&G[j0 + k * ld]);  // G(k, j) = G(j, k)
+        const float xa[4] = {x.x, x.y, x.z, x.w}, ya[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) g[a][b] = fmaf(xa[a], ya[b], g[a][b]);
       }
-      B[i0 + j0 * ld] = 1.5f * A[i0 + j0 * ld] - 0.5f * b00;
-      B[i0 + j1 * ld] = 1.5f * A[i0 + j1 * ld] - 0.5f * b01;
-      B[i1 + j0 * ld] = 1.5f * A[i1 + j0 * ld] - 0.5f * b10;
-      B[i1 + j1 * ld] = 1.5f * A[i1 + j1 * ld] - 0.5f * b11;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const float4 x = *reinterpret_cast<const float4*>(&A[i0 + (j0 + b) * ld]);
+        v[0][b] = 1.5f * x.x - 0.5f * g[0][b];
+        v[1][b] = 1.5f * x.y - 0.5f * g[1][b];
+        v[2][b] = 1.5f * x.z - 0.5f * g[2][b];
+        v[3][b] = 1.5f * x.w - 0.5f * g[3][b];
+      }
     }
     __syncthreads();
-    float* t = A;
-    A = B;
-    B = t;
+    if (act) {
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        *reinterpret_cast<float4*>(&A[i0 + (j0 + b) * ld]) = make_float4(v[0][b], v[1][b], v[2][b], v[3][b]);
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+        *reinterpret_cast<float4*>(&At[j0 + (i0 + a) * ld]) = make_float4(v[a][0], v[a][1], v[a][2], v[a][3]);
+    }
+    __syncthreads();
   }
   for (int e = threadIdx.x; e < mm; e += blockDim.x) O[e] = (double)A[(e % m) + (e / m) * ld];
   if (threadIdx.x == 0) info[0] = worst < 1e-4f ? 1 : 0;
@@ -446,11 +733,13 @@ void polar_ns(tnad_ctx* c, const double* X, int64_t m, int iters, double* O, int
   }
   static std::atomic<bool> attr{false};
   if (!attr) {
-    TNAD_CK(cudaFuncSetAttribute(k_polar_ns, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 129 * 128 * 4));
+    TNAD_CK(cudaFuncSetAttribute(k_polar_ns, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 128 * 132 * 4));
     attr = true;
   }
   KernelTimer kt(c, "polar_ns", 0.0);
-  k_polar_ns<<<1, 1024, (size_t)3 * (m + 1) * m * 4, c->stream>>>(X, (int)m, iters, O, dev_info);
+  const int nt = ((int)m + 3) / 4;
+  k_polar_ns<<<1, (nt * nt + 31) / 32 * 32, (size_t)3 * 4 * nt * (4 * nt + 4) * 4, c->stream>>>(X, (int)m, iters, O,
+                                                                                                 dev_info);
   count_launch(c);
   check_launch(c, "polar_ns");
 }

@@ -32,6 +32,7 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include "fp64_fast.cuh"
 #include "tc_common.cuh"
 #include "tnad_internal.h"
 
@@ -90,56 +91,6 @@ __device__ __forceinline__ float wsum_f(float v) {
   return v;
 }
 
-// FP64 ↔ FP32 by integer operations: the conversion instructions take ~95
-// clocks of the FP64 pipe each, these about 20 and 11 (truncation; values below
-// the FP32 normal range become 0, above it are not expected: everything is
-// scaled to [2^-60, 2^100])
-__device__ __forceinline__ float d2f(double d) {
-  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d), a = hi & 0x7fffffffu;
-  const unsigned r = a < (897u << 20) ? 0u : (((a - (896u << 20)) << 3) | (lo >> 29));
-  return __uint_as_float(r | (hi & 0x80000000u));
-}
-
-__device__ __forceinline__ double f2d(float f) {
-  const unsigned b = __float_as_uint(f), a = b & 0x7fffffffu;
-  const unsigned hi = a ? (a >> 3) + (896u << 20) : 0u;
-  return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)(b << 29));
-}
-
-// FP32 quotient and square root to 1-2 ulp (they start Newton steps or only
-// decide angles): ~30 clocks instead of ~150 for the rounded ones
-__device__ __forceinline__ float fsqrt_ap(float x) {
-  float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
-// tan of the rotation that diagonalises [[a, g], [g, b]] with df = b − a, g2 = 2g (FP32)
-__device__ __forceinline__ float jacobi_tan(float df, float g2) {
-  if (fabsf(df) >= fabsf(g2)) {
-    const float w = __fdividef(g2, df);
-    return __fdividef(w, 1.f + fsqrt_ap(fmaf(w, w, 1.f)));
-  }
-  const float w = __fdividef(df, g2);
-  return __fdividef(copysignf(1.f, w), fabsf(w) + fsqrt_ap(fmaf(w, w, 1.f)));
-}
-
-// 1/√x by one cubic Newton (Halley) step from the FP32 value: relative error
-// (5/16)·e³ with e ~ 2e-7.  x inside the FP32 normal range.  Six FP64
-// instructions; sqrt() and a division take about 1300 clocks of the FP64 pipe.
-__device__ __forceinline__ double rsqrt_fast(double x) {
-  const double y = f2d(rsqrtf(d2f(x)));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
-// 1/x by two Newton steps from the FP32 value
-__device__ __forceinline__ double rcp_fast(double x) {
-  double y = f2d(__fdividef(1.f, d2f(x)));
-  y = fma(fma(-x, y, 1.0), y, y);
-  return fma(fma(-x, y, 1.0), y, y);
-}
-
 // Barrier over the CTAs of one problem.  CL: they form one thread-block cluster
 // (hardware barrier, 0.24 µs).  Otherwise a counter in global memory (1.1 µs
 // for 16 to 152 CTAs): the wait is bounded (2 s of %globaltimer); a CTA that
@@ -152,7 +103,7 @@ struct GridBar {
   int* dead;  // shared: 1 once a wait gave up
   __device__ bool sync() {
     if (CL) {
-      asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
       return true;
     }
     __syncthreads();
