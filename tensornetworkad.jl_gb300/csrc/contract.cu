@@ -1,10 +1,11 @@
 // Pairwise tensor contraction on the device: the role OMEinsum's ein"..." plays
 // in the reference (e.g. src/ctmrg.jl:130-140, src/variationalipeps.jl:52).
 // A contraction is mapped to one GEMM: free labels of A become the rows, free
-// labels of B the columns, shared labels the inner dimension.  Operands whose
-// memory order already matches a (transposed) matrix view are used in place;
-// otherwise one permutation kernel packs them.  The output is permuted only
-// when the requested label order interleaves A's and B's free labels.
+// labels of B the columns, shared labels the inner dimension.  The DFMA GEMM
+// reads and writes tensors in any label order.  For the tensor-core GEMMs,
+// operands whose memory order already matches a (transposed) matrix view are
+// used in place and others packed by one permutation kernel, and the output is
+// permuted when the requested label order interleaves A's and B's free labels.
 #include <cstring>
 #include <string>
 
@@ -37,6 +38,31 @@ static void perm_to(tnad_ctx* c, const Ten& T, const std::string& have, const st
   int perm[10];
   for (size_t k = 0; k < want.size(); ++k) perm[k] = (int)have.find(want[k]);
   permute(c, T, perm, out);
+}
+
+// Extents and strides of the labels `sel` (first fastest) in a tensor stored with
+// labels `have`; labels adjacent in memory merge.  false: more than kMax extents.
+static bool label_map(const int64_t* dim, const std::string& have, const std::string& sel, GemmMap& m) {
+  m.nd = 0;
+  for (char ch : sel) {
+    const size_t k = have.find(ch);
+    int64_t stride = 1;
+    for (size_t i = 0; i < k; ++i) stride *= dim[i];
+    if (dim[k] == 1) continue;
+    if (m.nd > 0 && m.str[m.nd - 1] * (int64_t)m.dim[m.nd - 1] == stride) {
+      m.dim[m.nd - 1] *= (unsigned)dim[k];
+      continue;
+    }
+    if (m.nd == GemmMap::kMax) return false;
+    m.dim[m.nd] = (unsigned)dim[k];
+    m.str[m.nd++] = stride;
+  }
+  if (m.nd == 0) {
+    m.nd = 1;
+    m.dim[0] = 1;
+    m.str[0] = 1;
+  }
+  return true;
 }
 
 void contract(tnad_ctx* c, int prec, const Ten& A0, const char* la0, const Ten& B0, const char* lb0, Ten& C,
@@ -85,6 +111,15 @@ void contract(tnad_ctx* c, int prec, const Ten& A0, const char* la0, const Ten& 
   };
   int64_t M = dims_of(A, la, Ml), N = dims_of(B, lb, Nl), K = dims_of(A, la, Kl);
 
+  if (M > 0 && N > 0 && K > 0 && gemm_is_f64(c, prec, M, N, K)) {
+    // DFMA tiles read and write the tensors in place, in any label order
+    GemmMap am, ak, bk, bn, cm, cn;
+    if (label_map(A->dim, la, Ml, am) && label_map(A->dim, la, Kl, ak) && label_map(B->dim, lb, Kl, bk) &&
+        label_map(B->dim, lb, Nl, bn) && label_map(C.dim, lc, Ml, cm) && label_map(C.dim, lc, Nl, cn)) {
+      gemm_f64_map(c, M, N, K, alpha, A->p, am, ak, B->p, bk, bn, beta, C.p, cm, cn);
+      return;
+    }
+  }
   WsScope scope(c);
   const double* Ap = A->p;
   char ta = 'N';

@@ -117,6 +117,8 @@ extern "C" int tnad_ctx_create(tnad_ctx** out, int device) {
     TNAD_CK(cudaMallocHost(&c->h_pin, 64 * sizeof(double)));
     TNAD_CK(cudaMalloc(&c->d_flag, 64 * sizeof(int)));
     TNAD_CK(cudaMallocHost(&c->h_flag, 64 * sizeof(int)));
+    TNAD_CK(cudaMalloc(&c->d_cnt, kGemmCounters * sizeof(int)));
+    TNAD_CK(cudaMemsetAsync(c->d_cnt, 0, kGemmCounters * sizeof(int), c->stream));
     TNAD_CK(cudaMemsetAsync(c->d_flag, 0, 64 * sizeof(int), c->stream));
     if (const char* f = std::getenv("TNAD_EIG_POLISH")) c->eig_refine = std::strcmp(f, "jacobi") != 0;
     if (const char* f = std::getenv("TNAD_JACOBI_BLOCKS")) c->jacobi_blocks = std::strcmp(f, "0") != 0;
@@ -142,6 +144,7 @@ extern "C" void tnad_ctx_destroy(tnad_ctx* c) {
   if (c->d_red) cudaFree(c->d_red);
   if (c->h_pin) cudaFreeHost(c->h_pin);
   if (c->d_flag) cudaFree(c->d_flag);
+  if (c->d_cnt) cudaFree(c->d_cnt);
   if (c->h_flag) cudaFreeHost(c->h_flag);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;

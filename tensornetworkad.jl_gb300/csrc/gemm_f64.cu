@@ -1,101 +1,227 @@
-// FP64 (DFMA) GEMM of the plain path.  Column-major, op(A)/op(B) ∈ {N,T}.
-// GB300 issues FP64 at a small fraction of its FP32/tensor rate, so this kernel
-// is bound by the DFMA pipe: register-tiled TM×TN micro-tiles over a BM×BN×16
-// shared-memory tile, deterministic split-K (fixed-order partial sums) when the
-// output has too few tiles to fill the 152 SMs.
+// FP64 (DFMA) GEMM of the plain path, on matrices or on tensors in any label
+// order: the row, column and inner index of each operand is a list of extents
+// and strides (GemmMap), so a pairwise contraction needs no permutation pass.
+//
+// GB300 retires 1.7 DFMA a clock and SM, so everything but that pipe is cheap:
+// index arithmetic, shared loads, even 16×16 tiles (one multiply-add per two
+// shared loads).  What matters is that the 152 SMs get equal shares: the tile
+// (16, 32 or 64 square) and the split of K are those with the least work on the
+// busiest SM (gemm_f64_plan).  A split product is summed by the CTA that
+// arrives last at its tile, in fixed order.  The next K slice is loaded to
+// registers while the current one is multiplied.
 #include <algorithm>
 
 #include "tnad_internal.h"
 
 namespace tnad {
 
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-    k_gemm_f64(int ta, int tb, int64_t M, int64_t N, int64_t K, int64_t kchunk, double alpha,
-               const double* __restrict__ A, int64_t lda, const double* __restrict__ B, int64_t ldb,
-               double beta, double* __restrict__ C, int64_t ldc, double* __restrict__ Cpart) {
-  constexpr int BK = 16;
-  constexpr int NT = (BM / TM) * (BN / TN);
-  __shared__ double As[BK][BM + 1];
-  __shared__ double Bs[BK][BN + 1];
-  const int tid = threadIdx.x;
-  const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
-  const int64_t kbeg = (int64_t)blockIdx.z * kchunk;
-  const int64_t kend = min(K, kbeg + kchunk);
-  const int tr = (tid % (BM / TM)) * TM;
-  const int tc = (tid / (BM / TM)) * TN;
-  double acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0;
+namespace {
 
-  for (int64_t k0 = kbeg; k0 < kend; k0 += BK) {
-    // A tile: op(A)(i,k), i in [m0,m0+BM), k in [k0,k0+BK)
-    for (int e = tid; e < BM * BK; e += NT) {
-      int i, k;
-      if (!ta) { i = e % BM; k = e / BM; } else { k = e % BK; i = e / BK; }
-      int64_t gi = m0 + i, gk = k0 + k;
-      double v = 0.0;
-      if (gi < M && gk < kend) v = !ta ? A[gi + gk * lda] : A[gk + gi * lda];
-      As[k][i] = v;
+__device__ __forceinline__ int64_t map_off(const GemmMap& m, unsigned i) {
+  if (m.nd == 1) return (int64_t)i * m.str[0];
+  int64_t o = 0;
+#pragma unroll
+  for (int d = 0; d < GemmMap::kMax; ++d) {
+    if (d + 1 < m.nd) {
+      const unsigned q = i / m.dim[d];
+      o += (int64_t)(i - q * m.dim[d]) * m.str[d];
+      i = q;
+    } else if (d + 1 == m.nd) {
+      o += (int64_t)i * m.str[d];
     }
-    for (int e = tid; e < BN * BK; e += NT) {
-      int j, k;
-      if (!tb) { k = e % BK; j = e / BK; } else { j = e % BN; k = e / BN; }
-      int64_t gj = n0 + j, gk = k0 + k;
-      double v = 0.0;
-      if (gj < N && gk < kend) v = !tb ? B[gk + gj * ldb] : B[gj + gk * ldb];
-      Bs[k][j] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      double a[TM], b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[k][tr + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Bs[k][tc + j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
   }
-  if (Cpart) {
-    double* P = Cpart + (int64_t)blockIdx.z * M * N;
+  return o;
+}
+
+struct GemmArgs {
+  unsigned M, N, K, kchunk;
+  int ks;
+  double alpha, beta;
+  const double *A, *B;
+  double *C, *part;
+  int* cnt;
+  GemmMap am, ak, bk, bn, cm, cn;
+  int a_rows, b_rows;  // lanes run along the rows (columns) of the tile, else along K
+};
+
+template <int BM>
+__global__ void __launch_bounds__(256) k_gemm_f64(const GemmArgs g) {
+  constexpr int BK = 16, T = BM / 16;  // T×T outputs and T loads per operand and thread
+  __shared__ double As[2][BK][BM + 1];
+  __shared__ double Bs[2][BK][BM + 1];
+  __shared__ int last;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const unsigned m0 = blockIdx.x * BM, n0 = blockIdx.y * BM;
+  const unsigned kbeg = blockIdx.z * g.kchunk, kend = min(g.K, kbeg + g.kchunk);
+  // this thread's elements of a slice: (row ai[q], inner ak[q]) and (inner, column)
+  int ai[T], aK[T], bi[T], bK[T];
+  int64_t ao[T], bo[T];
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+  for (int q = 0; q < T; ++q) {
+    ai[q] = g.a_rows ? tid % BM : ty + 16 * q;
+    aK[q] = g.a_rows ? tid / BM + (256 / BM) * q : tx;
+    bi[q] = g.b_rows ? tid % BM : ty + 16 * q;
+    bK[q] = g.b_rows ? tid / BM + (256 / BM) * q : tx;
+    ao[q] = m0 + ai[q] < g.M ? map_off(g.am, m0 + ai[q]) : -1;
+    bo[q] = n0 + bi[q] < g.N ? map_off(g.bn, n0 + bi[q]) : -1;
+  }
+  double ra[T], rb[T], acc[T][T];
+  auto load = [&](unsigned k0) {
 #pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        int64_t gi = m0 + tr + i, gj = n0 + tc + j;
-        if (gi < M && gj < N) P[gi + gj * M] = acc[i][j];
+    for (int q = 0; q < T; ++q) {
+      const unsigned ka = k0 + aK[q], kb = k0 + bK[q];
+      ra[q] = (ao[q] >= 0 && ka < kend) ? g.A[ao[q] + map_off(g.ak, ka)] : 0.0;
+      rb[q] = (bo[q] >= 0 && kb < kend) ? g.B[bo[q] + map_off(g.bk, kb)] : 0.0;
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < T; ++i)
+#pragma unroll
+    for (int j = 0; j < T; ++j) acc[i][j] = 0.0;
+  load(kbeg);
+  int buf = 0;
+  for (unsigned k0 = kbeg; k0 < kend; k0 += BK, buf ^= 1) {
+#pragma unroll
+    for (int q = 0; q < T; ++q) {
+      As[buf][aK[q]][ai[q]] = ra[q];
+      Bs[buf][bK[q]][bi[q]] = rb[q];
+    }
+    __syncthreads();  // one barrier a slice: the other buffer was read before the last one
+    if (k0 + BK < kend) load(k0 + BK);
+    const int kn = min((unsigned)BK, kend - k0);
+    if (kn == BK) {
+#pragma unroll
+      for (int k = 0; k < BK; ++k) {
+        double a[T], b[T];
+#pragma unroll
+        for (int i = 0; i < T; ++i) a[i] = As[buf][k][tx + 16 * i];
+#pragma unroll
+        for (int j = 0; j < T; ++j) b[j] = Bs[buf][k][ty + 16 * j];
+#pragma unroll
+        for (int i = 0; i < T; ++i)
+#pragma unroll
+          for (int j = 0; j < T; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
       }
-  } else {
+    } else {
+      for (int k = 0; k < kn; ++k) {
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+        for (int i = 0; i < T; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        int64_t gi = m0 + tr + i, gj = n0 + tc + j;
-        if (gi < M && gj < N) {
-          double v = alpha * acc[i][j];
-          C[gi + gj * ldc] = beta == 0.0 ? v : v + beta * C[gi + gj * ldc];
-        }
+          for (int j = 0; j < T; ++j) acc[i][j] = fma(As[buf][k][tx + 16 * i], Bs[buf][k][ty + 16 * j], acc[i][j]);
       }
+    }
+  }
+  if (g.ks > 1) {
+    const int64_t tiles = (int64_t)gridDim.x * gridDim.y, tile = blockIdx.x + (int64_t)gridDim.x * blockIdx.y;
+    double* P = g.part + ((int64_t)blockIdx.z * tiles + tile) * (BM * BM);
+#pragma unroll
+    for (int i = 0; i < T; ++i)
+#pragma unroll
+      for (int j = 0; j < T; ++j) __stcg(&P[tid + 256 * (i * T + j)], acc[i][j]);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(&g.cnt[tile], 1) == g.ks - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+#pragma unroll
+    for (int i = 0; i < T; ++i)
+#pragma unroll
+      for (int j = 0; j < T; ++j) acc[i][j] = 0.0;
+    for (int z = 0; z < g.ks; ++z) {
+      const double* Pz = g.part + ((int64_t)z * tiles + tile) * (BM * BM);
+#pragma unroll
+      for (int i = 0; i < T; ++i)
+#pragma unroll
+        for (int j = 0; j < T; ++j) acc[i][j] += __ldcg(&Pz[tid + 256 * (i * T + j)]);
+    }
+    if (tid == 0) g.cnt[tile] = 0;  // for the next product on this stream
+  }
+#pragma unroll
+  for (int j = 0; j < T; ++j) {
+    const unsigned gj = n0 + ty + 16 * j;
+    if (gj >= g.N) continue;
+    const int64_t cj = map_off(g.cn, gj);
+#pragma unroll
+    for (int i = 0; i < T; ++i) {
+      const unsigned gi = m0 + tx + 16 * i;
+      if (gi >= g.M) continue;
+      double* c = g.C + cj + map_off(g.cm, gi);
+      const double v = g.alpha * acc[i][j];
+      *c = g.beta == 0.0 ? v : v + g.beta * (*c);
+    }
   }
 }
 
-__global__ void k_splitk_reduce(int64_t M, int64_t N, int ks, const double* __restrict__ P, double alpha,
-                                double beta, double* __restrict__ C, int64_t ldc) {
-  int64_t MN = M * N;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < MN; e += (int64_t)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int z = 0; z < ks; ++z) s += P[e + z * MN];
-    int64_t i = e % M, j = e / M;
-    double v = alpha * s;
-    C[i + j * ldc] = beta == 0.0 ? v : v + beta * C[i + j * ldc];
+// Tile and split with the least time on the busiest SM, in clocks: its share of
+// the tiles at 1.7 DFMA a clock, ~1200 for a CTA's first loads and stores (partly
+// hidden where an SM holds several), ~2500 more where K is split (partials,
+// counter, the sum).  Measured: 32×32×32 (one 32×32 tile, K in two halves and a
+// second kernel before) 11.6 → see DESIGN's table of cases; 1024³ stays at the pipe's limit.
+void gemm_f64_plan(int sms, int64_t M, int64_t N, int64_t K, int* tile, int* splits) {
+  double best = 1e300;
+  for (int t : {64, 32, 16}) {
+    const int64_t tiles = ((M + t - 1) / t) * ((N + t - 1) / t);
+    if (t < 64 && (N + t - 1) / t > 65535) continue;  // grid.y
+    const int64_t kmax = tiles <= kGemmCounters ? std::min<int64_t>(64, std::max<int64_t>(1, K / 16)) : 1;
+    for (int64_t ks = 1; ks <= kmax; ++ks) {
+      const int64_t kc = ((K + ks - 1) / ks + 15) / 16 * 16;
+      const int64_t per_sm = (tiles * ((K + kc - 1) / kc) + sms - 1) / sms;
+      const double cost =
+          (double)per_sm * ((double)t * t * (double)std::min(kc, K) / 1.7 + 400.0) + 1200.0 + (ks > 1 ? 2500.0 + 60.0 * ks : 0.0);
+      if (cost < best) {
+        best = cost;
+        *tile = t;
+        *splits = (int)ks;
+      }
+      if (tiles * ks > 8 * (int64_t)sms) break;
+    }
   }
+}
+
+}  // namespace
+
+void gemm_f64_map(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, const GemmMap& am,
+                  const GemmMap& ak, const double* B, const GemmMap& bk, const GemmMap& bn, double beta, double* C,
+                  const GemmMap& cm, const GemmMap& cn) {
+  TNAD_REQUIRE(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), TNAD_ERR_ARG, "gemm_f64: size");
+  int tile = 64, ks = 1;
+  gemm_f64_plan(c->sm_count, M, N, K, &tile, &ks);
+  GemmArgs g;
+  g.M = (unsigned)M;
+  g.N = (unsigned)N;
+  g.K = (unsigned)K;
+  const int64_t kc = ks > 1 ? ((K + ks - 1) / ks + 15) / 16 * 16 : K;
+  g.kchunk = (unsigned)kc;
+  g.ks = (int)((K + kc - 1) / kc);
+  g.alpha = alpha;
+  g.beta = beta;
+  g.A = A;
+  g.B = B;
+  g.C = C;
+  g.am = am;
+  g.ak = ak;
+  g.bk = bk;
+  g.bn = bn;
+  g.cm = cm;
+  g.cn = cn;
+  g.a_rows = am.str[0] == 1 || ak.str[0] != 1;
+  g.b_rows = bn.str[0] == 1 || bk.str[0] != 1;
+  g.cnt = c->d_cnt;
+  WsScope scope(c);
+  const int64_t tm = (M + tile - 1) / tile, tn = (N + tile - 1) / tile;
+  TNAD_REQUIRE(tn <= 65535, TNAD_ERR_ARG, "gemm_f64: too many columns");
+  g.part = g.ks > 1 ? ws_d(c, (int64_t)g.ks * tm * tn * tile * tile) : nullptr;
+  const dim3 grid((unsigned)tm, (unsigned)tn, (unsigned)g.ks);
+  KernelTimer kt(c, "gemm_f64", 2.0 * (double)M * (double)N * (double)K);
+  if (tile == 64)
+    k_gemm_f64<64><<<grid, 256, 0, c->stream>>>(g);
+  else if (tile == 32)
+    k_gemm_f64<32><<<grid, 256, 0, c->stream>>>(g);
+  else
+    k_gemm_f64<16><<<grid, 256, 0, c->stream>>>(g);
+  count_launch(c);
+  check_launch(c, "gemm_f64");
 }
 
 // Matrix-vector products (N = 1), the Gram–Schmidt steps of GMRES: a tiled
@@ -157,6 +283,14 @@ __global__ void k_gemv_t_sum(int64_t M, int nchunk, const double* __restrict__ p
   y[i] = beta == 0.0 ? v : v + beta * y[i];
 }
 
+static GemmMap map1(int64_t n, int64_t stride) {
+  GemmMap m;
+  m.nd = 1;
+  m.dim[0] = (unsigned)n;
+  m.str[0] = stride;
+  return m;
+}
+
 void gemm_f64(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, double alpha, const double* A,
               int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc) {
   if (M <= 0 || N <= 0) return;
@@ -192,43 +326,8 @@ void gemm_f64(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, do
     check_launch(c, "gemv_f64");
     return;
   }
-  // 64×64 tiles when they alone give half the SMs work, 32×32 otherwise
-  const int64_t tiles64 = ((M + 63) / 64) * ((N + 63) / 64);
-  const bool big = (M >= 64 && N >= 64 && tiles64 >= c->sm_count / 2);
-  const int BM = big ? 64 : 32, BN = big ? 64 : 32;
-  int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  // Each SM retires only ~2 DFMA per clock, so a GEMM whose output has fewer
-  // tiles than SMs is split along K until about two CTAs per SM are busy
-  // (chunks of at least 16 K values; partial sums reduced in fixed order).
-  int ks = 1;
-  if (tiles < 2 * c->sm_count && K >= 32) {
-    int64_t want = (2 * c->sm_count + tiles - 1) / tiles;
-    int64_t cap = K / 16;
-    ks = (int)std::max<int64_t>(1, std::min<int64_t>({want, cap, 128}));
-  }
-  int64_t kchunk = (K + ks - 1) / ks;
-  kchunk = (kchunk + 15) / 16 * 16;
-  ks = (int)((K + kchunk - 1) / kchunk);
-  WsScope scope(c);
-  double* part = nullptr;
-  if (ks > 1) part = ws_d(c, (int64_t)ks * M * N);
-  dim3 grid((unsigned)((M + BM - 1) / BM), (unsigned)((N + BN - 1) / BN), (unsigned)ks);
-  KernelTimer kt(c, "gemm_f64", 2.0 * (double)M * (double)N * (double)K);
-  if (big)
-    k_gemm_f64<64, 64, 4, 4><<<grid, 256, 0, c->stream>>>(ita, itb, M, N, K, kchunk, alpha, A, lda, B, ldb, beta, C,
-                                                          ldc, part);
-  else
-    k_gemm_f64<32, 32, 2, 2><<<grid, 256, 0, c->stream>>>(ita, itb, M, N, K, kchunk, alpha, A, lda, B, ldb, beta, C,
-                                                          ldc, part);
-  count_launch(c);
-  check_launch(c, "gemm_f64");
-  if (ks > 1) {
-    int64_t MN = M * N;
-    int nb = (int)std::min<int64_t>((MN + 255) / 256, 4096);
-    k_splitk_reduce<<<nb, 256, 0, c->stream>>>(M, N, ks, part, alpha, beta, C, ldc);
-    count_launch(c);
-    check_launch(c, "splitk_reduce");
-  }
+  gemm_f64_map(c, M, N, K, alpha, A, map1(M, ita ? lda : 1), map1(K, ita ? 1 : lda), B, map1(K, itb ? ldb : 1),
+               map1(N, itb ? 1 : ldb), beta, C, map1(M, 1), map1(N, ldc));
 }
 
 void gemm(tnad_ctx* c, int prec, char ta, char tb, int64_t M, int64_t N, int64_t K, double alpha, const double* A,

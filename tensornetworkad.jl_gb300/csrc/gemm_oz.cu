@@ -384,6 +384,11 @@ void oz_prepare(tnad_ctx* c) {
 // below this many multiply-adds the DFMA GEMM is as fast (launch-bound)
 static const double kOzMinWork = 4.0e6;
 
+bool gemm_is_f64(const tnad_ctx* c, int prec, int64_t M, int64_t N, int64_t K) {
+  return prec == TNAD_PREC_FP64 &&
+         (!c->fp64_tc || !c->tc_ok || (double)M * (double)N * (double)K < kOzMinWork);
+}
+
 void gemm_fp64tc(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, double alpha, const double* A,
                  int64_t lda, const double* B, int64_t ldb, double beta, double* Cm, int64_t ldc, bool always) {
   if (M <= 0 || N <= 0) return;

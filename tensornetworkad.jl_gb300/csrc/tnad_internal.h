@@ -81,6 +81,7 @@ struct tnad_ctx {
   double* h_pin = nullptr;  // pinned host mirror (64 doubles)
   int* d_flag = nullptr;    // device flags / counters (64 ints)
   int* h_flag = nullptr;    // pinned host mirror of the flags
+  int* d_cnt = nullptr;     // arrival counters of split products (kGemmCounters, zero between launches)
   bool tc_ok = false;       // tcgen05 GEMM path available (sm_100 family)
   // One-shot fault injection for the failure-path tests, set from the
   // environment variable TNAD_TEST_FAULT when the context is created:
@@ -121,6 +122,8 @@ struct tnad_ctx {
 };
 
 namespace tnad {
+
+constexpr int64_t kGemmCounters = 4096;  // tiles of a product whose K may be split
 
 enum { kFaultNone = 0, kFaultTcWithhold = 1, kFaultJacobiCap = 2 };
 
@@ -212,6 +215,19 @@ void normalize_inplace(tnad_ctx* c, double* x, int64_t n, double* dev_norm_out);
 void gemm_f64(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, double alpha,
               const double* A, int64_t lda, const double* B, int64_t ldb, double beta, double* C,
               int64_t ldc);
+// The same on tensors: element (i, k) of A at A[am(i) + ak(k)], where a map splits
+// its index into nd extents (the first fastest) with a stride each; likewise B and C.
+struct GemmMap {
+  static constexpr int kMax = 6;
+  int nd = 0;
+  unsigned dim[kMax] = {0, 0, 0, 0, 0, 0};
+  int64_t str[kMax] = {0, 0, 0, 0, 0, 0};
+};
+void gemm_f64_map(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, const GemmMap& am,
+                  const GemmMap& ak, const double* B, const GemmMap& bk, const GemmMap& bn, double beta, double* C,
+                  const GemmMap& cm, const GemmMap& cn);
+// Whether a product of this size runs as DFMA tiles under `prec` on this context.
+bool gemm_is_f64(const tnad_ctx* c, int prec, int64_t M, int64_t N, int64_t K);
 // Same contract, 3xTF32 on tcgen05 tensor cores with FP32 accumulation.
 void gemm_tf32x3(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, double alpha,
                  const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
