@@ -400,7 +400,7 @@ def run_gb300(args):
                         f"{pk_kind} bf16 burst (MEASURED_PEAKS.json)"),
         "gemm_f64": ("k_gemm_f64 / k_gemv (register-tiled DFMA GEMM, matrix-vector products)", "fp64", 1.0,
                      FP64_NOMINAL_TFLOPS, nominal),
-        "jacobi_round_f32": ("k_jacobi_block<64> (FP32 Jacobi sweeps of the 1024x1024 corner's symmetric SVD, "
+        "jacobi_round_f32": ("k_sweeps32<EIG> (FP32 Jacobi sweeps of the 1024x1024 corner's symmetric SVD, "
                              "eigenvalue rule, block rounds of 4 columns)", "fp32", 1.0, FP32_NOMINAL_TFLOPS, nominal),
         "jacobi_round_small": ("k_jacobi_round_cta<2, double> (FP64 rounds of the p x p Rayleigh-Ritz problems of the "
                                "subspace solver)", "fp64", 1.0, FP64_NOMINAL_TFLOPS, nominal),

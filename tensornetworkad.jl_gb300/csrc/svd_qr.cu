@@ -23,7 +23,7 @@
 // Measured on one GB300 against FP64 element rounds (k_jacobi_round_cta): TRG at
 // χ = 20, 7 steps with gradient 704 → 28 ms; D=3, χ=36 energy and gradient (n =
 // 324) 349 → 65 ms; one n = 80 decomposition 4.9 → 1.4 ms, n = 255 26.7 → 5.9 ms.
-// At n = 324 the first QR takes 2.0 ms, the FP32 sweeps 3.4, the FP64 ones 2.6.
+// At n = 324 the first QR takes 2.0 ms, the FP32 sweeps 2.2, the FP64 ones 2.3.
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
@@ -44,6 +44,7 @@ constexpr int kMaxSvdRows = 1024;
 constexpr int kSvdSweeps = 60;
 constexpr int kPreMin = 24;         // columns from which FP32 sweeps precede the FP64 ones
 constexpr int kPreSweeps = 20;
+constexpr int kEigSweeps = 30;      // cap of the corner's FP32 sweeps (their result is refined or replaced)
 constexpr float kPreCos = 1e-3f;    // a sweep that rotated no larger |cos| leaves ~1e-6: hand over
 constexpr int kScaleExp = 40;  // the largest |entry| is scaled to 2^40: squared norms of
                                // columns down to ½ε of it stay inside the FP32 range
@@ -52,7 +53,7 @@ constexpr int kScaleExp = 40;  // the largest |entry| is scaled to 2^40: squared
 // (0: none), barrier counter of each of the three kernels, rotations per sweep
 // and the largest |cos| of a rotated pair per sweep (float bits).
 enum { kiRank = 0, kiBad = 1, kiSweeps = 2, kiExp = 3, kiErr = 4, kiPre = 5, kiBar = 8, kiRot = 16, kiCos = 16 + kSvdSweeps,
-       kiTan = 16 + 2 * kSvdSweeps, kiRot32 = 16 + 3 * kSvdSweeps, kiCos32 = kiRot32 + kPreSweeps, kiCount = kiCos32 + kPreSweeps };
+       kiTan = 16 + 2 * kSvdSweeps, kiRot32 = 16 + 3 * kSvdSweeps, kiCos32 = kiRot32 + kEigSweeps, kiCount = kiCos32 + kEigSweeps };
 
 struct SvdProb {
   const double* A;
@@ -76,6 +77,7 @@ struct SvdArgs {
   float trunc;     // rank cut relative to the first pivot
   double tol;      // Jacobi: |cos| above which a pair rotates (FP64 and FP32 sweeps)
   float tol32;
+  const double* fro2;  // EIG: ‖A‖²_F
   int max_sweeps;
 };
 
@@ -109,7 +111,8 @@ struct GridBar {
     __syncthreads();
     tgt += G;
     if (threadIdx.x == 0) {
-      __threadfence();
+      // release and acquire at GPU scope; the CTA barriers around them order the
+      // other threads' accesses
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
       unsigned v, spins = 0;
       const uint64_t t0 = tc::gtime();
@@ -122,7 +125,6 @@ struct GridBar {
           break;
         }
       }
-      __threadfence();
     }
     __syncthreads();
     return *dead == 0;
@@ -556,356 +558,280 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// FP32 sweeps that precede the FP64 ones (n ≥ kPreMin): the same tournament on
-// an FP32 copy of X with blocks of four columns (two cross barriers fewer per
-// column pair than blocks of two; FP32 arithmetic is 64 times as wide, so a
-// round is barrier and L2 latency either way).  One-sided rotations keep the
-// relative accuracy of graded columns in FP32 too, so X·V comes out with
-// |cos| ~ 1e-6 between all columns, small ones included.
+// FP32 Jacobi sweeps, one launch: they precede the FP64 sweeps (n ≥ kPreMin) and
+// start the corner's product refinement (EIG).  Blocks of 8 columns; CTA k takes
+// the block pair of the round from L2 to shared memory (16-byte cp.async), W and
+// V of 16 columns, rotates the 64 cross pairs in 8 inner rounds of 8 disjoint
+// pairs (in a sweep's first round the pairs inside the blocks too, 7 inner
+// rounds), and stores them; one barrier a round, n/8 − 1 rounds a sweep.  WP
+// warps per pair, RV 16-byte chunks per lane and column, packed arithmetic
+// (fma.rn.f32x2).  Blocks this long because a round's barrier and L2 exchange
+// cost as much as ~6 inner rounds; longer ones leave too few CTAs at n = 1024.
+//
+// Rules: one-sided (a, b, g from W's columns, relative: graded columns keep
+// their relative accuracy in FP32, so X·V comes out with |cos| ~ 1e-6 between
+// all columns, small ones included), ended by a sweep that rotated no |cos|
+// above kPreCos; EIG: the 2×2 block of VᵀXV for symmetric X (±λ pairs are not
+// mixed), absolute threshold, ended by a sweep with at most 16n rotations.
+//
+// A group keeps its column of P in registers through the inner rounds, so that
+// shared memory carries Q's columns only (128 bytes a clock limit n = 1024).
+// Measured: n = 1024 15 ms for 9-10 sweeps, as 255 launches a sweep of 4-column
+// blocks 17.9; D=3, χ=36 energy and gradient (n = 324) 64 → 56 ms against one
+// 16-CTA cluster with scalar loads.
 // ---------------------------------------------------------------------------
-template <int RJ>
-__global__ void __launch_bounds__(256) k_svd_sweeps32(SvdArgs a) {
+__device__ __forceinline__ uint64_t pk2(float a, float b) {
+  return ((uint64_t)__float_as_uint(b) << 32) | __float_as_uint(a);
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float hsum2(uint64_t a) {
+  return __uint_as_float((unsigned)a) + __uint_as_float((unsigned)(a >> 32));
+}
+
+template <int B, int RV, int WP, bool EIG, bool CL>
+__global__ void __launch_bounds__(32 * B * WP) k_sweeps32(SvdArgs a) {
+  constexpr int LP = 32 * WP, NW = B * WP;  // lanes per pair, warps
   extern __shared__ __align__(16) unsigned char sm_raw[];
   const SvdProb& q = a.p[blockIdx.y];
-  const int rc = q.info[kiRank];
-  const bool two = a.second || rc < a.n;
+  const int rc = EIG ? a.n : q.info[kiRank];
+  const bool two = !EIG && (a.second || rc < a.n);
   const int mx = two ? rc : a.n;
-  const int nreal = (rc + 3) >> 2, NB = nreal + (nreal & 1);
+  const int nreal = (rc + B - 1) / B, NB = nreal + (nreal & 1);
   const int active = NB >> 1, cta = blockIdx.x;
-  if (cta >= active || q.info[kiErr]) return;
+  if (q.info[kiErr]) return;
+  if (!CL && cta >= active) return;  // a cluster's idle CTAs keep to its barriers
   float* W = q.W32;
   float* V = q.V32;
   const int ld = a.ld32;
-  const int ldw = (mx + 3) & ~3, ldv = (rc + 3) & ~3, cst = ldw + ldv;
-  float* sm = reinterpret_cast<float*>(sm_raw);  // 8 columns: W rows, then V rows
-  __shared__ float red[4][2][3];
+  const int q4 = (mx + 3) >> 2, v4 = (rc + 3) >> 2, c4 = q4 + v4;  // 16-byte chunks of W, V, a column
+  ulonglong2* sm = reinterpret_cast<ulonglong2*>(sm_raw);          // 16 columns: W rows, then V rows
+  __shared__ float red[B][WP][3];
   __shared__ int dead, nrot, cosmax;
   if (threadIdx.x == 0) dead = nrot = cosmax = 0;
   __syncthreads();
-  GridBar<false> bar{reinterpret_cast<unsigned*>(q.info + kiBar + 3), 0u, (unsigned)active, q.info + kiErr, &dead};
-  const double* X = two ? q.X2 : q.X;
-  for (int j = cta; j < rc; j += active) {
-    for (int i = threadIdx.x; i < mx; i += blockDim.x)
-      __stcg(&W[i + (int64_t)j * ld], d2f(X[i + (int64_t)j * a.ldx]));
-    for (int i = threadIdx.x; i < rc; i += blockDim.x) __stcg(&V[i + (int64_t)j * ld], i == j ? 1.f : 0.f);
+  GridBar<CL> bar{reinterpret_cast<unsigned*>(q.info + kiBar + 3), 0u, (unsigned)active, q.info + kiErr, &dead};
+  const double* X = EIG ? q.A : (two ? q.X2 : q.X);
+  for (int j = cta; j < rc; j += max(active, 1)) {
+    for (int i = threadIdx.x; i < 4 * q4; i += blockDim.x)
+      __stcg(&W[i + (int64_t)j * ld], i < mx ? d2f(X[i + (int64_t)j * a.ldx]) : 0.f);
+    for (int i = threadIdx.x; i < 4 * v4; i += blockDim.x) __stcg(&V[i + (int64_t)j * ld], i == j ? 1.f : 0.f);
   }
   if (!bar.sync()) return;
-  const int grp = threadIdx.x >> 6, lt = threadIdx.x & 63, wip = (threadIdx.x >> 5) & 1, lane = threadIdx.x & 31;
+  const float thr_abs = EIG ? 2.f * FLT_EPSILON * sqrtf((float)a.fro2[0]) : 0.f;
+  const int grp = threadIdx.x / LP, lt = threadIdx.x % LP, wip = (threadIdx.x >> 5) % WP, lane = threadIdx.x & 31;
 
-  auto process = [&](int x, int y, bool present) {
-    float* wx = sm + (int64_t)x * cst;
-    float* wy = sm + (int64_t)y * cst;
-    float u[RJ], v[RJ];
+  int my_rot = 0;  // of this thread's pairs, in the current sweep
+  float my_cos = 0.f;
+  // rotation of the pair (W, V) = (wx, vx), (wy, vy) held in registers; true when
+  // it rotates.  Every thread of the pair returns the same.
+  const ulonglong2 z = make_ulonglong2(0, 0);
+  auto rotate = [&](ulonglong2 (&wx)[RV], ulonglong2 (&vx)[RV], ulonglong2 (&wy)[RV], ulonglong2 (&vy)[RV],
+                    bool present) -> bool {
+    float na = 0.f, nb = 0.f, g2 = 0.f;  // a, b, 2g
     if (present) {
-      float na = 0.f, nb = 0.f, g = 0.f;
+      uint64_t sa = 0, sb = 0, sg = 0;
 #pragma unroll
-      for (int e = 0; e < RJ; ++e) {
-        const int i = lt + 64 * e;
-        u[e] = i < mx ? wx[i] : 0.f;
-        v[e] = i < mx ? wy[i] : 0.f;
+      for (int e = 0; e < RV; ++e) {
+        if (EIG) {
+          sa = fma2(vx[e].x, wx[e].x, sa);
+          sb = fma2(vy[e].x, wy[e].x, sb);
+          sg = fma2(vx[e].x, wy[e].x, sg);
+          sg = fma2(vy[e].x, wx[e].x, sg);
+          sa = fma2(vx[e].y, wx[e].y, sa);
+          sb = fma2(vy[e].y, wy[e].y, sb);
+          sg = fma2(vx[e].y, wy[e].y, sg);
+          sg = fma2(vy[e].y, wx[e].y, sg);
+        } else {
+          sa = fma2(wx[e].x, wx[e].x, sa);
+          sb = fma2(wy[e].x, wy[e].x, sb);
+          sg = fma2(wx[e].x, wy[e].x, sg);
+          sa = fma2(wx[e].y, wx[e].y, sa);
+          sb = fma2(wy[e].y, wy[e].y, sb);
+          sg = fma2(wx[e].y, wy[e].y, sg);
+        }
       }
-#pragma unroll
-      for (int e = 0; e < RJ; ++e) {
-        na = fmaf(u[e], u[e], na);
-        nb = fmaf(v[e], v[e], nb);
-        g = fmaf(u[e], v[e], g);
-      }
+      na = hsum2(sa);
+      nb = hsum2(sb);
+      g2 = EIG ? hsum2(sg) : 2.f * hsum2(sg);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         na += __shfl_xor_sync(0xffffffffu, na, o);
         nb += __shfl_xor_sync(0xffffffffu, nb, o);
-        g += __shfl_xor_sync(0xffffffffu, g, o);
+        g2 += __shfl_xor_sync(0xffffffffu, g2, o);
       }
-      if (lane == 0) {
+      if (WP > 1 && lane == 0) {
         red[grp][wip][0] = na;
         red[grp][wip][1] = nb;
-        red[grp][wip][2] = g;
+        red[grp][wip][2] = g2;
       }
     }
-    asm volatile("bar.sync %0, 64;" ::"r"(grp + 1) : "memory");
-    if (present) {
-      const float na = red[grp][0][0] + red[grp][1][0], nb = red[grp][0][1] + red[grp][1][1];
-      const float g = red[grp][0][2] + red[grp][1][2];
-      const float nn = fsqrt_ap(na) * fsqrt_ap(nb);
-      if (fabsf(g) > a.tol32 * nn) {
-        const float t = jacobi_tan(nb - na, 2.f * g);
-        const float cs = rsqrtf(fmaf(t, t, 1.f)), sn = cs * t;
+    if (WP > 1) {
+      asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(LP) : "memory");
+      if (present) {
+        na = nb = g2 = 0.f;
 #pragma unroll
-        for (int e = 0; e < RJ; ++e) {
-          const int i = lt + 64 * e;
-          if (i < mx) {
-            wx[i] = cs * u[e] - sn * v[e];
-            wy[i] = sn * u[e] + cs * v[e];
-          }
-        }
-        float* vx = wx + ldw;
-        float* vy = wy + ldw;
-#pragma unroll
-        for (int e = 0; e < RJ; ++e) {
-          const int i = lt + 64 * e;
-          u[e] = i < rc ? vx[i] : 0.f;
-          v[e] = i < rc ? vy[i] : 0.f;
-        }
-#pragma unroll
-        for (int e = 0; e < RJ; ++e) {
-          const int i = lt + 64 * e;
-          if (i < rc) {
-            vx[i] = cs * u[e] - sn * v[e];
-            vy[i] = sn * u[e] + cs * v[e];
-          }
-        }
-        if (lt == 0) {
-          atomicAdd(&nrot, 1);
-          atomicMax(&cosmax, __float_as_int(nn > 0.f ? fminf(__fdividef(fabsf(g), nn), 1.f) : 1.f));
+        for (int w = 0; w < WP; ++w) {
+          na += red[grp][w][0];
+          nb += red[grp][w][1];
+          g2 += red[grp][w][2];
         }
       }
     }
-    __syncthreads();  // columns change hands; red is free again
+    if (!present) return false;
+    const float ag = 0.5f * fabsf(g2), nn = fsqrt_ap(fabsf(na)) * fsqrt_ap(fabsf(nb));
+    if (!(EIG ? ag > thr_abs : ag > a.tol32 * nn)) return false;
+    const float t = jacobi_tan(nb - na, g2);
+    const float c = rsqrtf(fmaf(t, t, 1.f)), sn = c * t;
+    const uint64_t c2 = pk2(c, c), s2 = pk2(sn, sn), n2 = pk2(-sn, -sn);
+#pragma unroll
+    for (int e = 0; e < RV; ++e) {
+      const ulonglong2 wu = wx[e], vu = vx[e];
+      wx[e] = make_ulonglong2(fma2(c2, wu.x, mul2(n2, wy[e].x)), fma2(c2, wu.y, mul2(n2, wy[e].y)));
+      wy[e] = make_ulonglong2(fma2(c2, wy[e].x, mul2(s2, wu.x)), fma2(c2, wy[e].y, mul2(s2, wu.y)));
+      vx[e] = make_ulonglong2(fma2(c2, vu.x, mul2(n2, vy[e].x)), fma2(c2, vu.y, mul2(n2, vy[e].y)));
+      vy[e] = make_ulonglong2(fma2(c2, vy[e].x, mul2(s2, vu.x)), fma2(c2, vy[e].y, mul2(s2, vu.y)));
+    }
+    ++my_rot;
+    if (!EIG) my_cos = fmaxf(my_cos, nn > 0.f ? fminf(__fdividef(ag, nn), 1.f) : 1.f);
+    return true;
+  };
+  auto fetch = [&](int l, ulonglong2 (&w)[RV], ulonglong2 (&v)[RV]) {
+    const ulonglong2* c = sm + l * c4;
+#pragma unroll
+    for (int e = 0; e < RV; ++e) {
+      const int i = lt + LP * e;
+      w[e] = i < q4 ? c[i] : z;
+      v[e] = i < v4 ? c[q4 + i] : z;
+    }
+  };
+  auto keep = [&](int l, const ulonglong2 (&w)[RV], const ulonglong2 (&v)[RV]) {
+    ulonglong2* c = sm + l * c4;
+#pragma unroll
+    for (int e = 0; e < RV; ++e) {
+      const int i = lt + LP * e;
+      if (i < q4) c[i] = w[e];
+      if (i < v4) c[q4 + i] = v[e];
+    }
   };
 
   const int rounds = NB - 1;
   bool done = rc < 2;
-  for (int sweep = 0; sweep < kPreSweeps && !done; ++sweep) {
+  for (int sweep = 0; sweep < (EIG ? kEigSweeps : kPreSweeps) && !done; ++sweep) {
     for (int r = 0; r < rounds; ++r) {
-      int P, Q;
-      if (cta == 0) {
-        P = r;
-        Q = NB - 1;
-      } else {
-        P = (r + cta) % (NB - 1);
-        Q = (r - cta + (NB - 1)) % (NB - 1);
-      }
-      if (P > Q) {
-        const int t = P;
-        P = Q;
-        Q = t;
-      }
-      auto gcol = [&](int l) { return l < 4 ? 4 * P + l : 4 * Q + l - 4; };
-      for (int l = 0; l < 8; ++l) {
-        const int g = gcol(l);
-        if (g >= rc) continue;
-        const float* ws = W + (int64_t)g * ld;
-        const float* vs = V + (int64_t)g * ld;
-        const uint32_t dst = tc::su32(sm + (int64_t)l * cst);
-        for (int i = threadIdx.x; i < (ldw >> 2); i += blockDim.x)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(ws + 4 * i) : "memory");
-        for (int i = threadIdx.x; i < (ldv >> 2); i += blockDim.x)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4u * ldw + 16u * i), "l"(vs + 4 * i)
-                       : "memory");
-      }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncthreads();
-      if (r == 0) {  // pairs inside P (groups 0, 1) and inside Q (groups 2, 3)
-        for (int ir = 0; ir < 3; ++ir) {
-          int x, y;
-          if ((grp & 1) == 0) {
-            x = ir;
-            y = 3;
-          } else {
-            x = min((ir + 1) % 3, (ir + 2) % 3);
-            y = max((ir + 1) % 3, (ir + 2) % 3);
-          }
-          x += (grp >> 1) * 4;
-          y += (grp >> 1) * 4;
-          process(x, y, gcol(x) < rc && gcol(y) < rc);
+      if (cta < active) {
+        int P, Q;
+        if (cta == 0) {
+          P = r;
+          Q = NB - 1;
+        } else {
+          P = (r + cta) % (NB - 1);
+          Q = (r - cta + (NB - 1)) % (NB - 1);
         }
-      }
-      for (int ir = 0; ir < 4; ++ir) {
-        const int y = 4 + ((grp + ir) & 3);
-        process(grp, y, gcol(grp) < rc && gcol(y) < rc);
-      }
-      for (int l = 0; l < 8; ++l) {
-        const int g = gcol(l);
-        if (g >= rc) continue;
-        float4* wd = reinterpret_cast<float4*>(W + (int64_t)g * ld);
-        float4* vd = reinterpret_cast<float4*>(V + (int64_t)g * ld);
-        const float4* s4 = reinterpret_cast<const float4*>(sm + (int64_t)l * cst);
-        for (int i = threadIdx.x; i < (ldw >> 2); i += blockDim.x) __stcg(&wd[i], s4[i]);
-        for (int i = threadIdx.x; i < (ldv >> 2); i += blockDim.x) __stcg(&vd[i], s4[(ldw >> 2) + i]);
-      }
-      if (r == rounds - 1 && threadIdx.x == 0 && nrot) {
-        atomicAdd(&q.info[kiRot32 + sweep], nrot);
-        atomicMax(&q.info[kiCos32 + sweep], cosmax);
-        nrot = 0;
-        cosmax = 0;
-      }
-      if (!bar.sync()) return;
-    }
-    done = __ldcg(&q.info[kiRot32 + sweep]) == 0 || __int_as_float(__ldcg(&q.info[kiCos32 + sweep])) < kPreCos;
-    if (done && cta == 0 && threadIdx.x == 0) q.info[kiPre] = sweep + 1;
-  }
-  // V in FP64
-  for (int j = cta; j < rc; j += active)
-    for (int i = threadIdx.x; i < rc; i += blockDim.x)
-      q.Vx[i + (int64_t)j * a.ldx] = f2d(__ldcg(&V[i + (int64_t)j * ld]));
-}
-
-// The same sweeps by one thread-block cluster (n ≤ 512; C = 1, 2, 4, 8 or 16
-// CTAs, at most 16 columns a block): its hardware barrier takes 0.24 µs where
-// the grid barrier takes 1.1, and with blocks this long a sweep has 2C − 1
-// exchanges through L2 instead of n/4.  One warp per column pair, B inner
-// rounds of B disjoint pairs with a CTA barrier each.  n = 324: 3.4 ms (grid
-// variant 3.75); n = 64: 0.98 ms for the whole decomposition (1.17).
-template <int RJ>
-__global__ void __launch_bounds__(512) k_svd_sweeps32_cl(SvdArgs a) {
-  extern __shared__ __align__(16) unsigned char sm_raw[];
-  const SvdProb& q = a.p[blockIdx.y];
-  const int rc = q.info[kiRank];
-  if (q.info[kiErr]) return;
-  const bool two = a.second || rc < a.n;
-  const int mx = two ? rc : a.n;
-  const int C = gridDim.x, cta = blockIdx.x, NB = 2 * C;
-  const int B = (rc + NB - 1) / NB;  // columns per block (the last blocks may be short or empty)
-  float* W = q.W32;
-  float* V = q.V32;
-  const int ld = a.ld32;
-  const int ldw = (mx + 3) & ~3, ldv = (rc + 3) & ~3, cst = ldw + ldv;
-  float* sm = reinterpret_cast<float*>(sm_raw);  // 2B columns: W rows, then V rows
-  __shared__ int nrot, cosmax;
-  if (threadIdx.x == 0) nrot = cosmax = 0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double* X = two ? q.X2 : q.X;
-  for (int j = cta; j < rc; j += C) {
-    for (int i = threadIdx.x; i < mx; i += blockDim.x)
-      __stcg(&W[i + (int64_t)j * ld], d2f(X[i + (int64_t)j * a.ldx]));
-    for (int i = threadIdx.x; i < rc; i += blockDim.x) __stcg(&V[i + (int64_t)j * ld], i == j ? 1.f : 0.f);
-  }
-  GridBar<true> bar{nullptr, 0u, 0u, nullptr, nullptr};
-  bar.sync();
-
-  auto process = [&](int x, int y) {  // local columns, x before y in global order
-    float* wx = sm + (int64_t)x * cst;
-    float* wy = sm + (int64_t)y * cst;
-    float u[RJ], v[RJ];
-    float na = 0.f, nb = 0.f, g = 0.f;
-#pragma unroll
-    for (int e = 0; e < RJ; ++e) {
-      const int i = lane + 32 * e;
-      u[e] = i < mx ? wx[i] : 0.f;
-      v[e] = i < mx ? wy[i] : 0.f;
-    }
-#pragma unroll
-    for (int e = 0; e < RJ; ++e) {
-      na = fmaf(u[e], u[e], na);
-      nb = fmaf(v[e], v[e], nb);
-      g = fmaf(u[e], v[e], g);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      na += __shfl_xor_sync(0xffffffffu, na, o);
-      nb += __shfl_xor_sync(0xffffffffu, nb, o);
-      g += __shfl_xor_sync(0xffffffffu, g, o);
-    }
-    const float nn = fsqrt_ap(na) * fsqrt_ap(nb);
-    if (!(fabsf(g) > a.tol32 * nn)) return;
-    const float t = jacobi_tan(nb - na, 2.f * g);
-    const float cs = rsqrtf(fmaf(t, t, 1.f)), sn = cs * t;
-#pragma unroll
-    for (int e = 0; e < RJ; ++e) {
-      const int i = lane + 32 * e;
-      if (i < mx) {
-        wx[i] = cs * u[e] - sn * v[e];
-        wy[i] = sn * u[e] + cs * v[e];
-      }
-    }
-    float* vx = wx + ldw;
-    float* vy = wy + ldw;
-#pragma unroll
-    for (int e = 0; e < RJ; ++e) {
-      const int i = lane + 32 * e;
-      u[e] = i < rc ? vx[i] : 0.f;
-      v[e] = i < rc ? vy[i] : 0.f;
-    }
-#pragma unroll
-    for (int e = 0; e < RJ; ++e) {
-      const int i = lane + 32 * e;
-      if (i < rc) {
-        vx[i] = cs * u[e] - sn * v[e];
-        vy[i] = sn * u[e] + cs * v[e];
-      }
-    }
-    if (lane == 0) {
-      atomicAdd(&nrot, 1);
-      atomicMax(&cosmax, __float_as_int(nn > 0.f ? fminf(__fdividef(fabsf(g), nn), 1.f) : 1.f));
-    }
-  };
-
-  bool done = rc < 2;
-  for (int sweep = 0; sweep < kPreSweeps && !done; ++sweep) {
-    for (int r = 0; r < NB - 1; ++r) {
-      int P, Q;
-      if (cta == 0) {
-        P = r;
-        Q = NB - 1;
-      } else {
-        P = (r + cta) % (NB - 1);
-        Q = (r - cta + (NB - 1)) % (NB - 1);
-      }
-      if (P > Q) {
-        const int t = P;
-        P = Q;
-        Q = t;
-      }
-      auto gcol = [&](int l) { return l < B ? P * B + l : Q * B + l - B; };
-      for (int l = warp; l < 2 * B; l += 16) {  // one warp per column
-        const int g = gcol(l);
-        if (g >= rc) continue;
-        const float* ws = W + (int64_t)g * ld;
-        const float* vs = V + (int64_t)g * ld;
-        const uint32_t dst = tc::su32(sm + (int64_t)l * cst);
-        for (int i = lane; i < (ldw >> 2); i += 32)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(ws + 4 * i) : "memory");
-        for (int i = lane; i < (ldv >> 2); i += 32)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4u * ldw + 16u * i), "l"(vs + 4 * i)
-                       : "memory");
-      }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncthreads();
-      if (r == 0 && B > 1) {  // pairs inside P and inside Q: circle method over B (even: BE) columns
-        const int BE = B + (B & 1);
-        for (int ir = 0; ir < BE - 1; ++ir) {
-          for (int s = warp; s < BE; s += 16) {  // BE/2 slots for P, BE/2 for Q
-            const int k = s >= BE / 2 ? s - BE / 2 : s, off = s >= BE / 2 ? B : 0;
-            int x = k == 0 ? BE - 1 : (ir + k) % (BE - 1);
-            int y = k == 0 ? ir : (ir - k + (BE - 1)) % (BE - 1);
+        if (P > Q) {
+          const int t = P;
+          P = Q;
+          Q = t;
+        }
+        auto gcol = [&](int l) { return l < B ? B * P + l : B * Q + l - B; };
+        for (int l = threadIdx.x >> 5; l < 2 * B; l += NW) {  // one warp per column
+          const int g = gcol(l);
+          if (g >= rc) continue;
+          const float* ws = W + (int64_t)g * ld;
+          const float* vs = V + (int64_t)g * ld;
+          const uint32_t dst = tc::su32(sm + l * c4);
+          for (int i = lane; i < q4; i += 32)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(ws + 4 * i) : "memory");
+          for (int i = lane; i < v4; i += 32)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (q4 + i)), "l"(vs + 4 * i)
+                         : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        ulonglong2 wx[RV], vx[RV], wy[RV], vy[RV];
+        if (r == 0) {  // pairs inside P (first half of the groups) and inside Q: circle method over B
+          for (int ir = 0; ir < B - 1; ++ir) {
+            const int k = grp % (B / 2), off = grp < B / 2 ? 0 : B;
+            int x = k == 0 ? B - 1 : (ir + k) % (B - 1);
+            int y = k == 0 ? ir : (ir - k + (B - 1)) % (B - 1);
             if (x > y) {
               const int t = x;
               x = y;
               y = t;
             }
-            if (y < B && gcol(off + y) < rc) process(off + x, off + y);
+            const bool present = gcol(off + y) < rc;
+            if (present) {
+              fetch(off + x, wx, vx);
+              fetch(off + y, wy, vy);
+            }
+            if (rotate(wx, vx, wy, vy, present)) {
+              keep(off + x, wx, vx);
+              keep(off + y, wy, vy);
+            }
+            __syncthreads();
           }
+        }
+        // cross pairs: a group keeps its column of P in registers through the B
+        // inner rounds; Q's columns pass through shared memory
+        fetch(grp, wx, vx);
+        for (int ir = 0; ir < B; ++ir) {
+          const int y = B + ((grp + ir) & (B - 1));
+          const bool present = gcol(y) < rc;  // P comes before Q
+          if (present) fetch(y, wy, vy);
+          if (rotate(wx, vx, wy, vy, present)) keep(y, wy, vy);
           __syncthreads();
         }
-      }
-      for (int ir = 0; ir < B; ++ir) {
-        for (int s = warp; s < B; s += 16) {
-          const int y = B + (s + ir < B ? s + ir : s + ir - B);
-          if (gcol(s) < rc && gcol(y) < rc) process(s, y);
+        if (gcol(grp) < rc) {
+          ulonglong2* wd = reinterpret_cast<ulonglong2*>(W + (int64_t)gcol(grp) * ld);
+          ulonglong2* vd = reinterpret_cast<ulonglong2*>(V + (int64_t)gcol(grp) * ld);
+#pragma unroll
+          for (int e = 0; e < RV; ++e) {
+            const int i = lt + LP * e;
+            if (i < q4) __stcg(&wd[i], wx[e]);
+            if (i < v4) __stcg(&vd[i], vx[e]);
+          }
         }
+        for (int l = B + (threadIdx.x >> 5); l < 2 * B; l += NW) {
+          const int g = gcol(l);
+          if (g >= rc) continue;
+          ulonglong2* wd = reinterpret_cast<ulonglong2*>(W + (int64_t)g * ld);
+          ulonglong2* vd = reinterpret_cast<ulonglong2*>(V + (int64_t)g * ld);
+          const ulonglong2* s4 = sm + l * c4;
+          for (int i = lane; i < q4; i += 32) __stcg(&wd[i], s4[i]);
+          for (int i = lane; i < v4; i += 32) __stcg(&vd[i], s4[q4 + i]);
+        }
+      }
+      if (r == rounds - 1) {
+        if (lt == 0 && my_rot) {
+          atomicAdd(&nrot, my_rot);
+          atomicMax(&cosmax, __float_as_int(my_cos));
+        }
+        my_rot = 0;
+        my_cos = 0.f;
         __syncthreads();
+        if (threadIdx.x == 0 && nrot) {
+          atomicAdd(&q.info[kiRot32 + sweep], nrot);
+          atomicMax(&q.info[kiCos32 + sweep], cosmax);
+          nrot = 0;
+          cosmax = 0;
+        }
       }
-      for (int l = warp; l < 2 * B; l += 16) {
-        const int g = gcol(l);
-        if (g >= rc) continue;
-        float4* wd = reinterpret_cast<float4*>(W + (int64_t)g * ld);
-        float4* vd = reinterpret_cast<float4*>(V + (int64_t)g * ld);
-        const float4* s4 = reinterpret_cast<const float4*>(sm + (int64_t)l * cst);
-        for (int i = lane; i < (ldw >> 2); i += 32) __stcg(&wd[i], s4[i]);
-        for (int i = lane; i < (ldv >> 2); i += 32) __stcg(&vd[i], s4[(ldw >> 2) + i]);
-      }
-      if (r == NB - 2 && threadIdx.x == 0 && nrot) {
-        atomicAdd(&q.info[kiRot32 + sweep], nrot);
-        atomicMax(&q.info[kiCos32 + sweep], cosmax);
-        nrot = 0;
-        cosmax = 0;
-      }
-      bar.sync();
+      if (!bar.sync()) return;
     }
-    done = __ldcg(&q.info[kiRot32 + sweep]) == 0 || __int_as_float(__ldcg(&q.info[kiCos32 + sweep])) < kPreCos;
+    const int rot = __ldcg(&q.info[kiRot32 + sweep]);
+    done = EIG ? rot <= 16 * rc : rot == 0 || __int_as_float(__ldcg(&q.info[kiCos32 + sweep])) < kPreCos;
     if (done && cta == 0 && threadIdx.x == 0) q.info[kiPre] = sweep + 1;
   }
-  for (int j = cta; j < rc; j += C)  // V in FP64
+  // V in FP64
+  for (int j = cta; j < rc; j += max(active, 1))
     for (int i = threadIdx.x; i < rc; i += blockDim.x)
       q.Vx[i + (int64_t)j * a.ldx] = f2d(__ldcg(&V[i + (int64_t)j * ld]));
 }
@@ -1159,34 +1085,42 @@ void launch_sweeps(tnad_ctx* c, int np, SvdArgs& a) {
   }
 }
 
+template <int B, int RV, int WP, bool EIG, bool CL>
+void launch_sweeps32_rv(tnad_ctx* c, int np, SvdArgs& a) {
+  const int nreal = (a.n + B - 1) / B, G = std::max(1, (nreal + (nreal & 1)) / 2);
+  static std::atomic<bool> attr{false};
+  if (!attr) {
+    TNAD_CK(cudaFuncSetAttribute(k_sweeps32<B, RV, WP, EIG, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 2 * B * 2 * 128 * WP * RV * 4));  // 2B columns of W and V
+    attr = true;
+  }
+  launch_grid(c, k_sweeps32<B, RV, WP, EIG, CL>, CL, G, np, 32 * B * WP, (size_t)2 * B * 2 * a.ld32 * sizeof(float), a);
+}
+
+// Up to 128 columns the at most 8 CTAs form a cluster.  One warp per pair up to
+// 512 rows (a second one's share of the sums costs a barrier: n = 324 64 → 56 ms
+// as above), two beyond, where a lane would hold 64 registers of each column; and
+// there blocks of 4, which spread 1024 columns over 128 SMs' shared memories.
+template <bool EIG>
+void launch_sweeps32(tnad_ctx* c, int np, SvdArgs& a) {
+  if (a.n <= 128)
+    launch_sweeps32_rv<8, 1, 1, EIG, true>(c, np, a);
+  else if (a.n <= 256)
+    launch_sweeps32_rv<8, 2, 1, EIG, false>(c, np, a);
+  else if (a.n <= 384)
+    launch_sweeps32_rv<8, 3, 1, EIG, false>(c, np, a);
+  else if (a.n <= 512)
+    launch_sweeps32_rv<8, 4, 1, EIG, false>(c, np, a);
+  else
+    launch_sweeps32_rv<4, 4, 2, EIG, false>(c, np, a);
+}
+
 // FP32 sweeps, then V orthogonal to FP64 rounding (two first-order triangular
 // corrections: 1e-6 → 1e-12 → 1e-24) and W = X·V, all in DFMA products: the
 // tensor-core ones are accurate to the row and column scales only, not to the
 // small columns of graded operands.
-template <int RJ>
 void pre_sweeps(tnad_ctx* c, int np, SvdArgs& a, int* info_host) {
-  static std::atomic<bool> attr{false};
-  if constexpr (RJ <= 8) {  // n ≤ 512
-    const int C = a.n <= 32 ? 1 : a.n <= 64 ? 2 : a.n <= 128 ? 4 : a.n <= 256 ? 8 : 16;
-    const int B = (a.n + 2 * C - 1) / (2 * C);
-    const size_t smem = (size_t)2 * B * 2 * a.ld32 * sizeof(float);
-    if (!attr) {
-      TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps32_cl<2 * RJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   2 * 16 * 2 * 512 * 4));
-      TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps32_cl<2 * RJ>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-      attr = true;
-    }
-    launch_grid(c, k_svd_sweeps32_cl<2 * RJ>, true, C, np, 512, smem, a);
-  } else {
-    const int nreal = (a.n + 3) / 4, G = std::max(1, (nreal + (nreal & 1)) / 2);
-    const size_t smem = (size_t)8 * 2 * a.ld32 * sizeof(float);
-    if (!attr) {
-      TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps32<RJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   8 * 2 * kMaxSvdRows * 4));
-      attr = true;
-    }
-    launch_grid(c, k_svd_sweeps32<RJ>, false, G, np, 256, smem, a);
-  }
+  launch_sweeps32<false>(c, np, a);
   for (int p = 0; p < np; ++p)
     TNAD_CK(cudaMemcpyAsync(info_host + p * kiBar, a.p[p].info, sizeof(int) * kiBar, cudaMemcpyDeviceToHost, c->stream));
   TNAD_CK(cudaStreamSynchronize(c->stream));
@@ -1218,7 +1152,7 @@ template <int R>
 void svd_qrj_r(tnad_ctx* c, int np, bool symmetric, SvdArgs& a, int* info_host) {
   launch_qrcp<R, 0>(c, np, a.n, a);
   launch_qrcp<R, 1>(c, np, a.n, a);
-  if (a.n >= kPreMin) pre_sweeps<R / 2>(c, np, a, info_host);
+  if (a.n >= kPreMin) pre_sweeps(c, np, a, info_host);
   if (symmetric)
     launch_sweeps<R / 2, false>(c, np, a);
   else
@@ -1239,6 +1173,35 @@ void svd_qrj_r(tnad_ctx* c, int np, bool symmetric, SvdArgs& a, int* info_host) 
 }
 
 }  // namespace
+
+int sweeps32_eig(tnad_ctx* c, const double* A, int64_t n, const double* fro2, double* V) {
+  TNAD_REQUIRE(n >= 2 && n <= kMaxSvdRows, TNAD_ERR_SHAPE, "sweeps32_eig: n must be in [2,1024]");
+  WsScope scope(c);
+  SvdArgs a = {};
+  a.m = a.n = a.ldx = (int)n;
+  a.ld32 = (int)((n + 3) & ~(int64_t)3);
+  a.fro2 = fro2;
+  SvdProb& q = a.p[0];
+  q.A = A;
+  q.W32 = ws_f(c, (int64_t)a.ld32 * n);
+  q.V32 = ws_f(c, (int64_t)a.ld32 * n);
+  q.Vx = V;
+  q.info = (int*)c->ws.alloc(sizeof(int) * kiCount);
+  TNAD_CK(cudaMemsetAsync(q.info, 0, sizeof(int) * kiCount, c->stream));
+  {
+    KernelTimer kt(c, "jacobi_round_f32", 0.0);
+    launch_sweeps32<true>(c, 1, a);
+    check_launch(c, "sweeps32_eig");
+  }
+  int h[kiBar];
+  TNAD_CK(cudaMemcpyAsync(h, q.info, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+  TNAD_CK(cudaStreamSynchronize(c->stream));
+  TNAD_REQUIRE(h[kiErr] == 0, TNAD_ERR_TIMEOUT, "sweeps32_eig: a bounded barrier wait expired");
+  const int sweeps = h[kiPre] > 0 ? h[kiPre] : kEigSweeps;
+  // algorithmic work: per pair 4 dot products and the rotation of W and V
+  if (c->ktimer == "jacobi_round_f32") c->kt_work += 0.5 * sweeps * (double)n * (double)n * 20.0 * (double)n;
+  return sweeps;
+}
 
 bool svd_qrj_fits(int64_t m, int64_t n) { return m >= n && n >= 2 && m <= kMaxSvdRows; }
 

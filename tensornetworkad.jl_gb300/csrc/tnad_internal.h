@@ -105,8 +105,8 @@ struct tnad_ctx {
   // size go straight to the FP64 sweeps (jacobi.cu, kEigSkip)
   int64_t eig_skip_n = 0;
   int eig_skip_left = 0;
-  // FP32 Jacobi sweeps of the symmetric SVD as block rounds (k_jacobi_block;
-  // false: one launch per element round, set by TNAD_JACOBI_BLOCKS=0)
+  // FP32 Jacobi sweeps of the symmetric SVD as block rounds in one launch
+  // (k_sweeps32; false: one launch per element round, set by TNAD_JACOBI_BLOCKS=0)
   bool jacobi_blocks = true;
   // kernel timer (tnad_ctx_kernel_timer): events around every launch of one
   // kernel family, with the algorithmic work (flops or bytes) of each launch
@@ -269,14 +269,20 @@ void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, d
 // then Jacobi on the triangular factor, each one launch (svd_qr.cu).  Values
 // below the rounding of A come back as 0, their vectors as an orthonormal
 // completion.  symmetric: U = V·sign(λ) (±λ pairs: from A·V).
+// FP32 Jacobi sweeps with the eigenvalue rule on a symmetric A (n ≤ 1024), one
+// launch: V (n×n) orthogonal to ~1e-5, VᵀAV diagonal to ~1e-6·‖A‖.  fro2: ‖A‖²_F
+// on the device.  Returns the number of sweeps (waits for them).
+int sweeps32_eig(tnad_ctx* c, const double* A, int64_t n, const double* fro2, double* V);
 bool svd_qrj_fits(int64_t m, int64_t n);
 void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, double* const* U, double* const* S,
              double* const* V, bool symmetric);
 // Refines X (n×n, nearly orthonormal approximate eigenvectors of the symmetric
 // A, n ≤ 2048) to FP64 accuracy by matrix products; lam gets the eigenvalues
 // (column order of X).  fro2: ‖A‖²_F on the device.  false: no convergence
-// (X is then unusable and the caller falls back to Jacobi sweeps).
-bool eig_refine(tnad_ctx* c, const double* A, int64_t n, double* X, double* lam, const double* fro2);
+// (X is then unusable and the caller falls back to Jacobi sweeps); *graded: the
+// first measurement showed no approximate eigendecomposition, as for graded spectra.
+bool eig_refine(tnad_ctx* c, const double* A, int64_t n, double* X, double* lam, const double* fro2,
+                bool* graded = nullptr);
 // FP64-accurate eigendecomposition of a small symmetric p×p matrix (p ≤ 256):
 // one-CTA FP32 Jacobi, then eig_refine; W, lam sorted by |λ| descending.
 // false: the refinement did not converge (W, lam untouched).
