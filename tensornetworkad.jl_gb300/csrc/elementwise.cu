@@ -63,20 +63,29 @@ struct PermArgs {
   int64_t istr[10];  // input stride of the input axis that becomes output axis k
 };
 
+// I: index type (32 bits where the tensor allows it: a 64-bit quotient is a
+// subroutine of ~100 instructions, and there is one an axis and element).  The
+// factors are compared on the host: each comparison is an FP64 instruction (64
+// clocks of a warp's quadrant).
+template <typename I>
 __global__ void k_permute(PermArgs a, int64_t n, const double* __restrict__ in, double* __restrict__ out,
-                          double alpha, double beta) {
+                          double alpha, double beta, int scaled, int accum) {
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
-    int64_t rem = o, off = 0;
+    I rem = (I)o;
+    int64_t off = 0;
 #pragma unroll
     for (int k = 0; k < 10; ++k) {
-      if (k < a.nd) {
-        int64_t ck = rem % a.odim[k];
-        rem /= a.odim[k];
-        off += ck * a.istr[k];
+      if (k + 1 < a.nd) {
+        const I q = rem / (I)a.odim[k];
+        off += (int64_t)(rem - q * (I)a.odim[k]) * a.istr[k];
+        rem = q;
+      } else if (k + 1 == a.nd) {
+        off += (int64_t)rem * a.istr[k];
       }
     }
-    double v = alpha * in[off];
-    out[o] = beta == 0.0 ? v : v + beta * out[o];
+    double v = in[off];
+    if (scaled) v *= alpha;
+    out[o] = accum ? v + beta * out[o] : v;
   }
 }
 
@@ -238,7 +247,23 @@ void permute(tnad_ctx* c, const Ten& in, const int* perm, double* out, double al
     }
     return;
   }
-  k_permute<<<nblocks(n, 256, 8192), 256, 0, c->stream>>>(a, n, in.p, out, alpha, beta);
+  // output axes that follow each other in the input too are one axis
+  int nd = 0;
+  for (int k = 0; k < in.nd; ++k) {
+    if (a.odim[k] == 1) continue;
+    if (nd > 0 && a.istr[k] == a.istr[nd - 1] * a.odim[nd - 1]) {
+      a.odim[nd - 1] *= a.odim[k];
+      continue;
+    }
+    a.odim[nd] = a.odim[k];
+    a.istr[nd++] = a.istr[k];
+  }
+  a.nd = nd;
+  const int scaled = alpha != 1.0, accum = beta != 0.0, nb = nblocks(n, 256, 8192);
+  if (n < (1ll << 32))
+    k_permute<uint32_t><<<nb, 256, 0, c->stream>>>(a, n, in.p, out, alpha, beta, scaled, accum);
+  else
+    k_permute<int64_t><<<nb, 256, 0, c->stream>>>(a, n, in.p, out, alpha, beta, scaled, accum);
   count_launch(c);
   check_launch(c, "permute");
 }

@@ -41,6 +41,7 @@ struct GemmArgs {
   double *C, *part;
   int* cnt;
   GemmMap am, ak, bk, bn, cm, cn;
+  int scaled, accum;   // alpha ≠ 1, beta ≠ 0: compared once on the host, each comparison is an FP64 instruction
   int a_rows, b_rows;  // lanes run along the rows (columns) of the tile, else along K
 };
 
@@ -147,8 +148,9 @@ __global__ void __launch_bounds__(256) k_gemm_f64(const GemmArgs g) {
       const unsigned gi = m0 + tx + 16 * i;
       if (gi >= g.M) continue;
       double* c = g.C + cj + map_off(g.cm, gi);
-      const double v = g.alpha * acc[i][j];
-      *c = g.beta == 0.0 ? v : v + g.beta * (*c);
+      double v = acc[i][j];
+      if (g.scaled) v *= g.alpha;
+      *c = g.accum ? v + g.beta * (*c) : v;
     }
   }
 }
@@ -156,8 +158,9 @@ __global__ void __launch_bounds__(256) k_gemm_f64(const GemmArgs g) {
 // Tile and split with the least time on the busiest SM, in clocks: its share of
 // the tiles at 1.7 DFMA a clock, ~1200 for a CTA's first loads and stores (partly
 // hidden where an SM holds several), ~2500 more where K is split (partials,
-// counter, the sum).  Measured: 32×32×32 (one 32×32 tile, K in two halves and a
-// second kernel before) 11.6 → see DESIGN's table of cases; 1024³ stays at the pipe's limit.
+// counter, the sum).  Measured with its launch: 32×32×32 12.6 µs with one 32×32
+// tile, K in two halves and a second kernel, 7.8 µs by this rule; 1024³ stays at
+// the pipe's limit (2.07 ms).
 void gemm_f64_plan(int sms, int64_t M, int64_t N, int64_t K, int* tile, int* splits) {
   double best = 1e300;
   for (int t : {64, 32, 16}) {
@@ -196,6 +199,8 @@ void gemm_f64_map(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, co
   g.ks = (int)((K + kc - 1) / kc);
   g.alpha = alpha;
   g.beta = beta;
+  g.scaled = alpha != 1.0;
+  g.accum = beta != 0.0;
   g.A = A;
   g.B = B;
   g.C = C;

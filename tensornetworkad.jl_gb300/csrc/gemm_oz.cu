@@ -48,6 +48,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "fp64_fast.cuh"
 #include "tc_common.cuh"
 #include "tnad_internal.h"
 
@@ -81,48 +82,65 @@ __device__ __forceinline__ int exp_bound(double x) {
   return ex - 1022;
 }
 
-// e[r] = max over the row r of op(X) of exp_bound (atomicMax per 32×32 tile row)
-__global__ void k_oz_exp(const double* __restrict__ X, int64_t ld, int tr, int64_t rows, int64_t K,
-                         int* __restrict__ e) {
-  __shared__ double tile[32][33];
-  const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
+// One operand as the slicing kernels read it: op(X) is rows × K, column-major
+// with leading dimension ld, transposed when tr; e[r] bounds row r.
+struct OzIn {
+  const double* X;
+  int64_t ld, rows, rows_pad;
+  int tr;
+  int* e;
+  __nv_bfloat16* out;
+};
+
+// 32×32 tile of op(X) through shared memory
+__device__ __forceinline__ void oz_tile(const OzIn& in, int64_t r0, int64_t k0, int64_t K, double (*tile)[33]) {
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 × 8
+#pragma unroll
   for (int j = ty; j < 32; j += 8) {
     int64_t r, k;
-    if (!tr) { r = r0 + tx; k = k0 + j; } else { k = k0 + tx; r = r0 + j; }
+    if (!in.tr) { r = r0 + tx; k = k0 + j; } else { k = k0 + tx; r = r0 + j; }
     double v = 0.0;
-    if (r < rows && k < K) v = !tr ? X[r + k * ld] : X[k + r * ld];
-    if (!tr) tile[tx][j] = v; else tile[j][tx] = v;
+    if (r < in.rows && k < K) v = !in.tr ? in.X[r + k * in.ld] : in.X[k + r * in.ld];
+    if (!in.tr) tile[tx][j] = v; else tile[j][tx] = v;
   }
   __syncthreads();
+}
+
+// Both operands of a product in one launch each (tile rows [0, nya) are A's,
+// on a one-dimensional grid: the sum of both heights has no limit of its own):
+// a product of these sizes takes 15 to 40 µs, and each launch beside it 5 to
+// 8 µs with its gap.
+// e[r] = max over the row r of op(X) of exp_bound (atomicMax per 32×32 tile row)
+__global__ void k_oz_exp(OzIn a, OzIn b, int nya, int64_t K, int64_t k_pad) {
+  __shared__ double tile[32][33];
+  const int nk = (int)((k_pad + 31) / 32), by = (int)blockIdx.x / nk, bx = (int)blockIdx.x % nk;
+  const bool isa = by < nya;
+  const OzIn in = isa ? a : b;
+  const int64_t r0 = (int64_t)(isa ? by : by - nya) * 32, k0 = (int64_t)bx * 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 × 8
+  oz_tile(in, r0, k0, K, tile);
   for (int j = ty; j < 32; j += 8) {
     int m = exp_bound(tile[j][tx]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (tx == 0 && r0 + j < rows) atomicMax(e + r0 + j, m);
+    if (tx == 0 && r0 + j < in.rows) atomicMax(in.e + r0 + j, m);
   }
 }
 
 // six BF16 slice planes (K-major, rows_pad × k_pad each) of op(X)
-__global__ void k_oz_slice(const double* __restrict__ X, int64_t ld, int tr, int64_t rows, int64_t K,
-                           int64_t rows_pad, int64_t k_pad, const int* __restrict__ e,
-                           __nv_bfloat16* __restrict__ out) {
+__global__ void k_oz_slice(OzIn a, OzIn b, int nya, int64_t K, int64_t k_pad) {
   __shared__ double tile[32][33];
-  const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
+  const int nk = (int)((k_pad + 31) / 32), by = (int)blockIdx.x / nk, bx = (int)blockIdx.x % nk;
+  const bool isa = by < nya;
+  const OzIn in = isa ? a : b;
+  const int64_t r0 = (int64_t)(isa ? by : by - nya) * 32, k0 = (int64_t)bx * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int j = ty; j < 32; j += 8) {
-    int64_t r, k;
-    if (!tr) { r = r0 + tx; k = k0 + j; } else { k = k0 + tx; r = r0 + j; }
-    double v = 0.0;
-    if (r < rows && k < K) v = !tr ? X[r + k * ld] : X[k + r * ld];
-    if (!tr) tile[tx][j] = v; else tile[j][tx] = v;
-  }
-  __syncthreads();
-  const int64_t plane = rows_pad * k_pad;
+  oz_tile(in, r0, k0, K, tile);
+  const int64_t plane = in.rows_pad * k_pad;
   for (int j = ty; j < 32; j += 8) {
     const int64_t r = r0 + j, k = k0 + tx;
-    if (r >= rows_pad || k >= k_pad) continue;
-    const int er = r < rows ? e[r] : kExpZero - 1;
+    if (r >= in.rows_pad || k >= k_pad) continue;
+    const int er = r < in.rows ? in.e[r] : kExpZero - 1;
     int64_t Y = 0;
     if (er > kExpZero && er < kExpNonFinite) {
       // Y = round(x·2^(55−er)) from the bits of x (integer arithmetic only)
@@ -150,15 +168,25 @@ __global__ void k_oz_slice(const double* __restrict__ X, int64_t ld, int tr, int
       const int bsh = 48 - 8 * s;
       const int64_t q = (Y + (1ll << (bsh - 1))) >> bsh;  // balanced digit, |q| ≤ 128
       Y -= q << bsh;
-      out[s * plane + r * k_pad + k] = __float2bfloat16_rn((float)q * __int_as_float((127 - 8 * s) << 23));
+      in.out[s * plane + r * k_pad + k] = __float2bfloat16_rn((float)q * __int_as_float((127 - 8 * s) << 23));
     }
   }
+}
+
+// x·2^e for |x| in [2^-100, 2^100], any e: steps of a quarter, so that only the
+// last one can leave the normal range with a result that is not zero (a call to
+// ldexp would spill the accumulators around it)
+__device__ __forceinline__ double scale_far(double x, int e) {
+  e = max(-3200, min(3200, e));
+  const int e4 = e / 4;
+  const double f = __hiloint2double((1023 + e4) << 20, 0);
+  return x * f * f * f * __hiloint2double((1023 + e - 3 * e4) << 20, 0);
 }
 
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     k_gemm_oz(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, int M, int N,
               int kslices_total, int kps, const int* __restrict__ eA, const int* __restrict__ eB, double alpha,
-              double beta, double* __restrict__ C, int64_t ldc, double* __restrict__ P, int* err, uint64_t wait_ns) {
+              double beta, int scaled, int accum, double* __restrict__ C, int64_t ldc, double* __restrict__ P, int* err, uint64_t wait_ns) {
   const int kbeg = blockIdx.z * kps;
   const int kblocks = min(kps, kslices_total - kbeg);
   const int nchunks = (kblocks + OZ_CHUNK - 1) / OZ_CHUNK;
@@ -307,27 +335,60 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       }
     }
     // ---------------- epilogue ----------------
+    // One FP64 addition an element; conversions, scaling and the special cases
+    // are integer operations and selects (32 columns a warp took 20000 clocks with
+    // conversion instructions, ldexp and a branch for each case).
     const int row = m0 + q * 32 + lane;
     const bool err_set = (*(volatile int*)err) != 0;
-    if (ok && !err_set && row < M) {
-      const int ea = eA[row];
+    if (ok && !err_set) {
+      const int ea = row < M ? eA[row] : kExpZero, mycol = n0 + h * 32 + lane;
+      const int ebl = mycol < N ? eB[mycol] : kExpZero;
+      double* out = P ? P + (int64_t)blockIdx.z * M * N + row + (int64_t)(n0 + h * 32) * M
+                      : C + row + (int64_t)(n0 + h * 32) * ldc;
+      const int64_t ldo = P ? M : ldc;
+      const int nc = row < M ? min(32, N - (n0 + h * 32)) : 0;
+      const bool blend = !P && (scaled || accum);
+      bool far = false;  // a result that is not a normal number
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int col = n0 + h * 32 + j;
-        if (col >= N) continue;
-        const int eb = eB[col];
-        double v;
-        if (ea >= kExpNonFinite || eb >= kExpNonFinite)
-          v = __longlong_as_double(0x7ff8000000000000ll);  // NaN in, NaN out
-        else if (ea <= kExpZero || eb <= kExpZero)
-          v = 0.0;
-        else
-          v = ldexp(ldexp((double)Z[j], -32) + (double)F5[j], ea + eb - 14);
-        if (P) {
-          P[(int64_t)blockIdx.z * M * N + (int64_t)row + (int64_t)col * M] = v;
-        } else {
-          double* p = C + (int64_t)row + (int64_t)col * ldc;
-          *p = beta == 0.0 ? alpha * v : alpha * v + beta * (*p);
+      for (int j0 = 0; j0 < 32; j0 += 8) {
+        double x[8];
+        unsigned keep = 0;  // stored by the second pass
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int eb = __shfl_sync(0xffffffffu, ebl, j0 + j);
+          const bool zero = ea <= kExpZero || eb <= kExpZero, bad = ea >= kExpNonFinite || eb >= kExpNonFinite;
+          const double s = ll2d_scaled(Z[j0 + j], -32) + f2d_any(F5[j0 + j]);
+          const int hi = __double2hiint(s), lo = __double2loint(s), e = ea + eb - 14, ex = (hi >> 20) & 0x7ff;
+          const bool nil = zero || (((unsigned)hi << 1) == 0u && lo == 0);
+          if (!nil && !bad && !(ex + e > 0 && ex + e < 2047)) keep |= 1u << j;
+          const int rh = bad ? 0x7ff80000 : nil ? 0 : hi + (e << 20);  // NaN in, NaN out
+          x[j] = __hiloint2double(rh, bad || nil ? 0 : lo);
+        }
+        if (blend) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (scaled) x[j] *= alpha;
+            if (accum && j0 + j < nc) x[j] += beta * out[(j0 + j) * ldo];
+          }
+        }
+        far |= keep != 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j0 + j < nc && !(keep >> j & 1u)) out[(j0 + j) * ldo] = x[j];
+      }
+      if (__any_sync(0xffffffffu, far)) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const int eb = __shfl_sync(0xffffffffu, ebl, j), e = ea + eb - 14;
+          const double s = ll2d_scaled(Z[j], -32) + f2d_any(F5[j]);
+          const int ex = (__double2hiint(s) >> 20) & 0x7ff;
+          if (j < nc && ea > kExpZero && eb > kExpZero && ea < kExpNonFinite && eb < kExpNonFinite && s != 0.0 &&
+              !(ex + e > 0 && ex + e < 2047)) {
+            double v = scale_far(s, e);
+            if (!P && scaled) v *= alpha;
+            if (!P && accum) v += beta * out[j * ldo];
+            out[j * ldo] = v;
+          }
         }
       }
     }
@@ -342,13 +403,19 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 
 // C = alpha·Σ_z P[z] + beta·C (fixed order: deterministic)
 __global__ void k_oz_reduce(int64_t M, int64_t N, int splits, const double* __restrict__ P, double alpha,
-                            double beta, double* __restrict__ C, int64_t ldc) {
+                            double beta, int scaled, int accum, double* __restrict__ C, int64_t ldc) {
   const int64_t MN = M * N;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < MN; e += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
+#pragma unroll 8
     for (int z = 0; z < splits; ++z) s += P[e + z * MN];
-    const int64_t i = e % M, j = e / M;
-    C[i + j * ldc] = beta == 0.0 ? alpha * s : alpha * s + beta * C[i + j * ldc];
+    int64_t o = e;
+    if (ldc != M) {  // 64-bit quotients are subroutines
+      const int64_t j = MN < (1ll << 32) ? (int64_t)((uint32_t)e / (uint32_t)M) : e / M;
+      o = e - j * M + j * ldc;
+    }
+    if (scaled) s *= alpha;
+    C[o] = accum ? s + beta * C[o] : s;
   }
 }
 
@@ -402,49 +469,44 @@ void gemm_fp64tc(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K,
   const int64_t Mp = (M + OZ_BM - 1) / OZ_BM * OZ_BM, Np = (N + OZ_BN - 1) / OZ_BN * OZ_BN;
   const int64_t Kp = (K + OZ_KS - 1) / OZ_KS * OZ_KS;
   WsScope scope(c);
-  int* eA = (int*)c->ws.alloc((size_t)Mp * sizeof(int));
-  int* eB = (int*)c->ws.alloc((size_t)Np * sizeof(int));
+  int* eA = (int*)c->ws.alloc((size_t)(Mp + Np) * sizeof(int));
+  int* eB = eA + Mp;
   __nv_bfloat16* pa = (__nv_bfloat16*)c->ws.alloc((size_t)OZ_S * Mp * Kp * 2);
   __nv_bfloat16* pb = (__nv_bfloat16*)c->ws.alloc((size_t)OZ_S * Np * Kp * 2);
-  TNAD_CK(cudaMemsetAsync(eA, 0x80, (size_t)Mp * sizeof(int), c->stream));
-  TNAD_CK(cudaMemsetAsync(eB, 0x80, (size_t)Np * sizeof(int), c->stream));
-  const int ita = (ta == 'T' || ta == 't'), itb = (tb == 'T' || tb == 't');
+  TNAD_CK(cudaMemsetAsync(eA, 0x80, (size_t)(Mp + Np) * sizeof(int), c->stream));
   // op(B)ᵀ (N rows, K contiguous) is read as B untransposed with tr = !itb
-  {
-    dim3 g((unsigned)(Kp / 32), (unsigned)((M + 31) / 32)), b(32, 8);
-    k_oz_exp<<<g, b, 0, c->stream>>>(A, lda, ita, M, K, eA);
-    dim3 g2((unsigned)(Kp / 32), (unsigned)((N + 31) / 32));
-    k_oz_exp<<<g2, b, 0, c->stream>>>(B, ldb, itb ? 0 : 1, N, K, eB);
-    dim3 g3((unsigned)(Kp / 32), (unsigned)(Mp / 32));
-    k_oz_slice<<<g3, b, 0, c->stream>>>(A, lda, ita, M, K, Mp, Kp, eA, pa);
-    dim3 g4((unsigned)(Kp / 32), (unsigned)(Np / 32));
-    k_oz_slice<<<g4, b, 0, c->stream>>>(B, ldb, itb ? 0 : 1, N, K, Np, Kp, eB, pb);
-  }
-  count_launch(c, 4);
+  const int ita = (ta == 'T' || ta == 't'), itb = (tb == 'T' || tb == 't');
+  const OzIn ia{A, lda, M, Mp, ita, eA, pa}, ib{B, ldb, N, Np, itb ? 0 : 1, eB, pb};
+  const unsigned g = (unsigned)(Kp / 32 * ((Mp + Np) / 32));
+  const dim3 b(32, 8);
+  k_oz_exp<<<g, b, 0, c->stream>>>(ia, ib, (int)(Mp / 32), K, Kp);
+  k_oz_slice<<<g, b, 0, c->stream>>>(ia, ib, (int)(Mp / 32), K, Kp);
+  count_launch(c, 2);
   check_launch(c, "oz_slice");
   const CUtensorMap tA = make_plane_map(pa, Kp, Mp, OZ_BM);
   const CUtensorMap tB = make_plane_map(pb, Kp, Np, OZ_BN);
-  // split K over CTAs: about one wave of the GPU, at least one chunk per split,
-  // at most 32768 K values per CTA (int32 running sums)
+  // split K over CTAs: about one wave of the GPU, one chunk or at least two slices
+  // per split (a slice is 3300 clocks of products, a partial to add ~200), whole chunks
+  // above one; at most 32768 K values per CTA (int32 running sums)
   const int kst = (int)(Kp / OZ_KS);
   const int64_t tiles = (Mp / OZ_BM) * (Np / OZ_BN);
   int splits = (int)std::max<int64_t>(1, std::min<int64_t>((c->sm_count + tiles - 1) / tiles,
-                                                           (kst + OZ_CHUNK - 1) / OZ_CHUNK));
+                                                           kst > OZ_CHUNK ? (kst + 1) / 2 : 1));
   splits = std::max(splits, (kst + OZ_MAX_SLICES_PER_CTA - 1) / OZ_MAX_SLICES_PER_CTA);
   int kps = (kst + splits - 1) / splits;
-  kps = (kps + OZ_CHUNK - 1) / OZ_CHUNK * OZ_CHUNK;
+  if (kps > OZ_CHUNK) kps = (kps + OZ_CHUNK - 1) / OZ_CHUNK * OZ_CHUNK;
   splits = (kst + kps - 1) / kps;
   double* Pp = splits > 1 ? ws_d(c, (int64_t)splits * M * N) : nullptr;
   KernelTimer kt(c, "gemm_fp64tc", 2.0 * (double)M * (double)N * (double)K);  // logical FP64 flops
   dim3 grid((unsigned)(Mp / OZ_BM), (unsigned)(Np / OZ_BN), (unsigned)splits);
-  k_gemm_oz<<<grid, OZ_THREADS, OZ_SMEM, c->stream>>>(tA, tB, (int)M, (int)N, kst, kps, eA, eB, alpha, beta, Cm, ldc,
-                                                       Pp, c->d_flag + 8, 2000000000ull);
+  k_gemm_oz<<<grid, OZ_THREADS, OZ_SMEM, c->stream>>>(tA, tB, (int)M, (int)N, kst, kps, eA, eB, alpha, beta, alpha != 1.0,
+                                                       beta != 0.0, Cm, ldc, Pp, c->d_flag + 8, 2000000000ull);
   count_launch(c);
   check_launch(c, "gemm_fp64tc");
   if (Pp) {
     const int64_t MN = M * N;
     k_oz_reduce<<<(int)std::min<int64_t>((MN + 255) / 256, 4096), 256, 0, c->stream>>>(M, N, splits, Pp, alpha, beta,
-                                                                                      Cm, ldc);
+                                                                                      alpha != 1.0, beta != 0.0, Cm, ldc);
     count_launch(c);
     check_launch(c, "oz_reduce");
   }

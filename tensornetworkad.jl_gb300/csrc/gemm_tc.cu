@@ -28,6 +28,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "fp64_fast.cuh"
 #include "tc_common.cuh"
 #include "tnad_internal.h"
 
@@ -58,15 +59,53 @@ __device__ __forceinline__ float tf32_rn(float x) {
   return __uint_as_float(r);
 }
 
+// alpha·s + beta·C, with what the launch knows of the factors: an FP64 product
+// or comparison takes 64 clocks of a warp's quadrant, a conversion ~95.  Four of
+// them on each of a CTA's 128 columns cost 16 µs of a 20 µs product, so the
+// comparisons are the host's, a factor 1 is not multiplied, and conversions are
+// integer operations.
+struct Blend {
+  double alpha, beta;
+  int scaled, accum;  // alpha ≠ 1, beta ≠ 0
+};
+
+template <typename OutT>
+__device__ __forceinline__ OutT combine(double s, const Blend& b, OutT old) {
+  if (b.scaled) s *= b.alpha;
+  if constexpr (sizeof(OutT) == 4) {
+    if (b.accum) s += b.beta * f2d_any(old);
+    return d2f_rn(s);
+  } else {
+    if (b.accum) s += b.beta * old;
+    return s;
+  }
+}
+
+// the accumulator as it is stored with alpha = 1, beta = 0
+template <typename OutT>
+__device__ __forceinline__ OutT stored(float v) {
+  if constexpr (sizeof(OutT) == 4) return v;
+  else return f2d_any(v);
+}
+
+// what TcEpi asks for, on the stored value (selects: a branch an element costs
+// more than the rest of its epilogue); the FP64 products take no such step
+__device__ __forceinline__ double epilogue(const TcEpi&, double v, float, float) { return v; }
+__device__ __forceinline__ float epilogue(const TcEpi& ep, float v, float bias, float mask) {
+  v = ep.bias ? v + bias : v;
+  v = ep.relu ? fmaxf(v, 0.f) : v;
+  return mask > 0.f ? v : 0.f;
+}
+
 template <int BN, bool SPLIT, typename OutT>
 __global__ void __launch_bounds__(128, 1)
     k_gemm_tc(const __grid_constant__ CUtensorMap tAh, const __grid_constant__ CUtensorMap tAl,
               const __grid_constant__ CUtensorMap tBh, const __grid_constant__ CUtensorMap tBl, int M, int N,
-              int kblocks_total, int kps, double alpha, double beta, OutT* __restrict__ C, int64_t ldc,
-              double* __restrict__ P, int* err, uint64_t wait_ns, int withhold_first) {
+              int kblocks_total, int kps, Blend bl, OutT* __restrict__ C, int64_t ldc,
+              float* __restrict__ P, TcEpi ep, int* err, uint64_t wait_ns, int withhold_first) {
   using CF = Cfg<BN, SPLIT>;
   // split-K: CTA z owns K slices [kbeg, kbeg + kblocks); with P != null it
-  // writes its raw FP32 sum as an FP64 partial, reduced in FP64 afterwards
+  // writes its raw FP32 sum, and the partials are reduced in FP64 afterwards
   const int kbeg = blockIdx.z * kps;
   const int kblocks = min(kps, kblocks_total - kbeg);
   extern __shared__ uint8_t smem_raw[];
@@ -169,6 +208,7 @@ __global__ void __launch_bounds__(128, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const int row = m0 + warp * 32 + lane;
   const bool err_set = (*(volatile int*)err) != 0;
+  const float bias = ep.bias && row < M ? ep.bias[row] : 0.f;
 #pragma unroll 1
   for (int c0 = 0; c0 < BN; c0 += 16) {
     uint32_t v[16];
@@ -182,21 +222,42 @@ __global__ void __launch_bounds__(128, 1)
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     if (okd && !err_set && row < M) {
       if (P) {
-        double* Pz = P + (int64_t)blockIdx.z * M * N;
+        float* Pz = P + (int64_t)blockIdx.z * M * N;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int col = n0 + c0 + j;
-          if (col < N) Pz[(int64_t)row + (int64_t)col * M] = (double)__uint_as_float(v[j]);
+          if (col < N) Pz[(int64_t)row + (int64_t)col * M] = __uint_as_float(v[j]);
         }
       } else {
+        // what an element still needs is read for all 16 columns before the first
+        // store: a load behind a store that may alias it waits out its latency
+        const int nc = min(16, N - (n0 + c0));
+        OutT* p = C + (int64_t)row + (int64_t)(n0 + c0) * ldc;
+        if (!bl.scaled && !bl.accum) {
+          float mk[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int col = n0 + c0 + j;
-          if (col < N) {
-            double r = alpha * (double)__uint_as_float(v[j]);
-            OutT* p = C + (int64_t)row + (int64_t)col * ldc;
-            *p = (OutT)(beta == 0.0 ? r : r + beta * (double)(*p));
+          for (int j = 0; j < 16; ++j) mk[j] = 1.f;
+          if (ep.mask) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (j < nc) mk[j] = ep.mask[(int64_t)row + (int64_t)(n0 + c0 + j) * ldc];
           }
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < nc) p[(int64_t)j * ldc] = epilogue(ep, stored<OutT>(__uint_as_float(v[j])), bias, mk[j]);
+        } else {
+          OutT old[16];
+          float mk[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            old[j] = bl.accum && j < nc ? p[(int64_t)j * ldc] : OutT(0);
+            mk[j] = ep.mask && j < nc ? ep.mask[(int64_t)row + (int64_t)(n0 + c0 + j) * ldc] : 1.f;
+          }
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < nc)
+              p[(int64_t)j * ldc] =
+                  epilogue(ep, combine<OutT>(f2d_any(__uint_as_float(v[j])), bl, old[j]), bias, mk[j]);
         }
       }
     }
@@ -209,53 +270,75 @@ __global__ void __launch_bounds__(128, 1)
   }
 }
 
-// op(X) (rows × K, from FP64 column-major with leading dim ld, transposed when
-// tr) → K-major hi/lo FP32 planes of size rows_pad × k_pad.
-__global__ void k_pack_split(const double* __restrict__ X, int64_t ld, int tr, int64_t rows, int64_t K,
-                             int64_t rows_pad, int64_t k_pad, float* __restrict__ hi, float* __restrict__ lo) {
-  // 32×32 tiles through shared memory: reads coalesced in the source's fast
-  // index, writes coalesced along K.
-  __shared__ double tile[32][33];
-  const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
+// One operand of a product as the pack kernels read it: op(X) is rows × K,
+// column-major with leading dimension ld, transposed when tr.
+template <typename T>
+struct PackIn {
+  const T* X;
+  int64_t ld, rows, rows_pad;
+  int tr;
+};
+
+// 32×32 tile of op(X) through shared memory: reads coalesced in the source's
+// fast index, the caller's writes coalesced along K.
+template <typename T>
+__device__ __forceinline__ void pack_tile(const PackIn<T>& in, int64_t r0, int64_t k0, int64_t K, T (*tile)[33]) {
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 × 8
+#pragma unroll
   for (int j = ty; j < 32; j += 8) {
     // tile[rr][kk] = op(X)(r0+rr, k0+kk)
     int64_t r, k;
-    if (!tr) { r = r0 + tx; k = k0 + j; } else { k = k0 + tx; r = r0 + j; }
-    double v = 0.0;
-    if (r < rows && k < K) v = !tr ? X[r + k * ld] : X[k + r * ld];
-    if (!tr) tile[tx][j] = v; else tile[j][tx] = v;
+    if (!in.tr) { r = r0 + tx; k = k0 + j; } else { k = k0 + tx; r = r0 + j; }
+    T v = T(0);
+    if (r < in.rows && k < K) v = !in.tr ? in.X[r + k * in.ld] : in.X[k + r * in.ld];
+    if (!in.tr) tile[tx][j] = v; else tile[j][tx] = v;
   }
   __syncthreads();
+}
+
+// Both operands of a product in one launch (tile rows [0, nya) are A's,
+// on a one-dimensional grid: the sum of both heights has no limit of its own): the
+// products here take 5 to 15 µs, so that a launch of its own for each operand
+// (5 µs, its gap included) is a third of the product.
+// op(X) in FP64 → K-major hi/lo FP32 planes of rows_pad × k_pad.
+__global__ void k_pack_split(PackIn<double> a, PackIn<double> b, int nya, int64_t K, int64_t k_pad,
+                             float* __restrict__ ahi, float* __restrict__ alo, float* __restrict__ bhi,
+                             float* __restrict__ blo) {
+  __shared__ double tile[32][33];
+  const int nk = (int)((k_pad + 31) / 32), by = (int)blockIdx.x / nk, bx = (int)blockIdx.x % nk;
+  const bool isa = by < nya;
+  const PackIn<double> in = isa ? a : b;
+  float* hi = isa ? ahi : bhi;
+  float* lo = isa ? alo : blo;
+  const int64_t r0 = (int64_t)(isa ? by : by - nya) * 32, k0 = (int64_t)bx * 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  pack_tile(in, r0, k0, K, tile);
   for (int j = ty; j < 32; j += 8) {
     const int64_t r = r0 + j, k = k0 + tx;
-    if (r < rows_pad && k < k_pad) {
+    if (r < in.rows_pad && k < k_pad) {
       const double x = tile[j][tx];
-      const float h = tf32_rn((float)x);
-      const float l = tf32_rn((float)(x - (double)h));
+      const float h = tf32_rn(d2f_rn(x));
+      const float l = tf32_rn(d2f_rn(x - f2d_any(h)));
       hi[r * k_pad + k] = h;
       lo[r * k_pad + k] = l;
     }
   }
 }
 
-// op(X) (rows × K, FP32 column-major) → one K-major BF16 plane, zero padded
-__global__ void k_pack_bf16(const float* __restrict__ X, int64_t ld, int tr, int64_t rows, int64_t K,
-                            int64_t rows_pad, int64_t k_pad, __nv_bfloat16* __restrict__ out) {
+// op(X) in FP32 → one K-major BF16 plane, zero padded
+__global__ void k_pack_bf16(PackIn<float> a, PackIn<float> b, int nya, int64_t K, int64_t k_pad,
+                            __nv_bfloat16* __restrict__ aout, __nv_bfloat16* __restrict__ bout) {
   __shared__ float tile[32][33];
-  const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 × 8
-  for (int j = ty; j < 32; j += 8) {
-    int64_t r, k;
-    if (!tr) { r = r0 + tx; k = k0 + j; } else { k = k0 + tx; r = r0 + j; }
-    float v = 0.f;
-    if (r < rows && k < K) v = !tr ? X[r + k * ld] : X[k + r * ld];
-    if (!tr) tile[tx][j] = v; else tile[j][tx] = v;
-  }
-  __syncthreads();
+  const int nk = (int)((k_pad + 31) / 32), by = (int)blockIdx.x / nk, bx = (int)blockIdx.x % nk;
+  const bool isa = by < nya;
+  const PackIn<float> in = isa ? a : b;
+  __nv_bfloat16* out = isa ? aout : bout;
+  const int64_t r0 = (int64_t)(isa ? by : by - nya) * 32, k0 = (int64_t)bx * 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  pack_tile(in, r0, k0, K, tile);
   for (int j = ty; j < 32; j += 8) {
     const int64_t r = r0 + j, k = k0 + tx;
-    if (r < rows_pad && k < k_pad) out[r * k_pad + k] = __float2bfloat16_rn(tile[j][tx]);
+    if (r < in.rows_pad && k < k_pad) out[r * k_pad + k] = __float2bfloat16_rn(tile[j][tx]);
   }
 }
 
@@ -263,15 +346,21 @@ constexpr int kChunkBlocks = 4;  // 4 × 32 = 128 K values per FP32 tensor-core 
 
 // C = alpha·Σ_z P[z] + beta·C   (fixed order: deterministic)
 template <typename OutT>
-__global__ void k_splitk_sum(int64_t M, int64_t N, int splits, const double* __restrict__ P, double alpha,
-                             double beta, OutT* __restrict__ C, int64_t ldc) {
+__global__ void k_splitk_sum(int64_t M, int64_t N, int splits, const float* __restrict__ P, Blend bl,
+                             OutT* __restrict__ C, int64_t ldc, TcEpi ep) {
   const int64_t MN = M * N;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < MN; e += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int z = 0; z < splits; ++z) s += P[e + z * MN];
-    const int64_t i = e % M, j = e / M;
-    const double r = alpha * s;
-    C[i + j * ldc] = (OutT)(beta == 0.0 ? r : r + beta * (double)C[i + j * ldc]);
+#pragma unroll 4
+    for (int z = 0; z < splits; ++z) s += f2d_any(P[e + z * MN]);
+    int64_t i = 0, o = e;
+    if (ldc != M || ep.bias) {  // 64-bit quotients are subroutines
+      const int64_t j = MN < (1ll << 32) ? (int64_t)((uint32_t)e / (uint32_t)M) : e / M;
+      i = e - j * M;
+      o = i + j * ldc;
+    }
+    C[o] = epilogue(ep, combine<OutT>(s, bl, bl.accum ? C[o] : OutT(0)), ep.bias ? ep.bias[i] : 0.f,
+                    ep.mask ? ep.mask[o] : 1.f);
   }
 }
 
@@ -297,7 +386,8 @@ CUtensorMap make_map(void* base, int64_t k_pad, int64_t rows_pad, int box_rows, 
 
 template <int BN, bool SPLIT, typename OutT>
 void launch_tc(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, void* Ah, void* Al, void* Bh, void* Bl,
-               int64_t Mp, int64_t Np, int64_t Kp, double beta, OutT* Cm, int64_t ldc, const char* timer_name) {
+               int64_t Mp, int64_t Np, int64_t Kp, double beta, OutT* Cm, int64_t ldc, const char* timer_name,
+               const TcEpi& ep = TcEpi{}) {
   using CF = Cfg<BN, SPLIT>;
   static std::atomic<bool> attr{false};
   if (!attr) {
@@ -318,7 +408,8 @@ void launch_tc(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, void*
   dim3 grid((unsigned)(Mp / BM), (unsigned)(Np / BN), (unsigned)splits);
   int* err = c->d_flag + 8;
   WsScope scope(c);
-  double* P = splits > 1 ? ws_d(c, (int64_t)splits * M * N) : nullptr;
+  float* P = splits > 1 ? ws_f(c, (int64_t)splits * M * N) : nullptr;
+  const Blend bl{alpha, beta, alpha != 1.0, beta != 0.0};
   int withhold = 0;
   uint64_t wait_ns = 2000000000ull;
   if (c->fault_once == kFaultTcWithhold) {
@@ -327,14 +418,14 @@ void launch_tc(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, void*
     c->fault_once = kFaultNone;
   }
   KernelTimer kt(c, timer_name, 2.0 * (double)M * (double)N * (double)K);  // logical flops
-  k_gemm_tc<BN, SPLIT, OutT><<<grid, 128, CF::SMEM, c->stream>>>(tAh, tAl, tBh, tBl, (int)M, (int)N, kbt, kps, alpha,
-                                                                 beta, Cm, ldc, P, err, wait_ns, withhold);
+  k_gemm_tc<BN, SPLIT, OutT><<<grid, 128, CF::SMEM, c->stream>>>(tAh, tAl, tBh, tBl, (int)M, (int)N, kbt, kps, bl,
+                                                                 Cm, ldc, P, ep, err, wait_ns, withhold);
   count_launch(c);
   check_launch(c, timer_name);
   if (P) {
     const int64_t MN = M * N;
-    k_splitk_sum<OutT><<<(int)std::min<int64_t>((MN + 255) / 256, 4096), 256, 0, c->stream>>>(M, N, splits, P,
-                                                                                            alpha, beta, Cm, ldc);
+    k_splitk_sum<OutT><<<(int)std::min<int64_t>((MN + 255) / 256, 4096), 256, 0, c->stream>>>(M, N, splits, P, bl, Cm,
+                                                                                            ldc, ep);
     count_launch(c);
     check_launch(c, "splitk_sum");
   }
@@ -361,17 +452,12 @@ void gemm_tf32x3(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K,
   float* Bh = ws_f(c, Np * Kp);
   float* Bl = ws_f(c, Np * Kp);
   const int ita = (ta == 'T' || ta == 't'), itb = (tb == 'T' || tb == 't');
-  {
-    dim3 g((unsigned)(Kp / 32), (unsigned)(Mp / 32)), b(32, 8);
-    k_pack_split<<<g, b, 0, c->stream>>>(A, lda, ita, M, K, Mp, Kp, Ah, Al);
-  }
-  {
-    // op(B) is K×N; the packed operand is op(B)ᵀ (N rows, K contiguous): rows of
-    // op(B)ᵀ are columns of op(B), i.e. (B, not transposed) read with tr = !itb.
-    dim3 g((unsigned)(Kp / 32), (unsigned)(Np / 32)), b(32, 8);
-    k_pack_split<<<g, b, 0, c->stream>>>(B, ldb, itb ? 0 : 1, N, K, Np, Kp, Bh, Bl);
-  }
-  count_launch(c, 2);
+  // op(B) is K×N; the packed operand is op(B)ᵀ (N rows, K contiguous): rows of
+  // op(B)ᵀ are columns of op(B), i.e. (B, not transposed) read with tr = !itb.
+  k_pack_split<<<(unsigned)(Kp / 32 * ((Mp + Np) / 32)), dim3(32, 8), 0, c->stream>>>(
+      PackIn<double>{A, lda, M, Mp, ita}, PackIn<double>{B, ldb, N, Np, itb ? 0 : 1}, (int)(Mp / 32), K, Kp, Ah, Al,
+      Bh, Bl);
+  count_launch(c);
   check_launch(c, "pack_split");
   if (BN == 128)
     launch_tc<128, true, double>(c, M, N, K, alpha, Ah, Al, Bh, Bl, Mp, Np, Kp, beta, Cm, ldc, "gemm_tf32x3");
@@ -380,7 +466,7 @@ void gemm_tf32x3(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K,
 }
 
 void gemm_bf16(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, float alpha, const float* A,
-               int64_t lda, const float* B, int64_t ldb, float beta, float* Cm, int64_t ldc) {
+               int64_t lda, const float* B, int64_t ldb, float beta, float* Cm, int64_t ldc, const TcEpi& ep) {
   if (M <= 0 || N <= 0) return;
   TNAD_REQUIRE(c->tc_ok, TNAD_ERR_STATE, "BF16 GEMM needs an sm_100-family GPU (tcgen05)");
   TNAD_REQUIRE(K > 0 && M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), TNAD_ERR_ARG, "gemm_bf16: size");
@@ -390,20 +476,16 @@ void gemm_bf16(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, f
   __nv_bfloat16* Ab = (__nv_bfloat16*)c->ws.alloc((size_t)Mp * Kp * 2);
   __nv_bfloat16* Bb = (__nv_bfloat16*)c->ws.alloc((size_t)Np * Kp * 2);
   const int ita = (ta == 'T' || ta == 't'), itb = (tb == 'T' || tb == 't');
-  {
-    dim3 g((unsigned)(Kp / 32), (unsigned)(Mp / 32)), b(32, 8);
-    k_pack_bf16<<<g, b, 0, c->stream>>>(A, lda, ita, M, K, Mp, Kp, Ab);
-  }
-  {
-    dim3 g((unsigned)(Kp / 32), (unsigned)(Np / 32)), b(32, 8);
-    k_pack_bf16<<<g, b, 0, c->stream>>>(B, ldb, itb ? 0 : 1, N, K, Np, Kp, Bb);
-  }
-  count_launch(c, 2);
+  k_pack_bf16<<<(unsigned)(Kp / 32 * ((Mp + Np) / 32)), dim3(32, 8), 0, c->stream>>>(
+      PackIn<float>{A, lda, M, Mp, ita}, PackIn<float>{B, ldb, N, Np, itb ? 0 : 1}, (int)(Mp / 32), K, Kp, Ab, Bb);
+  count_launch(c);
   check_launch(c, "pack_bf16");
   if (BN == 128)
-    launch_tc<128, false, float>(c, M, N, K, alpha, Ab, nullptr, Bb, nullptr, Mp, Np, Kp, beta, Cm, ldc, "gemm_bf16");
+    launch_tc<128, false, float>(c, M, N, K, alpha, Ab, nullptr, Bb, nullptr, Mp, Np, Kp, beta, Cm, ldc, "gemm_bf16",
+                                  ep);
   else
-    launch_tc<64, false, float>(c, M, N, K, alpha, Ab, nullptr, Bb, nullptr, Mp, Np, Kp, beta, Cm, ldc, "gemm_bf16");
+    launch_tc<64, false, float>(c, M, N, K, alpha, Ab, nullptr, Bb, nullptr, Mp, Np, Kp, beta, Cm, ldc, "gemm_bf16",
+                                  ep);
 }
 
 EncodeTiledFn tensor_map_encoder() {

@@ -65,14 +65,6 @@ __global__ void k_init_uniform(float* __restrict__ P, int64_t n, uint64_t seed, 
   }
 }
 
-// H[r, j] = act(H[r, j] + b[r])
-__global__ void k_bias_act(float* __restrict__ H, const float* __restrict__ b, int rows, int64_t n, int relu) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-    const float v = H[e] + b[e % rows];
-    H[e] = relu ? fmaxf(v, 0.f) : v;
-  }
-}
-
 // dst[:, j] = src[:, idx[j]]
 __global__ void k_gather_cols(const float* __restrict__ src, int rows, const int* __restrict__ idx, int B,
                               float* __restrict__ dst) {
@@ -118,19 +110,24 @@ __global__ void k_sum_partials(const double* __restrict__ part, int nb, double i
   }
 }
 
-// db[r] = Σ_j dH[r, j]
-__global__ void k_rowsum(const float* __restrict__ dH, int rows, int B, float* __restrict__ db) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
+// db[r] = Σ_j dH[r, j].  A block takes 32 rows, its 32 warps the columns in
+// turn (coalesced: a warp reads 32 rows of one column), and the warps' FP64 sums
+// are added in a fixed order.  A thread per row alone walks the batch's columns
+// one load latency after another.
+__global__ void __launch_bounds__(1024) k_rowsum(const float* __restrict__ dH, int rows, int B,
+                                                 float* __restrict__ db) {
+  __shared__ double sh[32][33];
+  const int tx = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r = blockIdx.x * 32 + tx;
   double s = 0.0;
-  for (int j = 0; j < B; ++j) s += (double)dH[r + (int64_t)j * rows];
-  db[r] = (float)s;
-}
-
-// dH ∘= [H > 0]
-__global__ void k_relu_mask(float* __restrict__ dH, const float* __restrict__ H, int64_t n) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
-    if (!(H[e] > 0.f)) dH[e] = 0.f;
+  if (r < rows)
+    for (int j = w; j < B; j += 32) s += (double)dH[r + (int64_t)j * rows];
+  sh[w][tx] = s;
+  __syncthreads();
+  if (w == 0 && r < rows) {
+    for (int i = 1; i < 32; ++i) s += sh[i][tx];
+    db[r] = (float)s;
+  }
 }
 
 struct BiasRanges {
@@ -326,10 +323,8 @@ void mlp_forward(tnad_ctx* c, tnad_mlp* net, const float* X, int B) {
   const float* in = X;
   for (int l = 0; l < 3; ++l) {
     const int m = net->rows[l + 1], k = net->rows[l];
-    gemm_bf16(c, 'N', 'N', m, B, k, 1.f, net->P + net->off_w[l], m, in, k, 0.f, net->H[l], m);
-    k_bias_act<<<nblk((int64_t)m * B), 256, 0, c->stream>>>(net->H[l], net->P + net->off_b[l], m, (int64_t)m * B,
-                                                            l < 2 ? 1 : 0);
-    count_launch(c);
+    const TcEpi ep{net->P + net->off_b[l], nullptr, l < 2 ? 1 : 0};  // H = act(W·in + b)
+    gemm_bf16(c, 'N', 'N', m, B, k, 1.f, net->P + net->off_w[l], m, in, k, 0.f, net->H[l], m, ep);
     in = net->H[l];
   }
   check_launch(c, "mlp_forward");
@@ -346,12 +341,11 @@ void mlp_backward(tnad_ctx* c, tnad_mlp* net, const float* X, const float* Y, in
     const int m = net->rows[l + 1], k = net->rows[l];
     const float* in = l > 0 ? net->H[l - 1] : X;
     gemm_bf16(c, 'N', 'T', m, k, B, 1.f, net->dH[l], m, in, k, 0.f, net->G + net->off_w[l], m);
-    k_rowsum<<<(m + 255) / 256, 256, 0, c->stream>>>(net->dH[l], m, B, net->G + net->off_b[l]);
+    k_rowsum<<<(m + 31) / 32, 1024, 0, c->stream>>>(net->dH[l], m, B, net->G + net->off_b[l]);
     count_launch(c);
     if (l > 0) {
-      gemm_bf16(c, 'T', 'N', k, B, m, 1.f, net->P + net->off_w[l], m, net->dH[l], m, 0.f, net->dH[l - 1], k);
-      k_relu_mask<<<nblk((int64_t)k * B), 256, 0, c->stream>>>(net->dH[l - 1], net->H[l - 1], (int64_t)k * B);
-      count_launch(c);
+      const TcEpi ep{nullptr, net->H[l - 1], 0};  // dH_{l-1} = (Wᵀ·dH) ∘ [H_{l-1} > 0]
+      gemm_bf16(c, 'T', 'N', k, B, m, 1.f, net->P + net->off_w[l], m, net->dH[l], m, 0.f, net->dH[l - 1], k, ep);
     }
   }
   check_launch(c, "mlp_backward");

@@ -232,10 +232,18 @@ bool gemm_is_f64(const tnad_ctx* c, int prec, int64_t M, int64_t N, int64_t K);
 void gemm_tf32x3(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, double alpha,
                  const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
                  double* C, int64_t ldc);
+// What a network layer does to each element of a product while it is stored:
+// add its row's bias, clamp at zero, or clear it where mask (C's layout) is not
+// positive; null / 0 for nothing.
+struct TcEpi {
+  const float* bias = nullptr;
+  const float* mask = nullptr;
+  int relu = 0;
+};
 // FP32 C(M×N) = alpha·op(A)·op(B) + beta·C with operands rounded to BF16 and FP32
 // accumulation on tcgen05 tensor cores (chunks of 512 K values summed in FP64).
 void gemm_bf16(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, float alpha, const float* A,
-               int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc);
+               int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc, const TcEpi& ep = TcEpi{});
 // Same contract, FP64-accurate (about 2^−47 of the row/column scales) from BF16
 // slices on the tcgen05 tensor cores (gemm_oz.cu); unless `always`, products
 // below a few million multiply-adds go to gemm_f64 (as fast there).
