@@ -27,7 +27,7 @@
 
 namespace tnad {
 
-void chol_inv_upper(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* dev_fail);
+void chol_inv_upper(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* dev_fail, float near = 0.f);
 void randn(tnad_ctx* c, double* x, int64_t n, uint64_t seed, double scale, bool accumulate,
            const double* dev_sumsq = nullptr);
 
@@ -162,7 +162,10 @@ void cholqr2(tnad_ctx* c, int prec, const double* Y, int64_t n, int64_t p, doubl
   const double* src = t;
   for (int pass = 0; pass < 2; ++pass) {
     gemm(c, TNAD_PREC_FP64, 'T', 'N', p, p, n, 1.0, src, n, src, n, 0.0, G, p);
-    chol_inv_upper(c, G, p, Ri, fail);
+    // second pass: a Gram matrix that is the identity up to what the next product
+    // rounds (2^-21 in 3xTF32, 2^-53) needs no factorisation
+    const float near = pass == 0 ? 0.f : prec == TNAD_PREC_FP64 ? 0x1p-55f : 0x1p-26f;
+    chol_inv_upper(c, G, p, Ri, fail, near);
     gemm(c, prec, 'N', 'N', n, p, p, 1.0, src, n, Ri, p, 0.0, Q, n);
     if (pass == 0) {
       copy_d2d(c, t, Q, n * p);

@@ -45,23 +45,52 @@ constexpr int kCholMaxP = 160;
 constexpr int kCholLd = kCholMaxP + 1;  // column stride; slot kCholMaxP holds 1/L_kk
 constexpr int kCholPanels = (kCholMaxP / kCholNB + kCholC - 1) / kCholC;  // panels of one CTA
 
-__global__ void __launch_bounds__(256) k_chol_inv(const double* __restrict__ G, int p, double floor_rel,
+__global__ void __launch_bounds__(256) k_chol_inv(const double* __restrict__ G, int p, double floor_rel, float near,
                                                   double* __restrict__ Rinv, int* __restrict__ fail) {
   extern __shared__ __align__(16) double csm[];
   double* A = csm;                                        // own columns of L, kCholPanels·8 × kCholLd
   double* Y = A + kCholPanels * kCholNB * kCholLd;        // own columns of L⁻¹
   double* Lp = Y + kCholPanels * kCholNB * kCholLd;       // the current panel, 8 × kCholLd
   __shared__ double fl_sh;
+  __shared__ unsigned emax_sh;  // FP32 bits of max|E| over the own columns
   const int rank = blockIdx.x;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int np = (p + kCholNB - 1) / kCholNB;
   auto gcol = [&](int lc) { return ((lc / kCholNB) * kCholC + rank) * kCholNB + lc % kCholNB; };
+  if (threadIdx.x == 0) emax_sh = 0u;
+  __syncthreads();
+  unsigned emax = 0u;
   for (int lc = w; lc < kCholPanels * kCholNB; lc += 8) {
     const int j = gcol(lc);
     if (j >= p) continue;
     for (int i = lane; i < p; i += 32) {
-      A[lc * kCholLd + i] = G[i + (int64_t)j * p];
+      const double g = G[i + (int64_t)j * p];
+      A[lc * kCholLd + i] = g;
       Y[lc * kCholLd + i] = i == j ? 1.0 : 0.0;
+      if (near > 0.f) emax = max(emax, __float_as_uint(fabsf(d2f_rn(i == j ? g - 1.0 : g))));  // NaN: above all
+    }
+  }
+  if (near > 0.f) {
+    atomicMax(&emax_sh, emax);
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(remote)
+                 : "r"((uint32_t)__cvta_generic_to_shared(&emax_sh)), "r"(lane % kCholC));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(emax) : "r"(remote));
+    for (int o = 16; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+    const float e = __uint_as_float(emax);
+    if ((float)p * e * e <= near) {  // false for NaN
+      for (int lc = w; lc < kCholPanels * kCholNB; lc += 8) {
+        const int j = gcol(lc);
+        if (j >= p) continue;
+        for (int i = lane; i < p; i += 32) {
+          const double g = A[lc * kCholLd + i];
+          Rinv[i + (int64_t)j * p] = i > j ? 0.0 : i < j ? -g : fma(-0.5, g, 1.5);
+        }
+      }
+      asm volatile("barrier.cluster.arrive;\nbarrier.cluster.wait;" ::: "memory");  // emax_sh was read
+      return;
     }
   }
   if (w == 0) {
@@ -201,7 +230,7 @@ __global__ void __launch_bounds__(256) k_chol_inv(const double* __restrict__ G, 
   asm volatile("barrier.cluster.arrive;\nbarrier.cluster.wait;" ::: "memory");
 }
 
-void chol_inv_upper(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* dev_fail) {
+void chol_inv_upper(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* dev_fail, float near) {
   TNAD_REQUIRE(p >= 1 && p <= kCholMaxP, TNAD_ERR_SHAPE, "chol_inv_upper: p must be in [1,160]");
   constexpr size_t smem = (size_t)(2 * kCholPanels + 1) * kCholNB * kCholLd * sizeof(double);
   static std::atomic<bool> attr{false};
@@ -223,7 +252,7 @@ void chol_inv_upper(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* 
   at[0].val.clusterDim.z = 1;
   cf.attrs = at;
   cf.numAttrs = 1;
-  TNAD_CK(cudaLaunchKernelEx(&cf, k_chol_inv, G, (int)p, kPivotFloor, Rinv, dev_fail));
+  TNAD_CK(cudaLaunchKernelEx(&cf, k_chol_inv, G, (int)p, kPivotFloor, near, Rinv, dev_fail));
   count_launch(c);
   check_launch(c, "chol_inv");
 }

@@ -7,7 +7,8 @@ panels of the Cholesky cluster with and without a remainder (p = 8, 12, 20, 22,
 33, 49), 32-row chunks of the FP32 eigensolver (p = 32, 33, 64, 96, 97, 128, 129)
 and its largest size (160); the gauge alignment's polar factor takes χ, whose
 4×4 tiles end inside or at the matrix.  Uniform tensors have rank-deficient
-blocks (the pivot floor), N(0,1) ones have not.
+blocks (the pivot floor, a full second factorisation), N(0,1) ones have not (a
+second Gram matrix near the identity, which is not factored).
 
 Tolerance: both runs stop at 1e-10 on their spectra; the energy's error is of
 that order, 1e-9 allowed.
