@@ -46,6 +46,7 @@ constexpr int kPreMin = 24;         // columns from which FP32 sweeps precede th
 constexpr int kPreSweeps = 20;
 constexpr int kEigSweeps = 30;      // cap of the corner's FP32 sweeps (their result is refined or replaced)
 constexpr float kPreCos = 1e-3f;    // a sweep that rotated no larger |cos| leaves ~1e-6: hand over
+constexpr int kQrCl = 16;           // CTAs of a QR's cluster, at most
 constexpr int kScaleExp = 40;  // the largest |entry| is scaled to 2^40: squared norms of
                                // columns down to ½ε of it stay inside the FP32 range
 
@@ -61,7 +62,7 @@ struct SvdProb {
   double *H, *H2;         // Householder vectors of the two factorisations, m×n and n×n
   double *hinv, *hinv2;   // 2/vᵀv of each
   int *perm, *perm2;      // perm[k]: column at pivot position k
-  double *cand;           // 2 × G × ldc candidate columns
+  double *cand;           // 2 × G × ldc candidate columns, each entry with its tag
   unsigned long long* key;  // 2 × G candidate keys, and G column maxima
   float *W32, *V32;       // FP32 copies of X and of the rotations; leading dimension ld32
   double *W, *Wbuf;       // X·V after the FP32 sweeps (W null: none)
@@ -85,6 +86,17 @@ __device__ __forceinline__ double wsum_d(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+// Both sums with the additions of one: the half-warps take one value each
+__device__ __forceinline__ void wsum2_d(double& a, double& b) {
+  const bool up = (threadIdx.x & 16) != 0;
+  const double give = up ? a : b;
+  double v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, give, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  a = __shfl_sync(0xffffffffu, v, 0);
+  b = __shfl_sync(0xffffffffu, v, 16);
 }
 
 __device__ __forceinline__ float wsum_f(float v) {
@@ -131,14 +143,54 @@ struct GridBar {
   }
 };
 
+// A value and its step's tag as one 16-byte access: whoever reads the tag has
+// the value, without a fence on either side
+__device__ __forceinline__ void st_tagged(void* p, double v, unsigned long long tag) {
+  asm volatile("{.reg .b128 t;\nmov.b128 t, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], t;}" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"(tag)
+               : "memory");
+}
+__device__ __forceinline__ double ld_tagged(const void* p, unsigned long long* tag) {
+  long long v;
+  asm volatile("{.reg .b128 t;\nld.relaxed.gpu.global.b128 t, [%2];\nmov.b128 {%0, %1}, t;}"
+               : "=l"(v), "=l"(*tag)
+               : "l"(p)
+               : "memory");
+  return __longlong_as_double(v);
+}
+
+// Bounded spin: false once 2 s have passed or another CTA gave up (*err)
+struct SpinLimit {
+  unsigned n = 0;
+  uint64_t t0 = 0;
+  __device__ bool more(int* err) {
+    if ((++n & 255u) != 0) return true;
+    if (t0 == 0) t0 = tc::gtime();
+    if (tc::gtime() - t0 > 2000000000ull || atomicAdd(err, 0) != 0) {
+      atomicExch(err, 1);
+      return false;
+    }
+    return true;
+  }
+};
+
 // ---------------------------------------------------------------------------
 // Householder QR with column pivoting.  One warp per column, the column in
 // registers (R chunks of 32 rows); CTA b holds the columns b, b + G, b + 2G...
-// Step k: every CTA has published its longest remaining column with its norm;
-// one barrier; every warp finds the longest of all (ties: smallest index),
-// reads that column from L2, forms its Householder vector (the same arithmetic
-// in every warp) and updates its own column.  One barrier and two dependent L2
-// reads a step; the norms that only choose pivots are FP32 sums of squares.
+// Step k: every CTA publishes its longest remaining column with a key (norm,
+// column); every warp finds the longest of all (ties: smallest index), reads that
+// column, forms its Householder vector (the same arithmetic in every warp) and
+// updates its own column.  The norms that only choose pivots are FP32 sums of
+// squares.  A step is a chain of latencies, so
+//   - across SMs keys and column entries carry the step's number and are polled
+//     where they lie: no counter barrier, no fence and no read of the keys after
+//     them; a CTA reads the column once, for all its warps (read by every warp, 456
+//     requests queue on each of its lines);
+//   - in a cluster the keys, and columns up to 128 rows, are stored into every
+//     CTA's shared memory before the barrier;
+//   - ‖x‖² and xᵀc are summed in one pass over registers and shuffles (vᵀc =
+//     xᵀc − β·c_k needs no v).
+// Two buffers by parity: a CTA is at most one step ahead of the slowest.
 // STAGE 0: A (m×n, scaled by a power of two) → H, hinv, perm, rank, X = Rᵀ in
 // pivot order.  STAGE 1: the r columns of X → H2, hinv2, perm2, X2 = R₂ᵀ.
 // ---------------------------------------------------------------------------
@@ -160,7 +212,10 @@ __global__ void __launch_bounds__(256) k_qrcp(SvdArgs a) {
   double* hinv = STAGE == 0 ? q.hinv : q.hinv2;
   int* perm = STAGE == 0 ? q.perm : q.perm2;
   double* X = STAGE == 0 ? q.X : q.X2;
-  __shared__ unsigned long long wkey[8];
+  constexpr bool kPush = CL && R <= 4;  // candidate columns go to every CTA's shared memory
+  __shared__ unsigned long long wkey[8], rkey[8], ckey[CL ? 2 : 1][CL ? kQrCl : 1];
+  __shared__ double xs[kPush ? 1 : 32 * R];  // the step's column
+  __shared__ double ccol[kPush ? 2 : 1][kPush ? kQrCl : 1][kPush ? 32 * R : 1];
   __shared__ unsigned picked_mask[kMaxSvdRows / 32];
   __shared__ int dead;
   if (threadIdx.x == 0) dead = 0;
@@ -231,63 +286,166 @@ __global__ void __launch_bounds__(256) k_qrcp(SvdArgs a) {
   const int kmax = min(m, n);
   int k = 0;
   for (; k < kmax; ++k) {
-    // this CTA's longest remaining column
+    // this CTA's longest remaining column: (norm, 1024 − column, step)
+    const int buf = k & 1;
+    const unsigned tag = (unsigned)(STAGE * 2048 + k + 1);
+    const bool live = have && pos < 0;
     const unsigned long long mykey =
-        (have && pos < 0) ? (((unsigned long long)__float_as_uint(nr) << 32) | (0xffffffffu - (unsigned)col)) : 0ull;
+        live ? (((unsigned long long)__float_as_uint(nr) << 32) | ((unsigned)(kMaxSvdRows - col) << 21) | tag) : tag;
     if (lane == 0) wkey[warp] = mykey;
     __syncthreads();
-    unsigned long long best = 0;
-    for (int w = 0; w < nwarp; ++w) best = wkey[w] > best ? wkey[w] : best;
-    double* mine = q.cand + ((int64_t)(k & 1) * G + cta) * a.ldc;
-    if (best != 0 && best == mykey) {
+    unsigned long long best = wkey[0];
+    int bw = 0;
+    for (int w = 1; w < nwarp; ++w)
+      if (wkey[w] > best) {
+        best = wkey[w];
+        bw = w;
+      }
+    double* mine = q.cand + 2 * ((int64_t)buf * G + cta) * a.ldc;
+    if (warp == bw) {
+      if (CL ? lane < G : lane == 0) {
+        if (CL) {
+          uint32_t ra;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                       : "=r"(ra)
+                       : "r"((uint32_t)__cvta_generic_to_shared(&ckey[buf][cta])), "r"(lane));
+          asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ra), "l"(best) : "memory");
+        } else {
+          asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&q.key[buf * G + cta]), "l"(best) : "memory");
+        }
+      }
+      if (kPush) {
+        const uint32_t la = (uint32_t)__cvta_generic_to_shared(&ccol[buf][cta][0]);
+        for (int g = 0; g < G; ++g) {
+          uint32_t ra;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(la), "r"(g));
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-        if (32 * i < m && 32 * i + 31 >= k && lane + 32 * i < m) __stcg(&mine[lane + 32 * i], c[i]);
+          for (int i = 0; i < R; ++i)
+            if (32 * i < m && 32 * i + 31 >= k)
+              asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra + 8u * (lane + 32 * i)), "d"(c[i]) : "memory");
+        }
+      } else if (live) {
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if (32 * i + 31 >= k && lane + 32 * i < m) st_tagged(&mine[2 * (lane + 32 * i)], c[i], tag);
+      }
     }
-    if (threadIdx.x == 0) __stcg(&q.key[(k & 1) * G + cta], best);
-    if (!bar.sync()) return;
-    best = 0;
-    for (int g = lane; g < G; g += 32) {
-      const unsigned long long b = __ldcg(&q.key[(k & 1) * G + g]);
-      best = b > best ? b : best;
+    if (CL) {
+      bar.sync();
+      best = lane < G ? ckey[buf][lane] : 0ull;
+    } else {
+      best = 0;
+      SpinLimit spin;
+      for (int g0 = threadIdx.x; g0 < G; g0 += 5 * (int)blockDim.x) {
+        while (true) {  // the loads of one pass do not wait for one another
+          unsigned long long b[5];
+#pragma unroll
+          for (int u = 0; u < 5; ++u) {
+            const int g = g0 + u * (int)blockDim.x;
+            b[u] = tag;
+            if (g < G) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(b[u]) : "l"(&q.key[buf * G + g]) : "memory");
+          }
+          bool all = true;
+#pragma unroll
+          for (int u = 0; u < 5; ++u) {
+            all = all && ((unsigned)b[u] & 0x1fffffu) == tag;
+            best = b[u] > best ? b[u] : best;
+          }
+          if (all) break;
+          best = 0;
+          if (!spin.more(q.info + kiErr)) {
+            dead = 1;
+            break;
+          }
+        }
+      }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long b = __shfl_xor_sync(0xffffffffu, best, o);
-      best = b > best ? b : best;
+    {  // the largest of the warp: its norm, then the column among equal norms
+      const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
+      const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32) == hi ? (unsigned)best : 0u);
+      best = ((unsigned long long)hi << 32) | lo;
+    }
+    if (!CL) {
+      if (lane == 0) rkey[warp] = best;
+      __syncthreads();
+      if (dead) return;
+      for (int w = 0; w < nwarp; ++w) best = rkey[w] > best ? rkey[w] : best;
     }
     const float n2 = __uint_as_float((unsigned)(best >> 32));
-    const int wj = (int)(0xffffffffu - (unsigned)best);
+    const int wj = kMaxSvdRows - (int)((unsigned)best >> 21);
     if (STAGE == 0) {
       if (k == 0) thr2 = a.trunc * a.trunc * n2;
       if (n2 <= thr2) break;  // the rest is below the rounding of A
     }
     if (threadIdx.x == 0) picked_mask[wj >> 5] |= 1u << (wj & 31);
-    const double* win = q.cand + ((int64_t)(k & 1) * G + (wj % G)) * a.ldc;
+    if (!kPush) {
+      const double* win = q.cand + 2 * ((int64_t)buf * G + (wj % G)) * a.ldc;
+      SpinLimit spin;
+      for (int row0 = (k & ~31) + threadIdx.x; row0 < m; row0 += 4 * blockDim.x) {
+        double v[4];
+        while (true) {  // four loads in flight
+          unsigned long long t[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int row = row0 + u * (int)blockDim.x;
+            t[u] = tag;
+            if (row < m) v[u] = ld_tagged(&win[2 * row], &t[u]);
+          }
+          if (t[0] == tag && t[1] == tag && t[2] == tag && t[3] == tag) break;
+          if (!spin.more(q.info + kiErr)) {
+            dead = 1;
+            break;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (row0 + u * (int)blockDim.x < m) xs[row0 + u * (int)blockDim.x] = v[u];
+      }
+      __syncthreads();
+      if (dead) return;
+    }
+    if (!live && !(cta == 0 && warp == 0)) continue;  // nothing left to update
+    const double* wsh = kPush ? &ccol[kPush ? buf : 0][kPush ? wj % G : 0][0] : xs;
     double x[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int row = lane + 32 * i;
-      x[i] = (32 * i + 31 >= k && row >= k && row < m) ? __ldcg(&win[row]) : 0.0;
+      x[i] = (32 * i + 31 >= k && row >= k && row < m) ? wsh[row] : 0.0;
     }
     // v = x − β·e_k, β = −sign(α)·‖x‖, H = I − hk·v·vᵀ with hk = 2/vᵀv = 1/(‖x‖² + |α|‖x‖)
-    double s2 = 0.0, al = 0.0;
+    double s2 = 0.0, d = 0.0, s2b = 0.0, db = 0.0, al = 0.0, ck = 0.0;
+#pragma unroll
+    for (int i = 0; i < R; i += 2) {
+      if (32 * i < m && 32 * i + 63 >= k) {  // (x is 0 outside the rows k..m)
+        s2 = fma(x[i], x[i], s2);
+        d = fma(x[i], c[i], d);
+        s2b = fma(x[i + 1], x[i + 1], s2b);
+        db = fma(x[i + 1], c[i + 1], db);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      if (32 * i < m && 32 * i + 31 >= k) s2 = fma(x[i], x[i], s2);
-      if (i == (k >> 5)) al = x[i];
+      if (lane + 32 * i == k) {  // (by i == k / 32 the arrays would be indexed in local memory)
+        al = x[i];
+        ck = c[i];
+      }
     }
-    s2 = wsum_d(s2);
+    s2 += s2b;
+    d += db;
+    wsum2_d(s2, d);
     al = __shfl_sync(0xffffffffu, al, k & 31);
+    ck = __shfl_sync(0xffffffffu, ck, k & 31);
     double beta = 0.0, hk = 0.0;
-    if (s2 > 1e-30) {
-      const double y = rsqrt_fast(s2);
-      double sg = s2 * y;
-      sg = fma(0.5 * y, fma(-sg, sg, s2), sg);
-      beta = al >= 0.0 ? -sg : sg;
-      hk = rcp_fast(fma(fabs(al), sg, s2));
+    if (__double2hiint(s2) > (923 << 20)) {  // ‖x‖² > 2^-100 (1e-30)
+      // ‖x‖ and hk by one cubic step each from FP32 values (error ~ (2e-7)³)
+      const double y = f2d(rsqrtf(d2f(s2))), g0 = s2 * y, e = fma(-g0, y, 1.0);
+      const double sg = fma(g0 * e, fma(0.375, e, 0.5), g0);
+      beta = __double2hiint(al) >= 0 ? -sg : sg;
+      const double den = fma(fabs(al), sg, s2), h0 = f2d(__fdividef(1.f, d2f(den))), f = fma(-den, h0, 1.0);
+      hk = fma(h0, fma(f, f, f), h0);
 #pragma unroll
       for (int i = 0; i < R; ++i)
-        if (i == (k >> 5) && lane == (k & 31)) x[i] = al - beta;
+        if (lane + 32 * i == k) x[i] = al - beta;
     } else {
 #pragma unroll
       for (int i = 0; i < R; ++i) x[i] = 0.0;
@@ -310,19 +468,19 @@ __global__ void __launch_bounds__(256) k_qrcp(SvdArgs a) {
           c[i] = row < k ? c[i] : (row == k ? beta : 0.0);
         }
       } else {
-        double d = 0.0;
-#pragma unroll
-        for (int i = 0; i < R; ++i)
-          if (32 * i < m && 32 * i + 31 >= k) d = fma(x[i], c[i], d);
-        d = wsum_d(d) * hk;
+        d = fma(-beta, ck, d) * hk;
         nr = 0.f;
+        float nr1 = 0.f;
 #pragma unroll
-        for (int i = 0; i < R; ++i)
-          if (32 * i < m && 32 * i + 31 >= k) {
+        for (int i = 0; i < R; i += 2)
+          if (32 * i < m && 32 * i + 63 >= k) {
             c[i] = fma(-d, x[i], c[i]);
-            const float f = lane + 32 * i > k ? d2f(c[i]) : 0.f;
+            c[i + 1] = fma(-d, x[i + 1], c[i + 1]);
+            const float f = lane + 32 * i > k ? d2f(c[i]) : 0.f, f1 = lane + 32 * i + 32 > k ? d2f(c[i + 1]) : 0.f;
             nr = fmaf(f, f, nr);
+            nr1 = fmaf(f1, f1, nr1);
           }
+        nr += nr1;
         nr = wsum_f(nr);
       }
     }
@@ -487,29 +645,29 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
           P = Q;
           Q = t;
         }
-        const int gc[4] = {2 * P, 2 * P + 1, 2 * Q, 2 * Q + 1};
+        auto gc = [&](int l) { return l < 2 ? 2 * P + l : 2 * Q + l - 2; };  // (an array would be local memory)
         // 4 columns of W and V to shared memory
         for (int l = 0; l < 4; ++l) {
-          if (gc[l] >= rc) continue;
-          const double* ws = W + (int64_t)gc[l] * ldx;
+          if (gc(l) >= rc) continue;
+          const double* ws = W + (int64_t)gc(l) * ldx;
           const uint32_t dst = tc::su32(sm + (int64_t)l * cst);
           for (int i = threadIdx.x; i < (ldw >> 1); i += blockDim.x)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(ws + 2 * i) : "memory");
           if (ACCV) {
-            const double* vs = V + (int64_t)gc[l] * ldx;
+            const double* vs = V + (int64_t)gc(l) * ldx;
             for (int i = threadIdx.x; i < (ldv >> 1); i += blockDim.x)
               asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 8u * ldw + 16u * i), "l"(vs + 2 * i)
                            : "memory");
           }
         }
-        if (r > 0 && threadIdx.x < 4 && gc[threadIdx.x] < rc) nrm4[threadIdx.x] = __ldcg(&q.nrm[gc[threadIdx.x]]);
+        if (r > 0 && threadIdx.x < 4 && gc(threadIdx.x) < rc) nrm4[threadIdx.x] = __ldcg(&q.nrm[gc(threadIdx.x)]);
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         const int rot0 = nrot;
         if (r == 0) {  // norms anew: warp w takes column w
           const int w = threadIdx.x >> 5;
           double s = 0.0;
-          if (gc[w] < rc) {
+          if (gc(w) < rc) {
             const double* wc = sm + (int64_t)w * cst;
 #pragma unroll 4
             for (int i = lane; i < mx; i += 32) s = fma(wc[i], wc[i], s);
@@ -517,25 +675,25 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
             if (lane == 0) nrm4[w] = s;
           }
           __syncthreads();
-          process(2 * grp, 2 * grp + 1, gc[2 * grp + 1] < rc);
+          process(2 * grp, 2 * grp + 1, gc(2 * grp + 1) < rc);
           __syncthreads();
         }
-        process(grp, 2 + grp, gc[grp] < rc && gc[2 + grp] < rc);
+        process(grp, 2 + grp, gc(grp) < rc && gc(2 + grp) < rc);
         __syncthreads();
-        process(grp, 3 - grp, gc[grp] < rc && gc[3 - grp] < rc);
+        process(grp, 3 - grp, gc(grp) < rc && gc(3 - grp) < rc);
         __syncthreads();
         if (nrot != rot0 || r == 0) {
           for (int l = 0; l < 4; ++l) {
-            if (gc[l] >= rc) continue;
-            double2* wd = reinterpret_cast<double2*>(W + (int64_t)gc[l] * ldx);
+            if (gc(l) >= rc) continue;
+            double2* wd = reinterpret_cast<double2*>(W + (int64_t)gc(l) * ldx);
             const double2* s2 = reinterpret_cast<const double2*>(sm + (int64_t)l * cst);
             for (int i = threadIdx.x; i < (ldw >> 1); i += blockDim.x) __stcg(&wd[i], s2[i]);
             if (ACCV) {
-              double2* vd = reinterpret_cast<double2*>(V + (int64_t)gc[l] * ldx);
+              double2* vd = reinterpret_cast<double2*>(V + (int64_t)gc(l) * ldx);
               for (int i = threadIdx.x; i < (ldv >> 1); i += blockDim.x) __stcg(&vd[i], s2[(ldw >> 1) + i]);
             }
           }
-          if (threadIdx.x < 4 && gc[threadIdx.x] < rc) __stcg(&q.nrm[gc[threadIdx.x]], nrm4[threadIdx.x]);
+          if (threadIdx.x < 4 && gc(threadIdx.x) < rc) __stcg(&q.nrm[gc(threadIdx.x)], nrm4[threadIdx.x]);
         }
       }
       if (r == rounds - 1) {
@@ -1040,6 +1198,7 @@ void launch_grid(tnad_ctx* c, F* f, bool cluster, int G, int np, int threads, si
   cf.dynamicSmemBytes = smem;
   cf.stream = c->stream;
   cudaLaunchAttribute at[1];
+  if (cluster && G > 8) TNAD_CK(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   if (cluster) {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)G;
@@ -1057,10 +1216,12 @@ void launch_grid(tnad_ctx* c, F* f, bool cluster, int G, int np, int threads, si
 
 template <int R, int STAGE>
 void launch_qrcp(tnad_ctx* c, int np, int cols, SvdArgs& a) {
-  // up to 64 columns fit a cluster of 8 CTAs of 8 warps; beyond, as many CTAs
-  // as SMs (both problems together resident)
+  // up to 64 columns in a cluster, 4 warps a CTA (one an SM quadrant): n = 121 took
+  // 8000 clocks a step in 16 CTAs of 8 warps, whose FP64 instructions share the
+  // quadrants, 7200 with a CTA a column; beyond, as many CTAs as SMs (both
+  // problems together resident)
   if (cols <= 64) {
-    const int G = std::min(8, cols);
+    const int G = std::min(kQrCl, (cols + 3) / 4);
     launch_grid(c, k_qrcp<R, true, STAGE>, true, G, np, 32 * ((cols + G - 1) / G), 0, a);
   } else {
     const int G = std::min(cols, c->sm_count / np);
@@ -1072,7 +1233,7 @@ template <int RJ, bool ACCV>
 void launch_sweeps(tnad_ctx* c, int np, SvdArgs& a) {
   const int nreal = (a.n + 1) / 2, G = std::max(1, (nreal + (nreal & 1)) / 2);
   const size_t smem = (size_t)4 * ((a.n + 1) & ~1) * (ACCV ? 2 : 1) * sizeof(double);
-  if (G <= 8) {
+  if (G <= 16) {
     launch_grid(c, k_svd_sweeps<RJ, ACCV, true>, true, G, np, 128, smem, a);
   } else {
     static std::atomic<bool> attr{false};
@@ -1231,7 +1392,13 @@ void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, 
     c->fault_once = kFaultNone;
   }
   const int64_t G = c->sm_count;
-  int* info = (int*)c->ws.alloc(sizeof(int) * 2 * kiCount);
+  // candidates, keys and counters start at zero (what an earlier call left could carry this one's tags)
+  const int64_t cand = 2 * 2 * G * a.ldc;  // doubles of one problem
+  const size_t nzero = (size_t)np * cand * sizeof(double) +
+                       2 * (3 * G * sizeof(unsigned long long) + kiCount * sizeof(int));
+  double* cands = (double*)c->ws.alloc(nzero);
+  unsigned long long* zero = (unsigned long long*)(cands + np * cand);
+  int* info = (int*)(zero + 2 * 3 * G);
   for (int p = 0; p < np; ++p) {
     SvdProb& q = a.p[p];
     q.A = A[p];
@@ -1248,8 +1415,8 @@ void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, 
     q.hinv2 = q.hinv + n;
     q.perm = (int*)c->ws.alloc(sizeof(int) * 2 * n);
     q.perm2 = q.perm + n;
-    q.cand = ws_d(c, 2 * G * a.ldc);
-    q.key = (unsigned long long*)ws_d(c, 3 * G);
+    q.cand = cands + p * cand;
+    q.key = zero + p * 3 * G;
     q.nrm = ws_d(c, n);
     q.sv = ws_d(c, n);
     q.U = U[p];
@@ -1257,7 +1424,7 @@ void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, 
     q.V = V[p];
     q.info = info + p * kiCount;
   }
-  TNAD_CK(cudaMemsetAsync(info, 0, sizeof(int) * 2 * kiCount, c->stream));
+  TNAD_CK(cudaMemsetAsync(cands, 0, nzero, c->stream));
   const double nn = (double)n;
   int h[2 * kiBar];
   {
