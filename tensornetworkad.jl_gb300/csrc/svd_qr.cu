@@ -537,11 +537,12 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
   double* W = q.W ? q.W : (two ? q.X2 : q.X);
   double* V = q.Vx;
   const int ldx = a.ldx;
-  const int ldw = (mx + 1) & ~1, ldv = ACCV ? (rc + 1) & ~1 : 0, cst = ldw + ldv;
+  constexpr int ldw = 64 * RJ, cst = (ACCV ? 2 : 1) * ldw;
   double* sm = reinterpret_cast<double*>(sm_raw);  // 4 columns of cst doubles: W rows, then V rows
   __shared__ double nrm4[4], red[2][2];
   __shared__ int dead, nrot, cosmax, tanmax;
   if (threadIdx.x == 0) dead = nrot = cosmax = tanmax = 0;
+  for (int i = threadIdx.x; i < 4 * cst; i += blockDim.x) sm[i] = 0.0;  // rows beyond mx stay 0 and need no guard
   __syncthreads();
   GridBar<CL> bar{reinterpret_cast<unsigned*>(q.info + kiBar + 2), 0u, (unsigned)max(active, 1), q.info + kiErr,
                   &dead};
@@ -563,13 +564,16 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
     if (present) {
 #pragma unroll
       for (int e = 0; e < RJ; ++e) {
-        const int i = lt + 64 * e;
-        u[e] = i < mx ? wx[i] : 0.0;
-        v[e] = i < mx ? wy[i] : 0.0;
+        u[e] = wx[lt + 64 * e];
+        v[e] = wy[lt + 64 * e];
       }
+      double g1 = 0.0;
 #pragma unroll
-      for (int e = 0; e < RJ; ++e)
-        if (64 * e < mx) g = fma(u[e], v[e], g);
+      for (int e = 0; e < RJ; ++e) {
+        if (e & 1) g1 = fma(u[e], v[e], g1);
+        else g = fma(u[e], v[e], g);
+      }
+      if (RJ > 1) g += g1;
       g = wsum_d(g);
       if (lane == 0) red[grp][wip] = g;
     }
@@ -590,27 +594,22 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
 #pragma unroll
         for (int e = 0; e < RJ; ++e) {
           const int i = lt + 64 * e;
-          if (i < mx) {
-            wx[i] = cs * u[e] - sn * v[e];
-            wy[i] = sn * u[e] + cs * v[e];
-          }
+          wx[i] = cs * u[e] - sn * v[e];
+          wy[i] = sn * u[e] + cs * v[e];
         }
         if (ACCV) {
           double* vx = wx + ldw;
           double* vy = wy + ldw;
 #pragma unroll
           for (int e = 0; e < RJ; ++e) {
-            const int i = lt + 64 * e;
-            u[e] = i < rc ? vx[i] : 0.0;
-            v[e] = i < rc ? vy[i] : 0.0;
+            u[e] = vx[lt + 64 * e];
+            v[e] = vy[lt + 64 * e];
           }
 #pragma unroll
           for (int e = 0; e < RJ; ++e) {
             const int i = lt + 64 * e;
-            if (i < rc) {
-              vx[i] = cs * u[e] - sn * v[e];
-              vy[i] = sn * u[e] + cs * v[e];
-            }
+            vx[i] = cs * u[e] - sn * v[e];
+            vy[i] = sn * u[e] + cs * v[e];
           }
         }
         asm volatile("bar.sync %0, 64;" ::"r"(grp + 1) : "memory");  // norms read by all of the group
@@ -651,11 +650,13 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
           if (gc(l) >= rc) continue;
           const double* ws = W + (int64_t)gc(l) * ldx;
           const uint32_t dst = tc::su32(sm + (int64_t)l * cst);
-          for (int i = threadIdx.x; i < (ldw >> 1); i += blockDim.x)
+          for (int i = threadIdx.x; i < (mx >> 1); i += blockDim.x)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(ws + 2 * i) : "memory");
+          if ((mx & 1) && threadIdx.x == blockDim.x - 1) sm[(int64_t)l * cst + mx - 1] = __ldcg(&ws[mx - 1]);
           if (ACCV) {
             const double* vs = V + (int64_t)gc(l) * ldx;
-            for (int i = threadIdx.x; i < (ldv >> 1); i += blockDim.x)
+            if ((rc & 1) && threadIdx.x == blockDim.x - 2) sm[(int64_t)l * cst + ldw + rc - 1] = __ldcg(&vs[rc - 1]);
+            for (int i = threadIdx.x; i < (rc >> 1); i += blockDim.x)
               asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 8u * ldw + 16u * i), "l"(vs + 2 * i)
                            : "memory");
           }
@@ -685,12 +686,12 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
         if (nrot != rot0 || r == 0) {
           for (int l = 0; l < 4; ++l) {
             if (gc(l) >= rc) continue;
-            double2* wd = reinterpret_cast<double2*>(W + (int64_t)gc(l) * ldx);
+            double2* wd = reinterpret_cast<double2*>(W + (int64_t)gc(l) * ldx);  // (ldx is even: room for the pair)
             const double2* s2 = reinterpret_cast<const double2*>(sm + (int64_t)l * cst);
-            for (int i = threadIdx.x; i < (ldw >> 1); i += blockDim.x) __stcg(&wd[i], s2[i]);
+            for (int i = threadIdx.x; i < ((mx + 1) >> 1); i += blockDim.x) __stcg(&wd[i], s2[i]);
             if (ACCV) {
               double2* vd = reinterpret_cast<double2*>(V + (int64_t)gc(l) * ldx);
-              for (int i = threadIdx.x; i < (ldv >> 1); i += blockDim.x) __stcg(&vd[i], s2[(ldw >> 1) + i]);
+              for (int i = threadIdx.x; i < ((rc + 1) >> 1); i += blockDim.x) __stcg(&vd[i], s2[(ldw >> 1) + i]);
             }
           }
           if (threadIdx.x < 4 && gc(threadIdx.x) < rc) __stcg(&q.nrm[gc(threadIdx.x)], nrm4[threadIdx.x]);
@@ -1216,33 +1217,58 @@ void launch_grid(tnad_ctx* c, F* f, bool cluster, int G, int np, int threads, si
 
 template <int R, int STAGE>
 void launch_qrcp(tnad_ctx* c, int np, int cols, SvdArgs& a) {
-  // up to 64 columns in a cluster, 4 warps a CTA (one an SM quadrant): n = 121 took
-  // 8000 clocks a step in 16 CTAs of 8 warps, whose FP64 instructions share the
-  // quadrants, 7200 with a CTA a column; beyond, as many CTAs as SMs (both
-  // problems together resident)
+  // Up to 64 columns in a cluster, 4 warps a CTA (one an SM quadrant).  Beyond, CTAs
+  // over the whole GPU: a column each up to 128 (n = 121: 6200 clocks a step, 6800 in
+  // CTAs of 4 warps, 8000 in a cluster of 16 CTAs of 8, whose FP64 instructions
+  // share the quadrants), then 4 warps a CTA, or more where the SMs run out: fewer
+  // CTAs read the step's keys and column (n = 324: 10300 clocks, 12600 with 152 CTAs).
   if (cols <= 64) {
     const int G = std::min(kQrCl, (cols + 3) / 4);
     launch_grid(c, k_qrcp<R, true, STAGE>, true, G, np, 32 * ((cols + G - 1) / G), 0, a);
   } else {
-    const int G = std::min(cols, c->sm_count / np);
+    const int G = std::min(cols <= 128 ? cols : (cols + 3) / 4, c->sm_count / np);
     launch_grid(c, k_qrcp<R, false, STAGE>, false, G, np, 32 * ((cols + G - 1) / G), 0, a);
   }
 }
 
 template <int RJ, bool ACCV>
-void launch_sweeps(tnad_ctx* c, int np, SvdArgs& a) {
+void launch_sweeps_rj(tnad_ctx* c, int np, SvdArgs& a) {
   const int nreal = (a.n + 1) / 2, G = std::max(1, (nreal + (nreal & 1)) / 2);
-  const size_t smem = (size_t)4 * ((a.n + 1) & ~1) * (ACCV ? 2 : 1) * sizeof(double);
-  if (G <= 16) {
-    launch_grid(c, k_svd_sweeps<RJ, ACCV, true>, true, G, np, 128, smem, a);
-  } else {
-    static std::atomic<bool> attr{false};
-    if (!attr) {
-      TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps<RJ, ACCV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   4 * kMaxSvdRows * 2 * 8));
-      attr = true;
+  const size_t smem = (size_t)4 * 64 * RJ * (ACCV ? 2 : 1) * sizeof(double);
+  if constexpr (RJ == 1) {
+    if (G <= 16) {
+      launch_grid(c, k_svd_sweeps<RJ, ACCV, true>, true, G, np, 128, smem, a);
+      return;
     }
-    launch_grid(c, k_svd_sweeps<RJ, ACCV, false>, false, G, np, 128, smem, a);
+  }
+  static std::atomic<bool> attr{false};
+  if (!attr) {
+    TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps<RJ, ACCV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 4 * kMaxSvdRows * 2 * 8));
+    attr = true;
+  }
+  launch_grid(c, k_svd_sweeps<RJ, ACCV, false>, false, G, np, 128, smem, a);
+}
+
+// By the rows that there are, in steps of 64 (of 128 beyond 512): a guard on each
+// of a thread's rows cost a third of the rotation at n = 324
+template <bool ACCV>
+void launch_sweeps(tnad_ctx* c, int np, int rows, SvdArgs& a) {
+  switch ((rows + 63) / 64) {
+    case 0:
+    case 1: return launch_sweeps_rj<1, ACCV>(c, np, a);
+    case 2: return launch_sweeps_rj<2, ACCV>(c, np, a);
+    case 3: return launch_sweeps_rj<3, ACCV>(c, np, a);
+    case 4: return launch_sweeps_rj<4, ACCV>(c, np, a);
+    case 5: return launch_sweeps_rj<5, ACCV>(c, np, a);
+    case 6: return launch_sweeps_rj<6, ACCV>(c, np, a);
+    case 7: return launch_sweeps_rj<7, ACCV>(c, np, a);
+    case 8: return launch_sweeps_rj<8, ACCV>(c, np, a);
+    case 9:
+    case 10: return launch_sweeps_rj<10, ACCV>(c, np, a);
+    case 11:
+    case 12: return launch_sweeps_rj<12, ACCV>(c, np, a);
+    default: return launch_sweeps_rj<16, ACCV>(c, np, a);
   }
 }
 
@@ -1314,10 +1340,15 @@ void svd_qrj_r(tnad_ctx* c, int np, bool symmetric, SvdArgs& a, int* info_host) 
   launch_qrcp<R, 0>(c, np, a.n, a);
   launch_qrcp<R, 1>(c, np, a.n, a);
   if (a.n >= kPreMin) pre_sweeps(c, np, a, info_host);
+  int rows = 0;  // of the triangular factors
+  for (int p = 0; p < np; ++p) {
+    const int r = a.n >= kPreMin ? info_host[p * kiBar + kiRank] : a.n;
+    rows = std::max(rows, a.second || r < a.n ? r : a.n);
+  }
   if (symmetric)
-    launch_sweeps<R / 2, false>(c, np, a);
+    launch_sweeps<false>(c, np, rows, a);
   else
-    launch_sweeps<R / 2, true>(c, np, a);
+    launch_sweeps<true>(c, np, rows, a);
   const dim3 gw((unsigned)((a.n + 3) / 4), (unsigned)np), gc((unsigned)a.n, (unsigned)np);
   k_svd_norms<<<gw, 128, 0, c->stream>>>(a);
   if (symmetric) {
