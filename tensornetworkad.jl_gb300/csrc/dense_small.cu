@@ -392,11 +392,15 @@ __global__ void k_eigh_jacobi(const double* __restrict__ A, int p, int max_sweep
 
 // The FP32 solve, one-sided: W = A·V and V in shared memory, the rotation of a
 // pair from the 2×2 block of VᵀAV (a = v_p·w_p, b = v_q·w_q, g = (v_p·w_q +
-// v_q·w_p)/2), so that ±λ pairs stay apart.  8 lanes per pair, their rows as
-// 16-byte shared loads and packed FP32 pairs (fma.rn.f32x2): all ⌈p/2⌉ pairs of
-// a round in ⌈p/8⌉ warps at once and one barrier a round, where the two-sided
-// form (k_eigh_jacobi) takes three and two passes over H.  Latency bound (one
-// CTA): p = 96 in 455 µs, two-sided 758.  Same stop rule.
+// v_q·w_p)/2), so that ±λ pairs stay apart.  Columns in blocks of two, a block pair
+// per 8 lanes and round of the circle method: its 4 columns come to registers by
+// 16-byte shared loads, the cross pairs are rotated in two steps of two disjoint
+// ones (in a sweep's first round the pairs inside the blocks before them) in packed
+// FP32 (fma.rn.f32x2), and go back; one barrier a round.  With single columns W and
+// V passed through shared memory once a rotation (128 bytes a clock: 1150 of a
+// round's 1650 clocks at p = 96) and a sweep took p − 1 rounds (454 µs in the mean of a solve at p = 96, now 280);
+// the two-sided form (k_eigh_jacobi), with three barriers and two passes, 758.
+// Same stop rule.
 __device__ __forceinline__ uint64_t pk2(float a, float b) {
   return ((uint64_t)__float_as_uint(b) << 32) | __float_as_uint(a);
 }
@@ -417,24 +421,24 @@ __device__ __forceinline__ float hsum2(uint64_t a) {
 constexpr int kEigh32MaxP = 160;  // W and V of FP32 in one CTA's shared memory
 
 template <int RV>  // 16-byte row chunks per lane: ⌈p/32⌉
-__global__ void __launch_bounds__(640) k_eigh32(const double* __restrict__ A, int p, int max_sweeps,
+__global__ void __launch_bounds__(64 * RV, 1) k_eigh32(const double* __restrict__ A, int p, int max_sweeps,
                                                 double* __restrict__ lam, double* __restrict__ Wout,
                                                 int* __restrict__ info, int by_value) {
   extern __shared__ __align__(16) float esm[];
   const int pr = (p + 3) & ~3, cs = 2 * pr, q4 = pr >> 2;  // column: W rows, then V rows
-  __shared__ float fro_part[20];
+  __shared__ float fro_part[10];
   __shared__ int rotated;
   __shared__ float lam_sh[kEigh32MaxP];
-  const int NP = p + (p & 1), nb = NP >> 1;
+  const int nreal = (p + 1) >> 1, NB = nreal + (nreal & 1);  // blocks; columns from p on are zero
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l8 = lane & 7;
   float ss = 0.f;
-  for (int e = threadIdx.x; e < p * cs; e += blockDim.x) {
+  for (int e = threadIdx.x; e < 2 * NB * cs; e += blockDim.x) {
     const int i = e % cs, j = e / cs;
-    float v;
+    float v = 0.f;
     if (i < pr) {
-      v = i < p ? (float)A[i + (int64_t)j * p] : 0.f;
+      v = i < p && j < p ? d2f_rn(A[i + (int64_t)j * p]) : 0.f;
       ss = fmaf(v, v, ss);
-    } else {
+    } else if (j < p) {
       v = i - pr == j ? 1.f : 0.f;
     }
     esm[e] = v;
@@ -446,68 +450,115 @@ __global__ void __launch_bounds__(640) k_eigh32(const double* __restrict__ A, in
   for (int w = 0; w < (int)(blockDim.x >> 5); ++w) fro2 += fro_part[w];
   const float tol = 4.f * FLT_EPSILON * sqrtf((float)p);
   const float absfl = 2.f * FLT_EPSILON * sqrtf((float)p) * sqrtf(fro2);
-  const int k = warp * 4 + (lane >> 3);  // this lane group's pair
+  const int k = threadIdx.x >> 3;  // this lane group's block pair
+  const bool on = k < (NB >> 1);
+  ulonglong2 w[4][RV], v[4][RV];
+  float f[4];  // v_i·w_i
+
+  // rotate the pairs (i0, j0) and (i1, j1) of the four columns; true when one did
+  auto step = [&](const int i0, const int j0, const int i1, const int j1) -> bool {
+    uint64_t s0 = 0, s1 = 0;
+#pragma unroll
+    for (int e = 0; e < RV; ++e) {
+      s0 = fma2(v[i0][e].x, w[j0][e].x, s0);
+      s1 = fma2(v[i1][e].x, w[j1][e].x, s1);
+      s0 = fma2(v[j0][e].x, w[i0][e].x, s0);
+      s1 = fma2(v[j1][e].x, w[i1][e].x, s1);
+      s0 = fma2(v[i0][e].y, w[j0][e].y, s0);
+      s1 = fma2(v[i1][e].y, w[j1][e].y, s1);
+      s0 = fma2(v[j0][e].y, w[i0][e].y, s0);
+      s1 = fma2(v[j1][e].y, w[i1][e].y, s1);
+    }
+    float g[2] = {hsum2(s0), hsum2(s1)};  // 2g
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      g[0] += __shfl_xor_sync(0xffffffffu, g[0], o);
+      g[1] += __shfl_xor_sync(0xffffffffu, g[1], o);
+    }
+    bool any = false;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = h ? i1 : i0, j = h ? j1 : j0;
+      const float ag = 0.5f * fabsf(g[h]);
+      if (ag > tol * fsqrt_ap(fabsf(f[i])) * fsqrt_ap(fabsf(f[j])) && ag > absfl) {
+        const float t = jacobi_tan(f[j] - f[i], g[h]), tg = 0.5f * t * g[h];
+        const float c = rsqrtf(fmaf(t, t, 1.f)), sn = c * t;
+        const uint64_t c2 = pk2(c, c), s2 = pk2(sn, sn), n2 = pk2(-sn, -sn);
+        f[i] -= tg;
+        f[j] += tg;
+#pragma unroll
+        for (int e = 0; e < RV; ++e) {
+          const ulonglong2 wi = w[i][e], wj = w[j][e], vi = v[i][e], vj = v[j][e];
+          w[i][e] = make_ulonglong2(fma2(c2, wi.x, mul2(n2, wj.x)), fma2(c2, wi.y, mul2(n2, wj.y)));
+          w[j][e] = make_ulonglong2(fma2(c2, wj.x, mul2(s2, wi.x)), fma2(c2, wj.y, mul2(s2, wi.y)));
+          v[i][e] = make_ulonglong2(fma2(c2, vi.x, mul2(n2, vj.x)), fma2(c2, vi.y, mul2(n2, vj.y)));
+          v[j][e] = make_ulonglong2(fma2(c2, vj.x, mul2(s2, vi.x)), fma2(c2, vj.y, mul2(s2, vi.y)));
+        }
+        any = true;
+      }
+    }
+    return any;
+  };
+
   int sweep = 0;
   for (; sweep < max_sweeps; ++sweep) {
     if (threadIdx.x == 0) rotated = 0;
     __syncthreads();
-    for (int r = 0; r < NP - 1; ++r) {
-      int a = 0, b = 0;
-      bool on = k < nb;
-      if (on) {
-        circle_pair(r, k, NP, &a, &b);
-        on = a < p && b < p;
-        if (a > b) {
-          const int t = a;
-          a = b;
-          b = t;
-        }
+    for (int r = 0; r < NB - 1; ++r) {
+      int P = r, Q = NB - 1;
+      if (k > 0) {
+        P = r + k < NB - 1 ? r + k : r + k - (NB - 1);
+        Q = r >= k ? r - k : r - k + NB - 1;
       }
-      ulonglong2* xa = reinterpret_cast<ulonglong2*>(esm + a * cs);
-      ulonglong2* xb = reinterpret_cast<ulonglong2*>(esm + b * cs);
-      ulonglong2 wx[RV], wy[RV], vx[RV], vy[RV];
-      uint64_t sa = 0, sb = 0, sg = 0;
+      if (P > Q) {
+        const int t = P;
+        P = Q;
+        Q = t;
+      }
+      ulonglong2* cp = reinterpret_cast<ulonglong2*>(esm + (on ? 2 * P : 0) * cs);
+      ulonglong2* cq = reinterpret_cast<ulonglong2*>(esm + (on ? 2 * Q : 0) * cs);
+      const int c4 = cs >> 2;
+      const ulonglong2 z = make_ulonglong2(0, 0);
+      uint64_t sd[4] = {0, 0, 0, 0};
 #pragma unroll
-      for (int e = 0; e < RV; ++e) {
-        const int i = l8 + 8 * e;
-        const bool in = on && i < q4;
-        const ulonglong2 z = make_ulonglong2(0, 0);
-        wx[e] = in ? xa[i] : z;
-        wy[e] = in ? xb[i] : z;
-        vx[e] = in ? xa[q4 + i] : z;
-        vy[e] = in ? xb[q4 + i] : z;
-      }
-#pragma unroll
-      for (int e = 0; e < RV; ++e) {
-        sa = fma2(vx[e].x, wx[e].x, sa);
-        sb = fma2(vy[e].x, wy[e].x, sb);
-        sg = fma2(vx[e].x, wy[e].x, sg);
-        sg = fma2(vy[e].x, wx[e].x, sg);
-        sa = fma2(vx[e].y, wx[e].y, sa);
-        sb = fma2(vy[e].y, wy[e].y, sb);
-        sg = fma2(vx[e].y, wy[e].y, sg);
-        sg = fma2(vy[e].y, wx[e].y, sg);
-      }
-      float fa = hsum2(sa), fb = hsum2(sb), g2 = hsum2(sg);  // g2 = 2g
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) {
-        fa += __shfl_xor_sync(0xffffffffu, fa, o);
-        fb += __shfl_xor_sync(0xffffffffu, fb, o);
-        g2 += __shfl_xor_sync(0xffffffffu, g2, o);
-      }
-      const float ag = 0.5f * fabsf(g2);
-      if (on && ag > tol * fsqrt_ap(fabsf(fa)) * fsqrt_ap(fabsf(fb)) && ag > absfl) {
-        const float t = jacobi_tan(fb - fa, g2);
-        const float c = rsqrtf(fmaf(t, t, 1.f)), sn = c * t;
-        const uint64_t c2 = pk2(c, c), s2 = pk2(sn, sn), n2 = pk2(-sn, -sn);
+      for (int l = 0; l < 4; ++l) {
+        const ulonglong2* x = (l < 2 ? cp : cq) + (l & 1) * c4;
 #pragma unroll
         for (int e = 0; e < RV; ++e) {
           const int i = l8 + 8 * e;
-          if (i < q4) {
-            xa[i] = make_ulonglong2(fma2(c2, wx[e].x, mul2(n2, wy[e].x)), fma2(c2, wx[e].y, mul2(n2, wy[e].y)));
-            xb[i] = make_ulonglong2(fma2(c2, wy[e].x, mul2(s2, wx[e].x)), fma2(c2, wy[e].y, mul2(s2, wx[e].y)));
-            xa[q4 + i] = make_ulonglong2(fma2(c2, vx[e].x, mul2(n2, vy[e].x)), fma2(c2, vx[e].y, mul2(n2, vy[e].y)));
-            xb[q4 + i] = make_ulonglong2(fma2(c2, vy[e].x, mul2(s2, vx[e].x)), fma2(c2, vy[e].y, mul2(s2, vx[e].y)));
+          const bool in = on && i < q4;
+          w[l][e] = in ? x[i] : z;
+          v[l][e] = in ? x[q4 + i] : z;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < RV; ++e)
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          sd[l] = fma2(v[l][e].x, w[l][e].x, sd[l]);
+          sd[l] = fma2(v[l][e].y, w[l][e].y, sd[l]);
+        }
+#pragma unroll
+      for (int l = 0; l < 4; ++l) f[l] = hsum2(sd[l]);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int l = 0; l < 4; ++l) f[l] += __shfl_xor_sync(0xffffffffu, f[l], o);
+      bool any = false;
+      if (r == 0) any = step(0, 1, 2, 3);
+      any |= step(0, 2, 1, 3);
+      any |= step(0, 3, 1, 2);
+      if (any) {
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          ulonglong2* x = (l < 2 ? cp : cq) + (l & 1) * c4;
+#pragma unroll
+          for (int e = 0; e < RV; ++e) {
+            const int i = l8 + 8 * e;
+            if (i < q4) {
+              x[i] = w[l][e];
+              x[q4 + i] = v[l][e];
+            }
           }
         }
         if (l8 == 0) rotated = 1;
@@ -536,7 +587,7 @@ __global__ void __launch_bounds__(640) k_eigh32(const double* __restrict__ A, in
     }
     for (int o = 16; o > 0; o >>= 1) rk += __shfl_xor_sync(0xffffffffu, rk, o);
     if (lane == 0) lam[rk] = (double)lj;
-    for (int i = lane; i < p; i += 32) Wout[i + (int64_t)rk * p] = (double)esm[j * cs + pr + i];
+    for (int i = lane; i < p; i += 32) Wout[i + (int64_t)rk * p] = f2d_any(esm[j * cs + pr + i]);
   }
   if (threadIdx.x == 0 && info) info[0] = sweep;
 }
@@ -549,9 +600,9 @@ void eigh32_launch(tnad_ctx* c, const double* A, int p, int max_sweeps, double* 
                                  2 * kEigh32MaxP * kEigh32MaxP * 4));
     attr = true;
   }
-  const int pr = (p + 3) & ~3, nb = (p + 1) / 2;
-  k_eigh32<RV><<<1, 32 * ((nb + 3) / 4), (size_t)p * 2 * pr * sizeof(float), c->stream>>>(A, p, max_sweeps, lam, W,
-                                                                                          info, by_value);
+  const int pr = (p + 3) & ~3, nreal = (p + 1) / 2, NB = nreal + (nreal & 1);
+  k_eigh32<RV><<<1, (4 * NB + 31) / 32 * 32, (size_t)2 * NB * 2 * pr * sizeof(float), c->stream>>>(
+      A, p, max_sweeps, lam, W, info, by_value);
 }
 
 void eigh_small_prec(tnad_ctx* c, bool fp32, const double* A, int64_t p, double* W, double* lam, int max_sweeps,
