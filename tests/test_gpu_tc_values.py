@@ -74,6 +74,23 @@ def test_fp64_tc_over_the_exponent_range(tn, K, row, col, alpha, beta):
     assert np.all(got[3] == (beta * C0)[3])
 
 
+@pytest.mark.parametrize("ta,tb", [("N", "N"), ("T", "T")])
+@pytest.mark.parametrize("M_,N_,K_", [(70, 130, 700), (1300, 70, 1500), (2500, 90, 600), (5000, 40, 65), (70, 40, 4000)])
+def test_fp64_tc_slicing_blocks(tn, M_, N_, K_, ta, tb):
+    """4, 8, 16 and 32 rows a block of the one-pass slicing, and the two-kernel form
+    for an inner dimension that does not fit; rows over many binades."""
+    rng = np.random.default_rng(K_)
+    A = rng.standard_normal((M_, K_)) * np.ldexp(1.0, rng.integers(-60, 60, (M_, 1)))
+    B = rng.standard_normal((K_, N_)) * np.ldexp(1.0, rng.integers(-60, 60, (1, N_)))
+    A[7], B[:, 3] = 0.0, 0.0
+    got = tn.gemm(np.asfortranarray(A.T if ta == "T" else A), np.asfortranarray(B.T if tb == "T" else B), ta, tb,
+                  prec=tn._lib.PREC_FP64_TC)
+    # each of the K products is off by 2^-47 of scales up to twice the largest entries
+    tol = K_ * 2.0 ** -45 * np.abs(A).max(axis=1, keepdims=True) * np.abs(B).max(axis=0, keepdims=True)
+    assert np.all(np.abs(got - A @ B) <= tol)
+    assert not got[7].any() and not got[:, 3].any()
+
+
 @pytest.mark.parametrize("batch,n_in,width,n_out", [(1, 7, 40, 33), (31, 32, 64, 129), (33, 81, 65, 64),
                                                     (130, 20, 600, 70)])
 def test_network_gradient_edges(tn, batch, n_in, width, n_out):
