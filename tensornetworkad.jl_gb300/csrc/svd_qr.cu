@@ -21,9 +21,9 @@
 // it is 6-10, and the rank cut leaves ~250 of 400 columns of a χ = 20 split.
 // Each stage is one cooperative kernel (one launch instead of n − 1 per sweep).
 // Measured on one GB300 against FP64 element rounds (k_jacobi_round_cta): TRG at
-// χ = 20, 7 steps with gradient 704 → 28 ms; D=3, χ=36 energy and gradient (n =
-// 324) 349 → 65 ms; one n = 80 decomposition 4.9 → 1.4 ms, n = 255 26.7 → 5.9 ms.
-// At n = 324 the first QR takes 2.0 ms, the FP32 sweeps 2.2, the FP64 ones 2.3.
+// χ = 20, 7 steps with gradient 718 → 24 ms; D=3, χ=36 energy and gradient (n =
+// 324) 366 → 48 ms; one n = 80 decomposition 4.9 → 1.1 ms, n = 255 26.7 → 4.5 ms.
+// At n = 324 the first QR takes 1.5 ms, the FP32 sweeps 2.0, the FP64 ones 2.4.
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
@@ -554,6 +554,8 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
   }
   const int grp = threadIdx.x >> 6, lt = threadIdx.x & 63, wip = (threadIdx.x >> 5) & 1, lane = threadIdx.x & 31;
   const float tolf = (float)a.tol;
+  // a warp without rows in the last chunk leaves the FP64 units to the others (mx ≥ rc)
+  const bool last = 64 * (RJ - 1) + 32 * wip < mx;
 
   // rotate local columns x < y (in global order) of this thread group; their W
   // rows stay in registers between the dot product and the rotation
@@ -570,8 +572,10 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
       double g1 = 0.0;
 #pragma unroll
       for (int e = 0; e < RJ; ++e) {
-        if (e & 1) g1 = fma(u[e], v[e], g1);
-        else g = fma(u[e], v[e], g);
+        if (e < RJ - 1 || last) {
+          if (e & 1) g1 = fma(u[e], v[e], g1);
+          else g = fma(u[e], v[e], g);
+        }
       }
       if (RJ > 1) g += g1;
       g = wsum_d(g);
@@ -594,8 +598,10 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
 #pragma unroll
         for (int e = 0; e < RJ; ++e) {
           const int i = lt + 64 * e;
-          wx[i] = cs * u[e] - sn * v[e];
-          wy[i] = sn * u[e] + cs * v[e];
+          if (e < RJ - 1 || last) {
+            wx[i] = cs * u[e] - sn * v[e];
+            wy[i] = sn * u[e] + cs * v[e];
+          }
         }
         if (ACCV) {
           double* vx = wx + ldw;
@@ -608,8 +614,10 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
 #pragma unroll
           for (int e = 0; e < RJ; ++e) {
             const int i = lt + 64 * e;
-            vx[i] = cs * u[e] - sn * v[e];
-            vy[i] = sn * u[e] + cs * v[e];
+            if (e < RJ - 1 || last) {
+              vx[i] = cs * u[e] - sn * v[e];
+              vy[i] = sn * u[e] + cs * v[e];
+            }
           }
         }
         asm volatile("bar.sync %0, 64;" ::"r"(grp + 1) : "memory");  // norms read by all of the group
@@ -736,8 +744,9 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
 // A group keeps its column of P in registers through the inner rounds, so that
 // shared memory carries Q's columns only (128 bytes a clock limit n = 1024).
 // Measured: n = 1024 15 ms for 9-10 sweeps, as 255 launches a sweep of 4-column
-// blocks 17.9; D=3, χ=36 energy and gradient (n = 324) 64 → 56 ms against one
-// 16-CTA cluster with scalar loads.
+// blocks 17.9; n = 324 2.0 ms, 3.4 in one 16-CTA cluster with scalar loads.  A wait
+// for the round's two blocks only, by a flag a block, instead of the grid barrier
+// took 16.8 ms at n = 1024.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t pk2(float a, float b) {
   return ((uint64_t)__float_as_uint(b) << 32) | __float_as_uint(a);
@@ -1285,9 +1294,9 @@ void launch_sweeps32_rv(tnad_ctx* c, int np, SvdArgs& a) {
 }
 
 // Up to 128 columns the at most 8 CTAs form a cluster.  One warp per pair up to
-// 512 rows (a second one's share of the sums costs a barrier: n = 324 64 → 56 ms
-// as above), two beyond, where a lane would hold 64 registers of each column; and
-// there blocks of 4, which spread 1024 columns over 128 SMs' shared memories.
+// 512 rows (a second one's share of the sums costs a barrier), two beyond, where a
+// lane would hold 64 registers of each column; and there blocks of 4, which spread
+// 1024 columns over 128 SMs' shared memories.
 template <bool EIG>
 void launch_sweeps32(tnad_ctx* c, int np, SvdArgs& a) {
   if (a.n <= 128)
