@@ -10,16 +10,40 @@
 
 namespace tnad {
 
+// Tensors up to a quarter of a chunk are cut from chunks of 1 MB, doubling to
+// 32 MB: a recorded run asks for up to 16 small tensors a step, and a cudaMalloc
+// and cudaFree for each took 0.15 of 2.33 ms of TRG at χ = 5 (5 steps, gradient).
+// Larger ones are allocated by themselves.
+// Everything is given back with the pool.
 double* DevPool::d(int64_t n) {
-  void* p = nullptr;
-  size_t bytes = (size_t)std::max<int64_t>(n, 1) * 8;
-  cudaError_t e = cudaMalloc(&p, bytes);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    fail(TNAD_ERR_NOMEM, "tape cudaMalloc failed");
+  constexpr size_t kFirst = 1 << 20, kLast = 32 << 20;
+  const size_t want = (size_t)std::max<int64_t>(n, 1) * 8, need = (want + 255) & ~(size_t)255;
+  auto alloc = [&](size_t size) -> void* {
+    void* p = nullptr;
+    if (cudaMalloc(&p, size) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    ptrs.push_back(p);
+    return p;
+  };
+  if (need > left && need <= std::max(chunk, kFirst) / 4) {
+    const size_t size = std::min(chunk ? 2 * chunk : kFirst, kLast);
+    if (void* p = alloc(size)) {
+      cur = (char*)p;
+      left = chunk = size;
+    }
   }
-  ptrs.push_back(p);
-  this->bytes += (int64_t)bytes;
+  void* p;
+  if (need <= left) {
+    p = cur;
+    cur += need;
+    left -= need;
+  } else {
+    p = alloc(want);
+    if (!p) fail(TNAD_ERR_NOMEM, "tape cudaMalloc failed");
+  }
+  this->bytes += (int64_t)want;
   return (double*)p;
 }
 
@@ -27,6 +51,8 @@ void DevPool::free_all() {
   for (void* p : ptrs) cudaFree(p);
   ptrs.clear();
   bytes = 0;
+  cur = nullptr;
+  left = chunk = 0;
 }
 
 __global__ void k_init_raw(const double* __restrict__ a, int d, int chi, double* __restrict__ C,

@@ -11,7 +11,9 @@ namespace tnad {
 // Device memory owned by a tape (freed by tnad_tape_free).
 struct DevPool {
   std::vector<void*> ptrs;
-  int64_t bytes = 0;
+  int64_t bytes = 0;   // requested
+  char* cur = nullptr;  // rest of the newest chunk
+  size_t left = 0, chunk = 0;
   double* d(int64_t n);
   void free_all();
   ~DevPool() { free_all(); }
