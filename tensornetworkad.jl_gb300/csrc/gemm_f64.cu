@@ -45,13 +45,15 @@ struct GemmArgs {
   int a_rows, b_rows;  // lanes run along the rows (columns) of the tile, else along K
 };
 
-template <int BM>
+// SYM: C = Cᵀ, the tiles above the diagonal are the others' mirror images
+template <int BM, bool SYM>
 __global__ void __launch_bounds__(256) k_gemm_f64(const GemmArgs g) {
   constexpr int BK = 16, T = BM / 16;  // T×T outputs and T loads per operand and thread
   __shared__ double As[2][BK][BM + 1];
   __shared__ double Bs[2][BK][BM + 1];
   __shared__ int last;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  if (SYM && blockIdx.y > blockIdx.x) return;
   const unsigned m0 = blockIdx.x * BM, n0 = blockIdx.y * BM;
   const unsigned kbeg = blockIdx.z * g.kchunk, kend = min(g.K, kbeg + g.kchunk);
   // this thread's elements of a slice: (row ai[q], inner ak[q]) and (inner, column)
@@ -151,6 +153,7 @@ __global__ void __launch_bounds__(256) k_gemm_f64(const GemmArgs g) {
       double v = acc[i][j];
       if (g.scaled) v *= g.alpha;
       *c = g.accum ? v + g.beta * (*c) : v;
+      if (SYM && blockIdx.y < blockIdx.x) g.C[map_off(g.cm, gj) + map_off(g.cn, gi)] = *c;
     }
   }
 }
@@ -186,7 +189,7 @@ void gemm_f64_plan(int sms, int64_t M, int64_t N, int64_t K, int* tile, int* spl
 
 void gemm_f64_map(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, const GemmMap& am,
                   const GemmMap& ak, const double* B, const GemmMap& bk, const GemmMap& bn, double beta, double* C,
-                  const GemmMap& cm, const GemmMap& cn) {
+                  const GemmMap& cm, const GemmMap& cn, bool sym) {
   TNAD_REQUIRE(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), TNAD_ERR_ARG, "gemm_f64: size");
   int tile = 64, ks = 1;
   gemm_f64_plan(c->sm_count, M, N, K, &tile, &ks);
@@ -219,12 +222,13 @@ void gemm_f64_map(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, co
   g.part = g.ks > 1 ? ws_d(c, (int64_t)g.ks * tm * tn * tile * tile) : nullptr;
   const dim3 grid((unsigned)tm, (unsigned)tn, (unsigned)g.ks);
   KernelTimer kt(c, "gemm_f64", 2.0 * (double)M * (double)N * (double)K);
+  auto launch = [&](auto* kernel) { kernel<<<grid, 256, 0, c->stream>>>(g); };
   if (tile == 64)
-    k_gemm_f64<64><<<grid, 256, 0, c->stream>>>(g);
+    launch(sym ? k_gemm_f64<64, true> : k_gemm_f64<64, false>);
   else if (tile == 32)
-    k_gemm_f64<32><<<grid, 256, 0, c->stream>>>(g);
+    launch(sym ? k_gemm_f64<32, true> : k_gemm_f64<32, false>);
   else
-    k_gemm_f64<16><<<grid, 256, 0, c->stream>>>(g);
+    launch(sym ? k_gemm_f64<16, true> : k_gemm_f64<16, false>);
   count_launch(c);
   check_launch(c, "gemm_f64");
 }
@@ -294,6 +298,11 @@ static GemmMap map1(int64_t n, int64_t stride) {
   m.dim[0] = (unsigned)n;
   m.str[0] = stride;
   return m;
+}
+
+void gemm_f64_gram(tnad_ctx* c, int64_t n, int64_t K, const double* A, const double* B, double* C) {
+  gemm_f64_map(c, n, n, K, 1.0, A, map1(n, K), map1(K, 1), B, map1(K, 1), map1(n, K), 0.0, C, map1(n, 1), map1(n, n),
+               true);
 }
 
 void gemm_f64(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K, double alpha, const double* A,

@@ -225,7 +225,10 @@ struct GemmMap {
 };
 void gemm_f64_map(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, const GemmMap& am,
                   const GemmMap& ak, const double* B, const GemmMap& bk, const GemmMap& bn, double beta, double* C,
-                  const GemmMap& cm, const GemmMap& cn);
+                  const GemmMap& cm, const GemmMap& cn, bool sym = false);
+// C (n×n) = AᵀB for K×n A and B with a symmetric product (XᵀX, Xᵀ(MX) of symmetric
+// M): the tiles below the diagonal and their mirror images, half of the work
+void gemm_f64_gram(tnad_ctx* c, int64_t n, int64_t K, const double* A, const double* B, double* C);
 // Whether a product of this size runs as DFMA tiles under `prec` on this context.
 bool gemm_is_f64(const tnad_ctx* c, int prec, int64_t M, int64_t N, int64_t K);
 // Same contract, 3xTF32 on tcgen05 tensor cores with FP32 accumulation.
