@@ -96,33 +96,38 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-template <int MODE>  // 0: Σx², 1: Σx·y
-__global__ void k_reduce_partial(const double* __restrict__ x, const double* __restrict__ y, int64_t n,
-                                 double* __restrict__ part) {
+// out[0] = Σx² (MODE 0) or Σx·y (1); if sqrt_to != null also writes the root into
+// sqrt_to[0].  The block that arrives last adds the blocks' sums, in their order:
+// a second launch for that took 3.3 µs and its gap.
+template <int MODE>
+__global__ void k_reduce(const double* __restrict__ x, const double* __restrict__ y, int64_t n, double* part, int* cnt,
+                         double* out, double* sqrt_to) {
+  __shared__ double sh[32];
+  __shared__ int last;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   double s = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double v = x[i];
     s += MODE == 0 ? v * v : v * y[i];
   }
-  __shared__ double sh[32];
   s = warp_sum(s);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   if (l == 0) sh[w] = s;
   __syncthreads();
   if (w == 0) {
     double t = l < (int)(blockDim.x >> 5) ? sh[l] : 0.0;
     t = warp_sum(t);
-    if (l == 0) part[blockIdx.x] = t;
+    if (l == 0) {
+      __stcg(&part[blockIdx.x], t);
+      __threadfence();
+      last = atomicAdd(cnt, 1) == (int)gridDim.x - 1;
+    }
   }
-}
-
-// out[0] = Σ part[0..np); if sqrt_to != null also writes sqrt into sqrt_to[0]
-__global__ void k_reduce_final(const double* __restrict__ part, int np, double* out, double* sqrt_to) {
-  double s = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) s += part[i];
-  __shared__ double sh[32];
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  s = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) s += __ldcg(&part[i]);
   s = warp_sum(s);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   if (l == 0) sh[w] = s;
   __syncthreads();
   if (w == 0) {
@@ -131,6 +136,7 @@ __global__ void k_reduce_final(const double* __restrict__ part, int np, double* 
     if (l == 0) {
       out[0] = t;
       if (sqrt_to) sqrt_to[0] = sqrt(t);
+      *cnt = 0;  // for the next launch on this stream
     }
   }
 }
@@ -273,11 +279,10 @@ static void reduce2(tnad_ctx* c, int mode, const double* x, const double* y, int
   int nb = nblocks(n, 256, 1024);
   double* part = c->d_red + 2048;
   if (mode == 0)
-    k_reduce_partial<0><<<nb, 256, 0, c->stream>>>(x, y, n, part);
+    k_reduce<0><<<nb, 256, 0, c->stream>>>(x, y, n, part, c->d_cnt, out, sqrt_to);
   else
-    k_reduce_partial<1><<<nb, 256, 0, c->stream>>>(x, y, n, part);
-  k_reduce_final<<<1, 256, 0, c->stream>>>(part, nb, out, sqrt_to);
-  count_launch(c, 2);
+    k_reduce<1><<<nb, 256, 0, c->stream>>>(x, y, n, part, c->d_cnt, out, sqrt_to);
+  count_launch(c);
   check_launch(c, "reduce");
 }
 
@@ -321,9 +326,8 @@ void div_by_dev(tnad_ctx* c, double* x, int64_t n, const double* dev_s) {
 void normalize_inplace(tnad_ctx* c, double* x, int64_t n, double* dev_norm_out) {
   int nb = nblocks(n, 256, 1024);
   double* part = c->d_red + 2048;
-  k_reduce_partial<0><<<nb, 256, 0, c->stream>>>(x, nullptr, n, part);
-  k_reduce_final<<<1, 256, 0, c->stream>>>(part, nb, c->d_red + 8, dev_norm_out);
-  count_launch(c, 2);
+  k_reduce<0><<<nb, 256, 0, c->stream>>>(x, nullptr, n, part, c->d_cnt, c->d_red + 8, dev_norm_out);
+  count_launch(c);
   div_by_dev(c, x, n, dev_norm_out);
 }
 

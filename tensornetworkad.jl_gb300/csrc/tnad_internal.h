@@ -81,7 +81,7 @@ struct tnad_ctx {
   double* h_pin = nullptr;  // pinned host mirror (64 doubles)
   int* d_flag = nullptr;    // device flags / counters (64 ints)
   int* h_flag = nullptr;    // pinned host mirror of the flags
-  int* d_cnt = nullptr;     // arrival counters of split products (kGemmCounters, zero between launches)
+  int* d_cnt = nullptr;     // arrival counters of split products and reductions (kGemmCounters, zero between launches)
   bool tc_ok = false;       // tcgen05 GEMM path available (sm_100 family)
   // One-shot fault injection for the failure-path tests, set from the
   // environment variable TNAD_TEST_FAULT when the context is created:
