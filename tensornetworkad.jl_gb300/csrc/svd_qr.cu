@@ -671,8 +671,10 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
         }
         if (r > 0 && threadIdx.x < 4 && gc(threadIdx.x) < rc) nrm4[threadIdx.x] = __ldcg(&q.nrm[gc(threadIdx.x)]);
         asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
+        // read before the barrier: after it the other group may already count a
+        // rotation of this round, and the threads would not agree on the write-back
         const int rot0 = nrot;
+        __syncthreads();
         if (r == 0) {  // norms anew: warp w takes column w
           const int w = threadIdx.x >> 5;
           double s = 0.0;
