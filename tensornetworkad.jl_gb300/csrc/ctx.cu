@@ -125,6 +125,7 @@ extern "C" int tnad_ctx_create(tnad_ctx** out, int device) {
     if (const char* f = std::getenv("TNAD_TEST_FAULT")) {
       if (!std::strcmp(f, "tc_withhold")) c->fault_once = kFaultTcWithhold;
       if (!std::strcmp(f, "jacobi_cap")) c->fault_once = kFaultJacobiCap;
+      if (!std::strcmp(f, "qr_timeout")) c->fault_once = kFaultQrTimeout;
     }
   } catch (const Error& e) {
     int code = e.code;

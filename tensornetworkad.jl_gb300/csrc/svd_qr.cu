@@ -1023,7 +1023,7 @@ __global__ void k_svd_norms(SvdArgs a) {
   const SvdProb& q = a.p[blockIdx.y];
   const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int rc = q.info[kiRank];
-  if (j >= a.n) return;
+  if (j >= a.n || q.info[kiErr]) return;
   double s = 0.0;
   if (j < rc) {
     const bool two = a.second || rc < a.n;
@@ -1045,6 +1045,7 @@ __global__ void __launch_bounds__(128) k_svd_place(SvdArgs a) {
   const SvdProb& q = a.p[blockIdx.y];
   const int j = blockIdx.x, m = a.m, n = a.n;
   const int rc = q.info[kiRank];
+  if (q.info[kiErr]) return;  // a wait gave up: perm and perm2, which this kernel stores through, may be unwritten
   const bool two = a.second || rc < n;
   const double sj = q.sv[j];
   int rk = j;
@@ -1327,7 +1328,8 @@ void pre_sweeps(tnad_ctx* c, int np, SvdArgs& a, int* info_host) {
     const int r = info_host[p * kiBar + kiRank];
     const bool two = a.second || r < a.n;
     const int mx = two ? r : a.n;
-    if (r < 2 || info_host[p * kiBar + kiErr]) continue;  // (q.W stays null: nothing to hand over)
+    TNAD_REQUIRE(info_host[p * kiBar + kiErr] == 0, TNAD_ERR_TIMEOUT, "svd_qrj: a bounded barrier wait expired");
+    if (r < 2) continue;  // (q.W stays null: nothing to hand over)
     WsScope scope(c);
     double* F = ws_d(c, (int64_t)r * r);
     double* V2 = ws_d(c, (int64_t)a.ldx * r);
@@ -1349,6 +1351,10 @@ void pre_sweeps(tnad_ctx* c, int np, SvdArgs& a, int* info_host) {
 template <int R>
 void svd_qrj_r(tnad_ctx* c, int np, bool symmetric, SvdArgs& a, int* info_host) {
   launch_qrcp<R, 0>(c, np, a.n, a);
+  if (c->fault_once == kFaultQrTimeout) {  // failure-path test: as if a wait of the second QR had expired
+    for (int p = 0; p < np; ++p) TNAD_CK(cudaMemsetAsync(a.p[p].info + kiErr, 1, sizeof(int), c->stream));
+    c->fault_once = kFaultNone;
+  }
   launch_qrcp<R, 1>(c, np, a.n, a);
   if (a.n >= kPreMin) pre_sweeps(c, np, a, info_host);
   int rows = 0;  // of the triangular factors

@@ -89,7 +89,10 @@ struct tnad_ctx {
   //     loads of its first K slice and waits at most 20 ms on an mbarrier, so
   //     the bounded wait runs out (TNAD_ERR_TIMEOUT) with no copy in flight;
   //   kFaultJacobiCap — the next Jacobi SVD is capped at one FP64 sweep
-  //     (TNAD_ERR_NOT_CONVERGED).
+  //     (TNAD_ERR_NOT_CONVERGED);
+  //   kFaultQrTimeout — the next QR-preconditioned SVD finds its error word set
+  //     after the first factorisation, as a wait that expired leaves it
+  //     (TNAD_ERR_TIMEOUT).
   // Each is cleared when used; later calls on the context run normally.
   int fault_once = 0;
   // FP64 products (TNAD_PREC_FP64) of the current call run as gemm_fp64tc on
@@ -125,7 +128,7 @@ namespace tnad {
 
 constexpr int64_t kGemmCounters = 4096;  // tiles of a product whose K may be split
 
-enum { kFaultNone = 0, kFaultTcWithhold = 1, kFaultJacobiCap = 2 };
+enum { kFaultNone = 0, kFaultTcWithhold = 1, kFaultJacobiCap = 2, kFaultQrTimeout = 3 };
 
 // Phase timer: with TNAD_TRACE set in the environment, CUDA events bracket
 // named phases on the context stream and a per-phase summary goes to stderr
