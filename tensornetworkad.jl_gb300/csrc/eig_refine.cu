@@ -43,6 +43,7 @@
 #include <cstring>
 #include <vector>
 
+#include "orth_steps.h"
 #include "tnad_internal.h"
 
 namespace tnad {
@@ -768,8 +769,8 @@ bool eig_refine(tnad_ctx* c, const double* A, int64_t n64, double* X, double* la
       float em;
       std::memcpy(&em, hs + 3, sizeof(em));
       if (em <= 1e-8f) break;
-      // X is orthogonal up to ~4E²; every step squares that
-      for (double d = 16.0 * (double)em * em * em * em; d > 1e-16; d *= d) ++steps;
+      steps = orth_steps(em);
+      if (steps == 0) return false;
     }
     for (int ns = 0; ns < steps; ++ns) {
       if (ns > 0) copy_d2d(c, Xn, X, nn);
