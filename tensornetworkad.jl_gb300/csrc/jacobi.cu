@@ -488,6 +488,59 @@ __global__ void k_scatter_eig(const double* __restrict__ X, const double* __rest
   if (blockIdx.x == 0 && threadIdx.x == 0) S[r] = fabs(l);
 }
 
+// lam_j = x_j·w_j (one warp per column)
+__global__ void k_rayleigh(const double* __restrict__ X, const double* __restrict__ W, int64_t n,
+                           double* __restrict__ lam) {
+  const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (j >= n) return;
+  double s = 0.0;
+  for (int64_t i = lane; i < n; i += 32) s = fma(X[i + j * n], W[i + j * n], s);
+  s = wsum(s);
+  if (lane == 0) lam[j] = s;
+}
+
+void eig_separate(tnad_ctx* c, const double* A, int64_t n, double* X, double floor_rel, double* U, double* S,
+                  double* V) {
+  double s0 = 0.0;
+  TNAD_CK(cudaMemcpyAsync(&s0, S, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  TNAD_CK(cudaStreamSynchronize(c->stream));
+  const int e = std::max(-1000, std::min(1000, std::ilogb(s0)));  // sweeps on A·2^-e: no product of two entries overflows
+  WsScope scope(c);
+  double* W = ws_d(c, n * n);
+  double* lam = ws_d(c, n);
+  double* one = ws_d(c, 1);
+  int* rank = (int*)c->ws.alloc(n * sizeof(int));
+  fill(c, one, 1, 1.0);
+  gemm_f64(c, 'N', 'N', n, n, n, std::ldexp(1.0, -e), A, n, X, n, 0.0, W, n);
+  const double thr = floor_rel * std::ldexp(s0, -e), round_flops = (double)(n / 2) * 18.0 * (double)n;
+  SweepGraph<double, true> sweeps;
+  bool converged = false;
+  for (int sweep = 0; sweep < kMaxSweeps && !converged; ++sweep) {
+    sweeps.run(c, "jacobi_separate", W, X, n, n, (int)(n + (n & 1)), 0.0, thr, one, c->d_flag, round_flops);
+    TNAD_CK(cudaMemcpyAsync(c->h_flag, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    TNAD_CK(cudaStreamSynchronize(c->stream));
+    converged = c->h_flag[0] == 0;
+    if (std::getenv("TNAD_TRACE"))
+      std::fprintf(stderr, "[tnad trace] eig_separate n=%lld sweep %d rotations %d\n", (long long)n, sweep, c->h_flag[0]);
+  }
+  TNAD_REQUIRE(converged, TNAD_ERR_NOT_CONVERGED, "eig_separate: no convergence within the sweep cap");
+  // The rotations' rounding adds up over a large multiplet (5e-14 at n = 200), and the
+  // start's columns are orthogonal to a few √n·ε: X ← X·(3I − XᵀX)/2 squares both away
+  double* X2 = ws_d(c, n * n);
+  gemm_f64_gram(c, n, n, X, X, W);
+  copy_d2d(c, X2, X, n * n);
+  gemm_f64(c, 'N', 'N', n, n, n, -0.5, X, n, W, n, 1.5, X2, n);
+  gemm_f64(c, 'N', 'N', n, n, n, std::ldexp(1.0, -e), A, n, X2, n, 0.0, W, n);
+  k_rayleigh<<<(int)((n * 32 + 255) / 256), 256, 0, c->stream>>>(X2, W, n, lam);
+  if (e != 0) scale(c, n, std::ldexp(1.0, e), lam);
+  k_eig_rank<<<(int)((n * 32 + 255) / 256), 256, 0, c->stream>>>(lam, n, rank);
+  const dim3 g((unsigned)std::min<int64_t>((n + 255) / 256, 16), (unsigned)n);
+  k_scatter_eig<<<g, 256, 0, c->stream>>>(X2, lam, rank, n, U, S, V);
+  count_launch(c, 3);
+  check_launch(c, "eig_separate");
+}
+
 void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, double* S, double* V,
                 bool symmetric, int rel_sweeps) {
   TNAD_REQUIRE(m >= n && n >= 1, TNAD_ERR_SHAPE, "svd_jacobi: needs m >= n >= 1");

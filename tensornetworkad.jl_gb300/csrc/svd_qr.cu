@@ -12,7 +12,8 @@
 //
 // so that A = (Q·P₂·Wn)·Σ·(P·Q₂·Vx)ᵀ, completed by the trailing columns of Q
 // and P·Q₂ where r < n.  Symmetric A with r = n skips the second QR and the
-// accumulation of Vx: the eigenvectors are P·Wn.
+// accumulation of Vx: the singular vectors are P·Wn, and k_svd_sym_basis makes
+// eigenvectors of them.
 //
 // Why: GB300 issues one FP64 instruction per warp and SM quadrant every 64
 // clocks (76 with all four busy), so the sweeps are paid in instructions and in
@@ -51,9 +52,9 @@ constexpr int kScaleExp = 40;  // the largest |entry| is scaled to 2^40: squared
                                // columns down to ½ε of it stay inside the FP32 range
 
 // Per-problem counters (ints): rank, non-finite input, converged sweep count
-// (0: none), barrier counter of each of the three kernels, rotations per sweep
+// (0: none), scale, error, FP32 sweeps, multiplets to separate, barrier counter of each of the three kernels, rotations per sweep
 // and the largest |cos| of a rotated pair per sweep (float bits).
-enum { kiRank = 0, kiBad = 1, kiSweeps = 2, kiExp = 3, kiErr = 4, kiPre = 5, kiBar = 8, kiRot = 16, kiCos = 16 + kSvdSweeps,
+enum { kiRank = 0, kiBad = 1, kiSweeps = 2, kiExp = 3, kiErr = 4, kiPre = 5, kiMulti = 6, kiBar = 8, kiRot = 16, kiCos = 16 + kSvdSweeps,
        kiTan = 16 + 2 * kSvdSweeps, kiRot32 = 16 + 3 * kSvdSweeps, kiCos32 = kiRot32 + kEigSweeps, kiCount = kiCos32 + kEigSweeps };
 
 struct SvdProb {
@@ -1144,62 +1145,64 @@ __global__ void __launch_bounds__(128) k_svd_apply_q(SvdArgs a) {
   }
 }
 
-// Left vectors of a symmetric A from its right ones: U_j = sign(λ_j)·V_j with
-// λ_j = v_j·(A·v_j).  Where σ_j is shared (to 1e-8) and above 1e-8·σ_1, V only
-// spans the singular subspace (a ±λ pair may come out mixed) and U follows
-// from A·V: a pair takes the 2×2 block h = VᵀAV/σ of its subspace, which is a
-// reflection [[c, s], [s, −c]] for ±λ (or ±I), normalised so that U stays
-// orthonormal to rounding; larger groups take A·v/σ.  One CTA per column.
-__global__ void __launch_bounds__(128) k_svd_sym_left(int n, const double* __restrict__ V,
-                                                      const double* __restrict__ AV, const double* __restrict__ S,
-                                                      double* __restrict__ U) {
+// Eigenvectors of a symmetric A from its singular vectors X (σ descending in S).
+// X spans what it has to, but only up to rotations by ~ε·‖A‖/||λ_i| − |λ_j|| between
+// columns: where λ_i and λ_j have opposite signs and about the same size (exact ±λ
+// pairs, any size; or close ones), x_j is then no eigenvector and ±x_j no left vector.
+// M = XᵀAX shows it: an entry above thr_rel·σ_1, twice the rounding of M, is such a
+// coupling.  A column without one is kept, a pair takes the eigenvectors of its 2×2
+// block, and a column in a larger group (a multiplet of both signs) sets *multi,
+// upon which the caller separates them by eigenvalue sweeps (eig_separate).
+// U = V·sign(λ).  One CTA per column.
+__global__ void __launch_bounds__(128) k_svd_sym_basis(int n, const double* __restrict__ X,
+                                                       const double* __restrict__ M, const double* __restrict__ S,
+                                                       double thr_rel, double* __restrict__ U, double* __restrict__ V,
+                                                       int* __restrict__ multi) {
   const int j = blockIdx.x;
-  __shared__ double red[4][4];
-  const double sj = S[j];
-  auto near = [&](int x, int y) { return fabs(S[x] - S[y]) <= 1e-8 * S[y]; };
-  int lo = j, hi = j;
-  if (sj > 1e-8 * S[0]) {
-    while (lo > 0 && j - lo < 2 && near(lo - 1, lo)) --lo;
-    while (hi + 1 < n && hi - j < 2 && near(hi, hi + 1)) ++hi;
-  }
-  const int o = hi - lo == 1 ? (j == lo ? hi : lo) : j;  // partner of a pair
-  double h[4] = {0.0, 0.0, 0.0, 0.0};  // v_j·Av_j, v_o·Av_o, v_o·Av_j, v_j·Av_o
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double vj = V[i + (int64_t)j * n], wj = AV[i + (int64_t)j * n];
-    h[0] = fma(vj, wj, h[0]);
-    if (o != j) {
-      const double vo = V[i + (int64_t)o * n], wo = AV[i + (int64_t)o * n];
-      h[1] = fma(vo, wo, h[1]);
-      h[2] = fma(vo, wj, h[2]);
-      h[3] = fma(vj, wo, h[3]);
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const double t = wsum_d(h[e]);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][e] = t;
+  const double thr = thr_rel * S[0];
+  __shared__ int cnt[2], who[2];  // coupled columns of this one and of its partner
+  if (threadIdx.x < 2) {
+    cnt[threadIdx.x] = 0;
+    who[threadIdx.x] = -1;
   }
   __syncthreads();
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    h[e] = red[0][e] + red[1][e] + red[2][e] + red[3][e];
-    if (sj > 0.0) h[e] /= sj;
+  auto scan = [&](int col, int slot) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+      if (i != col && fabs(M[i + (int64_t)col * n]) > thr) {
+        atomicAdd(&cnt[slot], 1);
+        who[slot] = i;
+      }
+  };
+  scan(j, 0);
+  __syncthreads();
+  const int o = cnt[0] == 1 ? who[0] : -1;
+  if (o >= 0) scan(o, 1);
+  __syncthreads();
+  const bool pair = o >= 0 && cnt[1] == 1;  // (M is symmetric to the bit: the partner's partner is j)
+  if (cnt[0] > 0 && !pair && threadIdx.x == 0) *multi = 1;
+  const int lo = pair ? min(j, o) : j, hi = pair ? max(j, o) : j;
+  double cl = 1.0, ch = 0.0, lam = M[j + (int64_t)j * n];
+  if (pair) {
+    const double a = M[lo + (int64_t)lo * n], b = M[hi + (int64_t)hi * n], g = M[hi + (int64_t)lo * n];
+    const double tau = (b - a) / (2.0 * g);
+    const double t = copysign(1.0, tau) / (fabs(tau) + sqrt(fma(tau, tau, 1.0)));
+    const double c = 1.0 / sqrt(fma(t, t, 1.0)), s = c * t, la = a - t * g, lb = b + t * g;
+    const bool swap = fabs(la) < fabs(lb);  // S is in descending order
+    if ((j == lo) != swap) {
+      cl = c;
+      ch = -s;
+      lam = la;
+    } else {
+      cl = s;
+      ch = c;
+      lam = lb;
+    }
   }
-  double cj = h[0] < 0.0 ? -1.0 : 1.0, co = 0.0;
-  const bool from_av = hi - lo > 1;
-  const double b = 0.5 * (h[2] + h[3]);  // the same bits for both columns of the pair
-  if (o != j && (h[0] * h[1] < 0.0 || fabs(b) > 0.5)) {  // a ±λ pair: U_j = c·V_j + s·V_o
-    const double c0 = 0.5 * (h[0] - h[1]), r = 1.0 / sqrt(c0 * c0 + b * b);
-    cj = c0 * r;
-    co = b * r;
-  }
+  const double sg = lam < 0.0 ? -1.0 : 1.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    double u;
-    if (from_av)
-      u = AV[i + (int64_t)j * n] / sj;
-    else
-      u = co == 0.0 ? cj * V[i + (int64_t)j * n] : cj * V[i + (int64_t)j * n] + co * V[i + (int64_t)o * n];
-    U[i + (int64_t)j * n] = u;
+    const double v = pair ? cl * X[i + (int64_t)lo * n] + ch * X[i + (int64_t)hi * n] : X[i + (int64_t)j * n];
+    V[i + (int64_t)j * n] = v;
+    U[i + (int64_t)j * n] = sg * v;
   }
 }
 
@@ -1469,7 +1472,7 @@ void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, 
     q.sv = ws_d(c, n);
     q.U = U[p];
     q.S = S[p];
-    q.V = V[p];
+    q.V = symmetric ? ws_d(c, n * n) : V[p];  // the basis that k_svd_sym_basis starts from
     q.info = info + p * kiCount;
   }
   TNAD_CK(cudaMemsetAsync(cands, 0, nzero, c->stream));
@@ -1488,14 +1491,18 @@ void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, 
     else
       svd_qrj_r<32>(c, np, symmetric, a, h);
   }
+  const double couple = 8.0 * std::sqrt((double)std::max<int64_t>(n, 16)) * DBL_EPSILON;
   if (symmetric) {
-    for (int p = 0; p < np; ++p) {
+    for (int p = 0; p < np; ++p) {  // DFMA products: M has to be accurate to the rounding of A
       WsScope inner(c);
-      double* AV = ws_d(c, n * n);
-      gemm(c, TNAD_PREC_FP64, 'N', 'N', n, n, n, 1.0, A[p], n, V[p], n, 0.0, AV, n);
-      k_svd_sym_left<<<(unsigned)n, 128, 0, c->stream>>>((int)n, V[p], AV, S[p], U[p]);
+      double* AX = ws_d(c, n * n);
+      double* M = ws_d(c, n * n);
+      gemm_f64(c, 'N', 'N', n, n, n, 1.0, A[p], n, a.p[p].V, n, 0.0, AX, n);
+      gemm_f64_gram(c, n, n, a.p[p].V, AX, M);
+      k_svd_sym_basis<<<(unsigned)n, 128, 0, c->stream>>>((int)n, a.p[p].V, M, S[p], couple, U[p], V[p],
+                                                          a.p[p].info + kiMulti);
       count_launch(c);
-      check_launch(c, "svd_sym_left");
+      check_launch(c, "svd_sym_basis");
     }
   }
   for (int p = 0; p < np; ++p)
@@ -1507,6 +1514,7 @@ void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, 
     if (std::getenv("TNAD_TRACE"))
       std::fprintf(stderr, "[tnad trace] svd_qrj n=%lld rank %d sweeps %d (FP32 %d)\n", (long long)n,
                    h[p * kiBar + kiRank], h[p * kiBar + kiSweeps], h[p * kiBar + kiPre]);
+    if (symmetric && h[p * kiBar + kiMulti]) eig_separate(c, A[p], n, a.p[p].V, couple, U[p], S[p], V[p]);
   }
 }
 

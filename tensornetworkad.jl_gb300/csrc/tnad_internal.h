@@ -282,14 +282,20 @@ void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, d
 // of the same shape m×n (svd_qrj_fits: 1024 ≥ m ≥ n ≥ 2): rank-revealing QR,
 // then Jacobi on the triangular factor, each one launch (svd_qr.cu).  Values
 // below the rounding of A come back as 0, their vectors as an orthonormal
-// completion.  symmetric: U = V·sign(λ) (±λ pairs: from A·V).
+// completion.  symmetric: V eigenvectors, U = V·sign(λ).
+bool svd_qrj_fits(int64_t m, int64_t n);
+void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, double* const* U, double* const* S,
+             double* const* V, bool symmetric);
+// Eigenvectors of a symmetric A (n ≤ 1024) from an orthonormal basis X that
+// diagonalises it up to groups of equal |λ|, by FP64 Jacobi sweeps with the
+// eigenvalue rule: they rotate what is coupled above floor_rel·σ_1.  S[0] = σ_1 on
+// entry.  S = |λ| descending, V the eigenvectors, U = V·sign(λ); X is overwritten.
+void eig_separate(tnad_ctx* c, const double* A, int64_t n, double* X, double floor_rel, double* U, double* S,
+                  double* V);
 // FP32 Jacobi sweeps with the eigenvalue rule on a symmetric A (n ≤ 1024), one
 // launch: V (n×n) orthogonal to ~1e-5, VᵀAV diagonal to ~1e-6·‖A‖.  fro2: ‖A‖²_F
 // on the device.  Returns the number of sweeps (waits for them).
 int sweeps32_eig(tnad_ctx* c, const double* A, int64_t n, const double* fro2, double* V);
-bool svd_qrj_fits(int64_t m, int64_t n);
-void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, double* const* U, double* const* S,
-             double* const* V, bool symmetric);
 // Refines X (n×n, nearly orthonormal approximate eigenvectors of the symmetric
 // A, n ≤ 2048) to FP64 accuracy by matrix products; lam gets the eigenvalues
 // (column order of X).  fro2: ‖A‖²_F on the device.  false: no convergence
