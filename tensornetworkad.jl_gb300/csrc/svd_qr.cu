@@ -34,6 +34,7 @@
 #include <cstdlib>
 
 #include "fp64_fast.cuh"
+#include "sweep_rule.h"
 #include "tc_common.cuh"
 #include "tnad_internal.h"
 
@@ -742,7 +743,7 @@ __global__ void __launch_bounds__(128) k_svd_sweeps(SvdArgs a) {
 // their relative accuracy in FP32, so X·V comes out with |cos| ~ 1e-6 between
 // all columns, small ones included), ended by a sweep that rotated no |cos|
 // above kPreCos; EIG: the 2×2 block of VᵀXV for symmetric X (±λ pairs are not
-// mixed), absolute threshold, ended by a sweep with at most 16n rotations.
+// mixed), absolute threshold, ended by a sweep with at most eig_sweep_last(n) rotations.
 //
 // A group keeps its column of P in registers through the inner rounds, so that
 // shared memory carries Q's columns only (128 bytes a clock limit n = 1024).
@@ -998,7 +999,7 @@ __global__ void __launch_bounds__(32 * B * WP) k_sweeps32(SvdArgs a) {
       if (!bar.sync()) return;
     }
     const int rot = __ldcg(&q.info[kiRot32 + sweep]);
-    done = EIG ? rot <= 16 * rc : rot == 0 || __int_as_float(__ldcg(&q.info[kiCos32 + sweep])) < kPreCos;
+    done = EIG ? rot <= eig_sweep_last(rc) : rot == 0 || __int_as_float(__ldcg(&q.info[kiCos32 + sweep])) < kPreCos;
     if (done && cta == 0 && threadIdx.x == 0) q.info[kiPre] = sweep + 1;
   }
   // V in FP64
