@@ -8,10 +8,10 @@
 //    accumulate in global memory);
 //  - a counter-based Gaussian generator for deterministic start blocks.
 #include <cfloat>
-#include <atomic>
 #include <cmath>
 
 #include "fp64_fast.cuh"
+#include "per_device.h"
 #include "tnad_internal.h"
 
 namespace tnad {
@@ -233,11 +233,11 @@ __global__ void __launch_bounds__(256) k_chol_inv(const double* __restrict__ G, 
 void chol_inv_upper(tnad_ctx* c, const double* G, int64_t p, double* Rinv, int* dev_fail, float near) {
   TNAD_REQUIRE(p >= 1 && p <= kCholMaxP, TNAD_ERR_SHAPE, "chol_inv_upper: p must be in [1,160]");
   constexpr size_t smem = (size_t)(2 * kCholPanels + 1) * kCholNB * kCholLd * sizeof(double);
-  static std::atomic<bool> attr{false};
-  if (!attr) {
+  static PerDevice attr;
+  if (!attr.has(c->device)) {
     TNAD_CK(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     TNAD_CK(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    attr = true;
+    attr.mark(c->device);
   }
   KernelTimer kt(c, "chol", (double)p * p * p / 3.0);
   cudaLaunchConfig_t cf = {};
@@ -594,11 +594,11 @@ __global__ void __launch_bounds__(64 * RV, 1) k_eigh32(const double* __restrict_
 
 template <int RV>
 void eigh32_launch(tnad_ctx* c, const double* A, int p, int max_sweeps, double* lam, double* W, int* info, int by_value) {
-  static std::atomic<bool> attr{false};
-  if (!attr) {
+  static PerDevice attr;
+  if (!attr.has(c->device)) {
     TNAD_CK(cudaFuncSetAttribute(k_eigh32<RV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  2 * kEigh32MaxP * kEigh32MaxP * 4));
-    attr = true;
+    attr.mark(c->device);
   }
   const int pr = (p + 3) & ~3, nreal = (p + 1) / 2, NB = nreal + (nreal & 1);
   k_eigh32<RV><<<1, (4 * NB + 31) / 32 * 32, (size_t)2 * NB * 2 * pr * sizeof(float), c->stream>>>(
@@ -627,10 +627,10 @@ void eigh_small_prec(tnad_ctx* c, bool fp32, const double* A, int64_t p, double*
     const size_t sm = (size_t)(p + 1) * p * 8;
     const size_t kMaxSm = 200 * 1024;
     TNAD_REQUIRE(sm <= kMaxSm, TNAD_ERR_SHAPE, "eigh_small: matrix does not fit in shared memory");
-    static std::atomic<bool> attr64{false};
-    if (!attr64) {
+    static PerDevice attr64;
+    if (!attr64.has(c->device)) {
       TNAD_CK(cudaFuncSetAttribute(k_eigh_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSm));
-      attr64 = true;
+      attr64.mark(c->device);
     }
     // eigenvectors accumulate in global memory (L1-cached); H lives in shared memory
     double* Z = ws_d(c, p * p);
@@ -811,10 +811,10 @@ void polar_ns(tnad_ctx* c, const double* X, int64_t m, int iters, double* O, int
     polar_ns_gemm(c, X, m, iters, O, dev_info);
     return;
   }
-  static std::atomic<bool> attr{false};
-  if (!attr) {
+  static PerDevice attr;
+  if (!attr.has(c->device)) {
     TNAD_CK(cudaFuncSetAttribute(k_polar_ns, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 128 * 132 * 4));
-    attr = true;
+    attr.mark(c->device);
   }
   KernelTimer kt(c, "polar_ns", 0.0);
   const int nt = ((int)m + 3) / 4;

@@ -36,7 +36,6 @@
 // decomposes A in FP64 instead (graded spectra, whose small eigenvalues FP32
 // cannot separate).
 #include <algorithm>
-#include <atomic>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
@@ -45,6 +44,7 @@
 #include <vector>
 
 #include "orth_steps.h"
+#include "per_device.h"
 #include "tnad_internal.h"
 
 namespace tnad {
@@ -637,14 +637,14 @@ void solve_large_groups(tnad_ctx* c, int n, const double* S, const int* perm, co
 bool eig_refine(tnad_ctx* c, const double* A, int64_t n64, double* X, double* lam, const double* fro2, bool* graded) {
   if (n64 < 2 || n64 > kMaxN) return false;
   const int n = (int)n64;
-  static std::atomic<bool> attr{false};
-  if (!attr) {
+  static PerDevice attr;
+  if (!attr.has(c->device)) {
     const int rr_sm = (kMaxGroup * (kMaxGroup + 1) + kMaxGroup * kMaxGroup) * 8;
     const int rot_sm = (kMaxGroup * kMaxGroup + 128 * kMaxGroup) * 8;
     TNAD_CK(cudaFuncSetAttribute(k_ref_rr, cudaFuncAttributeMaxDynamicSharedMemorySize, rr_sm));
     TNAD_CK(cudaFuncSetAttribute(k_ref_rot_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, rot_sm));
     TNAD_CK(cudaFuncSetAttribute(k_ref_rot_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, rot_sm));
-    attr = true;
+    attr.mark(c->device);
   }
   WsScope scope(c);
   const int64_t nn = (int64_t)n * n;

@@ -44,12 +44,11 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstring>
-#include <mutex>
 
 #include "fp64_fast.cuh"
 #include "tc_common.cuh"
+#include "per_device.h"
 #include "tnad_internal.h"
 
 namespace tnad {
@@ -236,10 +235,10 @@ __global__ void __launch_bounds__(256) k_oz_prep(OzIn a, OzIn b, int nya, int64_
 
 template <int RB>
 void launch_oz_prep(tnad_ctx* c, const OzIn& a, const OzIn& b, int64_t K, int64_t Kp) {
-  static std::atomic<bool> attr{false};
-  if (!attr) {
+  static PerDevice attr;
+  if (!attr.has(c->device)) {
     TNAD_CK(cudaFuncSetAttribute(k_oz_prep<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOzPrepSmem));
-    attr = true;
+    attr.mark(c->device);
   }
   k_oz_prep<RB><<<(unsigned)((a.rows_pad + b.rows_pad) / RB), 256, (size_t)RB * (Kp + 1) * 8, c->stream>>>(
       a, b, (int)(a.rows_pad / RB), K, (int)Kp);
@@ -509,13 +508,10 @@ CUtensorMap make_plane_map(void* base, int64_t k_pad, int64_t rows_pad, int box_
 }
 
 void oz_prepare(tnad_ctx* c) {
-  static std::atomic<bool> done{false};
-  static std::mutex mu;
-  if (done) return;
-  std::lock_guard<std::mutex> lock(mu);
-  if (done) return;
+  static PerDevice done;
+  if (done.has(c->device)) return;
   TNAD_CK(cudaFuncSetAttribute(k_gemm_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
-  done = true;
+  done.mark(c->device);
 }
 
 }  // namespace

@@ -21,7 +21,6 @@
 // Every mbarrier wait is bounded (~2 s of %globaltimer); on timeout the CTA
 // records an error, drains its own TMA loads (bounded), frees TMEM and exits,
 // and the host reports TNAD_ERR_TIMEOUT.
-#include <atomic>
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -30,6 +29,7 @@
 
 #include "fp64_fast.cuh"
 #include "tc_common.cuh"
+#include "per_device.h"
 #include "tnad_internal.h"
 
 namespace tnad {
@@ -389,10 +389,10 @@ void launch_tc(tnad_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, void*
                int64_t Mp, int64_t Np, int64_t Kp, double beta, OutT* Cm, int64_t ldc, const char* timer_name,
                const TcEpi& ep = TcEpi{}) {
   using CF = Cfg<BN, SPLIT>;
-  static std::atomic<bool> attr{false};
-  if (!attr) {
+  static PerDevice attr;
+  if (!attr.has(c->device)) {
     TNAD_CK(cudaFuncSetAttribute(k_gemm_tc<BN, SPLIT, OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM));
-    attr = true;
+    attr.mark(c->device);
   }
   CUtensorMap tAh = make_map(Ah, Kp, Mp, BM, !SPLIT);
   CUtensorMap tBh = make_map(Bh, Kp, Np, BN, !SPLIT);

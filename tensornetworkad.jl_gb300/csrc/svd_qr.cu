@@ -26,7 +26,6 @@
 // 324) 366 → 48 ms; one n = 80 decomposition 4.9 → 1.1 ms, n = 255 26.7 → 4.5 ms.
 // At n = 324 the first QR takes 1.5 ms, the FP32 sweeps 2.0, the FP64 ones 2.4.
 #include <algorithm>
-#include <atomic>
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -34,6 +33,7 @@
 #include <cstdlib>
 
 #include "fp64_fast.cuh"
+#include "per_device.h"
 #include "sweep_rule.h"
 #include "tc_common.cuh"
 #include "tnad_internal.h"
@@ -1257,11 +1257,11 @@ void launch_sweeps_rj(tnad_ctx* c, int np, SvdArgs& a) {
       return;
     }
   }
-  static std::atomic<bool> attr{false};
-  if (!attr) {
+  static PerDevice attr;
+  if (!attr.has(c->device)) {
     TNAD_CK(cudaFuncSetAttribute(k_svd_sweeps<RJ, ACCV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  4 * kMaxSvdRows * 2 * 8));
-    attr = true;
+    attr.mark(c->device);
   }
   launch_grid(c, k_svd_sweeps<RJ, ACCV, false>, false, G, np, 128, smem, a);
 }
@@ -1291,11 +1291,11 @@ void launch_sweeps(tnad_ctx* c, int np, int rows, SvdArgs& a) {
 template <int B, int RV, int WP, bool EIG, bool CL>
 void launch_sweeps32_rv(tnad_ctx* c, int np, SvdArgs& a) {
   const int nreal = (a.n + B - 1) / B, G = std::max(1, (nreal + (nreal & 1)) / 2);
-  static std::atomic<bool> attr{false};
-  if (!attr) {
+  static PerDevice attr;
+  if (!attr.has(c->device)) {
     TNAD_CK(cudaFuncSetAttribute(k_sweeps32<B, RV, WP, EIG, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  2 * B * 2 * 128 * WP * RV * 4));  // 2B columns of W and V
-    attr = true;
+    attr.mark(c->device);
   }
   launch_grid(c, k_sweeps32<B, RV, WP, EIG, CL>, CL, G, np, 32 * B * WP, (size_t)2 * B * 2 * a.ld32 * sizeof(float), a);
 }
