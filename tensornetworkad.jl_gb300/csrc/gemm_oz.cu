@@ -561,7 +561,8 @@ void gemm_fp64tc(tnad_ctx* c, char ta, char tb, int64_t M, int64_t N, int64_t K,
     TNAD_CK(cudaMemsetAsync(eA, 0x80, (size_t)(Mp + Np) * sizeof(int), c->stream));
     const unsigned g = (unsigned)(Kp / 32 * ((Mp + Np) / 32));
     const dim3 b(32, 8);
-    k_oz_exp<<<g, b, 0, c->stream>>>(ia, ib, (int)(Mp / 32), K, Kp);
+    const int64_t ma = (M + 31) / 32, nb = (N + 31) / 32;  // padding has no bound to find
+    k_oz_exp<<<(unsigned)(Kp / 32 * (ma + nb)), b, 0, c->stream>>>(ia, ib, (int)ma, K, Kp);
     k_oz_slice<<<g, b, 0, c->stream>>>(ia, ib, (int)(Mp / 32), K, Kp);
     count_launch(c, 2);
   }
