@@ -2,8 +2,8 @@
 // in the reference (e.g. src/ctmrg.jl:130-140, src/variationalipeps.jl:52).
 // A contraction is mapped to one GEMM: free labels of A become the rows, free
 // labels of B the columns, shared labels the inner dimension.  The DFMA GEMM
-// reads and writes tensors in any label order.  For the tensor-core GEMMs,
-// operands whose memory order already matches a (transposed) matrix view are
+// reads and writes tensors in any label order.  For the tensor-core GEMMs and
+// large matrix-vector products, operands whose memory order already matches a (transposed) matrix view are
 // used in place and others packed by one permutation kernel, and the output is
 // permuted when the requested label order interleaves A's and B's free labels.
 #include <cstring>
@@ -111,7 +111,14 @@ void contract(tnad_ctx* c, int prec, const Ten& A0, const char* la0, const Ten& 
   };
   int64_t M = dims_of(A, la, Ml), N = dims_of(B, lb, Nl), K = dims_of(A, la, Kl);
 
-  if (M > 0 && N > 0 && K > 0 && gemm_is_f64(c, prec, M, N, K)) {
+  // A matrix in memory times a vector: the GEMM's matrix-vector kernels read it once,
+  // where a tile does 16 columns' multiply-adds for one.  They are the faster ones with
+  // a thread per row from four 16-row tiles an SM on (20000×50: 99 µs against 122 by
+  // tiles; 2000×2000: 686 against 322, a thread walks all of K), and by columns for up to
+  // 32 of them and long K (20×10^5: 198 against 286; 32×8192: 100 against 95).
+  const bool by_rows = is_concat(la, Ml, Kl), by_cols = is_concat(la, Kl, Ml);
+  const bool gemv = N == 1 && (by_rows ? M >= 64 * (int64_t)c->sm_count : by_cols && M <= 32 && K >= 16384);
+  if (M > 0 && N > 0 && K > 0 && !gemv && gemm_is_f64(c, prec, M, N, K)) {
     // DFMA tiles read and write the tensors in place, in any label order
     GemmMap am, ak, bk, bn, cm, cn;
     if (label_map(A->dim, la, Ml, am) && label_map(A->dim, la, Kl, ak) && label_map(B->dim, lb, Kl, bk) &&
@@ -124,10 +131,10 @@ void contract(tnad_ctx* c, int prec, const Ten& A0, const char* la0, const Ten& 
   const double* Ap = A->p;
   char ta = 'N';
   int64_t lda = M > 0 ? M : 1;
-  if (is_concat(la, Ml, Kl)) {
+  if (by_rows) {
     ta = 'N';
     lda = M;
-  } else if (is_concat(la, Kl, Ml)) {
+  } else if (by_cols) {
     ta = 'T';
     lda = K;
   } else {
