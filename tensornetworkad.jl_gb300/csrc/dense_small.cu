@@ -418,8 +418,6 @@ __device__ __forceinline__ float hsum2(uint64_t a) {
   return __uint_as_float((unsigned)a) + __uint_as_float((unsigned)(a >> 32));
 }
 
-constexpr int kEigh32MaxP = 160;  // W and V of FP32 in one CTA's shared memory
-
 template <int RV>  // 16-byte row chunks per lane: ⌈p/32⌉
 __global__ void __launch_bounds__(64 * RV, 1) k_eigh32(const double* __restrict__ A, int p, int max_sweeps,
                                                 double* __restrict__ lam, double* __restrict__ Wout,

@@ -802,11 +802,11 @@ bool eig_refine(tnad_ctx* c, const double* A, int64_t n64, double* X, double* la
 }
 
 // Eigendecomposition H = W·diag(lam)·Wᵀ of a small symmetric p×p matrix
-// (p ≤ 256) to FP64 accuracy: the one-CTA FP32 Jacobi solve (eigenvalue rule,
+// (p ≤ kEigh32MaxP) to FP64 accuracy: the one-CTA FP32 Jacobi solve (eigenvalue rule,
 // so ±λ pairs stay apart) polished by the product refinement above, sorted by
-// |λ| descending.  false: the refinement did not converge (W, lam untouched).
+// |λ| descending.  false: a larger p, or no convergence (W, lam untouched).
 bool eigh_fp32_refined(tnad_ctx* c, const double* H, int64_t p, double* W, double* lam) {
-  if (!c->eig_refine || p < 2 || p > 256) return false;
+  if (!c->eig_refine || p < 2 || p > kEigh32MaxP) return false;
   WsScope scope(c);
   double* X = ws_d(c, p * p);
   double* l = ws_d(c, p);

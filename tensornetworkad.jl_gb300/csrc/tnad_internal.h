@@ -303,14 +303,15 @@ int sweeps32_eig(tnad_ctx* c, const double* A, int64_t n, const double* fro2, do
 // first measurement showed no approximate eigendecomposition, as for graded spectra.
 bool eig_refine(tnad_ctx* c, const double* A, int64_t n, double* X, double* lam, const double* fro2,
                 bool* graded = nullptr);
-// FP64-accurate eigendecomposition of a small symmetric p×p matrix (p ≤ 256):
-// one-CTA FP32 Jacobi, then eig_refine; W, lam sorted by |λ| descending.
-// false: the refinement did not converge (W, lam untouched).
+constexpr int kEigh32MaxP = 160;  // FP32 eigenproblems in one CTA: W and V fit its shared memory
+// FP64-accurate eigendecomposition of a small symmetric p×p matrix: one-CTA FP32
+// Jacobi, then eig_refine; W, lam sorted by |λ| descending.  false: p > kEigh32MaxP,
+// or the refinement did not converge (W, lam untouched).
 bool eigh_fp32_refined(tnad_ctx* c, const double* H, int64_t p, double* W, double* lam);
-// Symmetric eigendecomposition of a small p×p matrix (p ≤ 256) by cyclic Jacobi in
+// Symmetric eigendecomposition of a small p×p matrix (p ≤ 159) by cyclic Jacobi in
 // one CTA: A = W·diag(lam)·Wᵀ, sorted by |lam| descending.
 void eigh_small(tnad_ctx* c, const double* A, int64_t p, double* W, double* lam);
-// The same with the sweep precision (fp32: FP32 rotations, FP64 in/out), a sweep
+// The same with the sweep precision (fp32: FP32 rotations, FP64 in/out, p ≤ kEigh32MaxP), a sweep
 // cap, the sweep count in dev_info[0] (may be null), and the order: |λ|
 // descending, or λ descending when by_value.
 void eigh_small_prec(tnad_ctx* c, bool fp32, const double* A, int64_t p, double* W, double* lam, int max_sweeps,
