@@ -546,9 +546,9 @@ void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, d
   TNAD_REQUIRE(m >= n && n >= 1, TNAD_ERR_SHAPE, "svd_jacobi: needs m >= n >= 1");
   // symmetric A at LAPACK-level accuracy: below kPrecondMinN, and where the
   // refinement below is not taken, QR-preconditioned sweeps (svd_qr.cu)
-  const bool qrj = symmetric && rel_sweeps == 0 && m == n && svd_qrj_fits(n, n);
+  const bool qrj = symmetric && rel_sweeps == 0 && m == n && svd_qrj_fits(n);
   if (qrj && (n < kPrecondMinN || !c->eig_refine)) {
-    svd_qrj(c, 1, &A, n, n, &U, &S, &V, true);
+    svd_qrj(c, 1, &A, n, &U, &S, &V, true);
     return;
   }
   WsScope scope(c);
@@ -601,7 +601,7 @@ void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, d
       ++c->eig_fallback;
       refine = false;
       if (qrj) {
-        svd_qrj(c, 1, &A, n, n, &U, &S, &V, true);
+        svd_qrj(c, 1, &A, n, &U, &S, &V, true);
         return;
       }
     }
@@ -675,7 +675,7 @@ void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, d
         c->eig_skip_left = kEigSkip;
       }
       if (qrj) {
-        svd_qrj(c, 1, &A, n, n, &U, &S, &V, true);
+        svd_qrj(c, 1, &A, n, &U, &S, &V, true);
         return;
       }
     }

@@ -61,7 +61,7 @@ enum { kiRank = 0, kiBad = 1, kiSweeps = 2, kiExp = 3, kiErr = 4, kiPre = 5, kiM
 struct SvdProb {
   const double* A;
   double *X, *X2, *Vx;    // Rᵀ (n×n), R₂ᵀ and the accumulated rotations; leading dimension ldx
-  double *H, *H2;         // Householder vectors of the two factorisations, m×n and n×n
+  double *H, *H2;         // Householder vectors of the two factorisations, n×n
   double *hinv, *hinv2;   // 2/vᵀv of each
   int *perm, *perm2;      // perm[k]: column at pivot position k
   double *cand;           // 2 × G × ldc candidate columns, each entry with its tag
@@ -75,7 +75,7 @@ struct SvdProb {
 
 struct SvdArgs {
   SvdProb p[2];
-  int m, n, ldx, ldc, ld32;
+  int n, ldx, ldc, ld32;
   int second;      // run the second QR also when r = n
   float trunc;     // rank cut relative to the first pivot
   double tol;      // Jacobi: |cos| above which a pair rotates (FP64 and FP32 sweeps)
@@ -188,12 +188,12 @@ struct SpinLimit {
 //     where they lie: no counter barrier, no fence and no read of the keys after
 //     them; a CTA reads the column once, for all its warps (read by every warp, 456
 //     requests queue on each of its lines);
-//   - in a cluster the keys, and columns up to 128 rows, are stored into every
-//     CTA's shared memory before the barrier;
+//   - in a cluster (up to 64 columns) keys and columns are stored into every CTA's
+//     shared memory before the barrier;
 //   - ‖x‖² and xᵀc are summed in one pass over registers and shuffles (vᵀc =
 //     xᵀc − β·c_k needs no v).
 // Two buffers by parity: a CTA is at most one step ahead of the slowest.
-// STAGE 0: A (m×n, scaled by a power of two) → H, hinv, perm, rank, X = Rᵀ in
+// STAGE 0: A (n×n, scaled by a power of two) → H, hinv, perm, rank, X = Rᵀ in
 // pivot order.  STAGE 1: the r columns of X → H2, hinv2, perm2, X2 = R₂ᵀ.
 // ---------------------------------------------------------------------------
 template <int R, bool CL, int STAGE>
@@ -203,8 +203,7 @@ __global__ void __launch_bounds__(256) k_qrcp(SvdArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
   int m, n;
   if (STAGE == 0) {
-    m = a.m;
-    n = a.n;
+    m = n = a.n;
   } else {
     m = a.n;
     n = q.info[kiRank];
@@ -214,10 +213,9 @@ __global__ void __launch_bounds__(256) k_qrcp(SvdArgs a) {
   double* hinv = STAGE == 0 ? q.hinv : q.hinv2;
   int* perm = STAGE == 0 ? q.perm : q.perm2;
   double* X = STAGE == 0 ? q.X : q.X2;
-  constexpr bool kPush = CL && R <= 4;  // candidate columns go to every CTA's shared memory
   __shared__ unsigned long long wkey[8], rkey[8], ckey[CL ? 2 : 1][CL ? kQrCl : 1];
-  __shared__ double xs[kPush ? 1 : 32 * R];  // the step's column
-  __shared__ double ccol[kPush ? 2 : 1][kPush ? kQrCl : 1][kPush ? 32 * R : 1];
+  __shared__ double xs[CL ? 1 : 32 * R];  // the step's column
+  __shared__ double ccol[CL ? 2 : 1][CL ? kQrCl : 1][CL ? 32 * R : 1];  // CL: candidate columns of every CTA
   __shared__ unsigned picked_mask[kMaxSvdRows / 32];
   __shared__ int dead;
   if (threadIdx.x == 0) dead = 0;
@@ -316,7 +314,7 @@ __global__ void __launch_bounds__(256) k_qrcp(SvdArgs a) {
           asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&q.key[buf * G + cta]), "l"(best) : "memory");
         }
       }
-      if (kPush) {
+      if (CL) {
         const uint32_t la = (uint32_t)__cvta_generic_to_shared(&ccol[buf][cta][0]);
         for (int g = 0; g < G; ++g) {
           uint32_t ra;
@@ -380,7 +378,7 @@ __global__ void __launch_bounds__(256) k_qrcp(SvdArgs a) {
       if (n2 <= thr2) break;  // the rest is below the rounding of A
     }
     if (threadIdx.x == 0) picked_mask[wj >> 5] |= 1u << (wj & 31);
-    if (!kPush) {
+    if (!CL) {
       const double* win = q.cand + 2 * ((int64_t)buf * G + (wj % G)) * a.ldc;
       SpinLimit spin;
       for (int row0 = (k & ~31) + threadIdx.x; row0 < m; row0 += 4 * blockDim.x) {
@@ -407,7 +405,7 @@ __global__ void __launch_bounds__(256) k_qrcp(SvdArgs a) {
       if (dead) return;
     }
     if (!live && !(cta == 0 && warp == 0)) continue;  // nothing left to update
-    const double* wsh = kPush ? &ccol[kPush ? buf : 0][kPush ? wj % G : 0][0] : xs;
+    const double* wsh = CL ? &ccol[CL ? buf : 0][CL ? wj % G : 0][0] : xs;
     double x[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -1045,7 +1043,7 @@ __global__ void k_svd_norms(SvdArgs a) {
 template <bool SYM>
 __global__ void __launch_bounds__(128) k_svd_place(SvdArgs a) {
   const SvdProb& q = a.p[blockIdx.y];
-  const int j = blockIdx.x, m = a.m, n = a.n;
+  const int j = blockIdx.x, n = a.n;
   const int rc = q.info[kiRank];
   if (q.info[kiErr]) return;  // a wait gave up: perm and perm2, which this kernel stores through, may be unwritten
   const bool two = a.second || rc < n;
@@ -1063,12 +1061,12 @@ __global__ void __launch_bounds__(128) k_svd_place(SvdArgs a) {
     __syncthreads();
     rk = part[0] + part[1] + part[2] + part[3];
   }
-  double* u = SYM ? nullptr : q.U + (int64_t)rk * m;
+  double* u = SYM ? nullptr : q.U + (int64_t)rk * n;
   double* v = q.V + (int64_t)rk * n;
   if (q.info[kiBad]) {
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     if (!SYM)
-      for (int i = threadIdx.x; i < m; i += blockDim.x) u[i] = nan;
+      for (int i = threadIdx.x; i < n; i += blockDim.x) u[i] = nan;
     for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = nan;
     if (threadIdx.x == 0) q.S[rk] = nan;
     return;
@@ -1076,7 +1074,7 @@ __global__ void __launch_bounds__(128) k_svd_place(SvdArgs a) {
   if (threadIdx.x == 0) q.S[rk] = scalbn(sj, q.info[kiExp]);
   if (j >= rc) {
     if (!SYM)
-      for (int i = threadIdx.x; i < m; i += blockDim.x) u[i] = i == j ? 1.0 : 0.0;
+      for (int i = threadIdx.x; i < n; i += blockDim.x) u[i] = i == j ? 1.0 : 0.0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = i == j ? 1.0 : 0.0;
     return;
   }
@@ -1088,8 +1086,7 @@ __global__ void __launch_bounds__(128) k_svd_place(SvdArgs a) {
   }
   const double* w = (q.W ? q.W : q.X2) + (int64_t)j * a.ldx;
   double* o = SYM ? v : u;
-  const int mo = SYM ? n : m;
-  for (int i = rc + threadIdx.x; i < mo; i += blockDim.x) o[i] = 0.0;
+  for (int i = rc + threadIdx.x; i < n; i += blockDim.x) o[i] = 0.0;
   for (int i = threadIdx.x; i < rc; i += blockDim.x) o[q.perm2[i]] = w[i] * inv;
   if (!SYM) {
     const double* x = q.Vx + (int64_t)j * a.ldx;
@@ -1107,7 +1104,7 @@ __global__ void __launch_bounds__(128) k_svd_apply_q(SvdArgs a) {
   const int rc = q.info[kiRank], n = a.n;
   if (q.info[kiErr] || q.info[kiBad]) return;
   if (SYM && rc == n) return;  // the eigenvectors are in place
-  const int rows = STAGE == 0 ? a.m : n;
+  const int rows = n;
   const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (col >= n) return;
   const double* H = STAGE == 0 ? q.H : q.H2;
@@ -1238,7 +1235,7 @@ void launch_qrcp(tnad_ctx* c, int np, int cols, SvdArgs& a) {
   // CTAs of 4 warps, 8000 in a cluster of 16 CTAs of 8, whose FP64 instructions
   // share the quadrants), then 4 warps a CTA, or more where the SMs run out: fewer
   // CTAs read the step's keys and column (n = 324: 10300 clocks, 12600 with 152 CTAs).
-  if (cols <= 64) {
+  if constexpr (R == 2) {
     const int G = std::min(kQrCl, (cols + 3) / 4);
     launch_grid(c, k_qrcp<R, true, STAGE>, true, G, np, 32 * ((cols + G - 1) / G), 0, a);
   } else {
@@ -1391,7 +1388,7 @@ int sweeps32_eig(tnad_ctx* c, const double* A, int64_t n, const double* fro2, do
   TNAD_REQUIRE(n >= 2 && n <= kMaxSvdRows, TNAD_ERR_SHAPE, "sweeps32_eig: n must be in [2,1024]");
   WsScope scope(c);
   SvdArgs a = {};
-  a.m = a.n = a.ldx = (int)n;
+  a.n = a.ldx = (int)n;
   a.ld32 = (int)((n + 3) & ~(int64_t)3);
   a.fro2 = fro2;
   SvdProb& q = a.p[0];
@@ -1416,28 +1413,27 @@ int sweeps32_eig(tnad_ctx* c, const double* A, int64_t n, const double* fro2, do
   return sweeps;
 }
 
-bool svd_qrj_fits(int64_t m, int64_t n) { return m >= n && n >= 2 && m <= kMaxSvdRows; }
+bool svd_qrj_fits(int64_t n) { return n >= 2 && n <= kMaxSvdRows; }
 
-void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, double* const* U, double* const* S,
+void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t n, double* const* U, double* const* S,
              double* const* V, bool symmetric) {
-  TNAD_REQUIRE(svd_qrj_fits(m, n) && (np == 1 || np == 2), TNAD_ERR_SHAPE, "svd_qrj: needs 1024 >= m >= n >= 2");
+  TNAD_REQUIRE(svd_qrj_fits(n) && (np == 1 || np == 2), TNAD_ERR_SHAPE, "svd_qrj: n must be in [2,1024]");
   if (np == 2 && n > 8 * (int64_t)(c->sm_count / 2)) {  // a CTA of the QR holds at most 8 columns
-    svd_qrj(c, 1, A, m, n, U, S, V, symmetric);
-    svd_qrj(c, 1, A + 1, m, n, U + 1, S + 1, V + 1, symmetric);
+    svd_qrj(c, 1, A, n, U, S, V, symmetric);
+    svd_qrj(c, 1, A + 1, n, U + 1, S + 1, V + 1, symmetric);
     return;
   }
   TNAD_REQUIRE(n <= 8 * (int64_t)(c->sm_count / np), TNAD_ERR_SHAPE, "svd_qrj: too many columns for this GPU");
   WsScope scope(c);
   SvdArgs a = {};
-  a.m = (int)m;
   a.n = (int)n;
   a.ldx = (int)((n + 1) & ~(int64_t)1);
-  a.ldc = (int)m;
+  a.ldc = (int)n;
   a.ld32 = (int)((n + 3) & ~(int64_t)3);
   a.second = symmetric ? 0 : 1;
   a.trunc = 0.5f * (float)DBL_EPSILON;
-  a.tol = 2.0 * std::sqrt((double)std::max<int64_t>(m, 16)) * DBL_EPSILON;
-  a.tol32 = 4.0f * std::sqrt((float)m) * FLT_EPSILON;
+  a.tol = 2.0 * std::sqrt((double)std::max<int64_t>(n, 16)) * DBL_EPSILON;
+  a.tol32 = 4.0f * std::sqrt((float)n) * FLT_EPSILON;
   a.max_sweeps = kSvdSweeps;
   if (c->fault_once == kFaultJacobiCap) {  // failure-path test: one sweep only
     a.max_sweeps = 1;
@@ -1461,7 +1457,7 @@ void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, 
     q.Wbuf = pre ? ws_d(c, (int64_t)a.ldx * n) : nullptr;
     q.W32 = pre ? ws_f(c, (int64_t)a.ld32 * n) : nullptr;
     q.V32 = pre ? ws_f(c, (int64_t)a.ld32 * n) : nullptr;
-    q.H = ws_d(c, m * n);
+    q.H = ws_d(c, n * n);
     q.H2 = ws_d(c, n * n);
     q.hinv = ws_d(c, 2 * n);
     q.hinv2 = q.hinv + n;
@@ -1481,13 +1477,13 @@ void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, 
   int h[2 * kiBar];
   {
     KernelTimer kt(c, "svd_qrj", np * 9.0 * nn * nn * nn, 8);
-    if (m <= 64)
+    if (n <= 64)
       svd_qrj_r<2>(c, np, symmetric, a, h);
-    else if (m <= 128)
+    else if (n <= 128)
       svd_qrj_r<4>(c, np, symmetric, a, h);
-    else if (m <= 256)
+    else if (n <= 256)
       svd_qrj_r<8>(c, np, symmetric, a, h);
-    else if (m <= 512)
+    else if (n <= 512)
       svd_qrj_r<16>(c, np, symmetric, a, h);
     else
       svd_qrj_r<32>(c, np, symmetric, a, h);

@@ -279,12 +279,12 @@ Ten contract_shape(const Ten& A, const char* la, const Ten& B, const char* lb, c
 void svd_jacobi(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, double* S,
                 double* V, bool symmetric, int rel_sweeps = 20);
 // SVD to LAPACK-level accuracy (ε·‖A‖ on every triplet) of np (1 or 2) matrices
-// of the same shape m×n (svd_qrj_fits: 1024 ≥ m ≥ n ≥ 2): rank-revealing QR,
+// of the same size n×n (svd_qrj_fits: 2 ≤ n ≤ 1024): rank-revealing QR,
 // then Jacobi on the triangular factor, each one launch (svd_qr.cu).  Values
 // below the rounding of A come back as 0, their vectors as an orthonormal
 // completion.  symmetric: V eigenvectors, U = V·sign(λ).
-bool svd_qrj_fits(int64_t m, int64_t n);
-void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t m, int64_t n, double* const* U, double* const* S,
+bool svd_qrj_fits(int64_t n);
+void svd_qrj(tnad_ctx* c, int np, const double* const* A, int64_t n, double* const* U, double* const* S,
              double* const* V, bool symmetric);
 // Eigenvectors of a symmetric A (n ≤ 1024) from an orthonormal basis X that
 // diagonalises it up to groups of equal |λ|, by FP64 Jacobi sweeps with the

@@ -83,18 +83,15 @@ __global__ void k_maxnorm_bwd(int64_t n, const double* __restrict__ dan, double 
   }
 }
 
-// thin SVD for any shape; U m×ns, V n×ns, ns = min(m,n).  lapack: accurate to
-// ε·‖A‖ (svd_qrj) instead of relative to every singular value
-static void svd_any(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, double* S, double* V, bool lapack) {
+// thin SVD for any shape; U m×ns, V n×ns, ns = min(m,n)
+static void svd_any(tnad_ctx* c, const double* A, int64_t m, int64_t n, double* U, double* S, double* V) {
   if (m < n) {
     WsScope scope(c);
     double* At = ws_d(c, m * n);
     Ten t = make_ten(const_cast<double*>(A), {m, n});
     int perm[2] = {1, 0};
     permute(c, t, perm, At);
-    svd_any(c, At, n, m, V, S, U, lapack);  // Aᵀ = V S Uᵀ
-  } else if (lapack && svd_qrj_fits(m, n)) {
-    svd_qrj(c, 1, &A, m, n, &U, &S, &V, false);
+    svd_any(c, At, n, m, V, S, U);  // Aᵀ = V S Uᵀ
   } else {
     svd_jacobi(c, A, m, n, U, S, V, false);
   }
@@ -151,27 +148,27 @@ static void trg_svd_finish(tnad_ctx* c, int chi, double tol, std::vector<double>
 
 void trg_svd_fwd(tnad_ctx* c, const double* t, const int64_t dd[4], int chi, double tol, TrgSvd& s, DevPool* pool) {
   trg_svd_alloc(dd, s, pool);
-  svd_any(c, t, s.m, s.n, s.U, s.S, s.V, false);
+  svd_any(c, t, s.m, s.n, s.U, s.S, s.V);
   std::vector<double> hs(s.ns);
   TNAD_CK(cudaMemcpyAsync(hs.data(), s.S, s.ns * 8, cudaMemcpyDeviceToHost, c->stream));
   TNAD_CK(cudaStreamSynchronize(c->stream));
   trg_svd_finish(c, chi, tol, hs, s, pool);
 }
 
-// Both splits of a TRG step.  They are independent and of the same shape (the
-// two diagonals of one tensor), so one batch of svd_qrj decomposes both: its
-// sweeps are latency-bound and a 400×400 split alone leaves half of the SMs idle.
+// Both splits of a TRG step.  They are independent and of the same square shape
+// (the two diagonals of one tensor), so one batch of svd_qrj decomposes both, to ε·‖A‖:
+// its sweeps are latency-bound and a 400×400 split alone leaves half of the SMs idle.
 static void trg_svd_pair(tnad_ctx* c, const double* t1, const int64_t d1[4], const double* t2, const int64_t d2[4],
                          int chi, double tol, TrgSvd& s1, TrgSvd& s2, DevPool* pool) {
   trg_svd_alloc(d1, s1, pool);
   trg_svd_alloc(d2, s2, pool);
-  if (s1.m == s2.m && s1.n == s2.n && svd_qrj_fits(s1.m, s1.n)) {
+  if (s1.m == s1.n && s2.m == s1.m && s2.n == s1.n && svd_qrj_fits(s1.n)) {
     const double* A[2] = {t1, t2};
     double *U[2] = {s1.U, s2.U}, *S[2] = {s1.S, s2.S}, *V[2] = {s1.V, s2.V};
-    svd_qrj(c, 2, A, s1.m, s1.n, U, S, V, false);
+    svd_qrj(c, 2, A, s1.n, U, S, V, false);
   } else {
-    svd_any(c, t1, s1.m, s1.n, s1.U, s1.S, s1.V, true);
-    svd_any(c, t2, s2.m, s2.n, s2.U, s2.S, s2.V, true);
+    svd_any(c, t1, s1.m, s1.n, s1.U, s1.S, s1.V);
+    svd_any(c, t2, s2.m, s2.n, s2.U, s2.S, s2.V);
   }
   std::vector<double> h1(s1.ns), h2(s2.ns);
   TNAD_CK(cudaMemcpyAsync(h1.data(), s1.S, s1.ns * 8, cudaMemcpyDeviceToHost, c->stream));
