@@ -175,7 +175,7 @@ FP32_NOMINAL_TFLOPS = 80.5
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the FP64 tensor-core
 # GEMM (k_gemm_oz), mean over the first 300 of its launches in one cold D=4,
 # chi=64 solve (one ncu capture of that kernel on this workload)
-OZ_TRAFFIC_BYTES = 3321780
+OZ_TRAFFIC_BYTES = 3314889
 
 
 def peaks():
@@ -402,10 +402,10 @@ def run_gb300(args):
                      FP64_NOMINAL_TFLOPS, nominal),
         "jacobi_round_f32": ("k_sweeps32<EIG> (FP32 Jacobi sweeps of the 1024x1024 corner's symmetric SVD, "
                              "eigenvalue rule, block rounds of 4 columns)", "fp32", 1.0, FP32_NOMINAL_TFLOPS, nominal),
-        "jacobi_round_small": ("k_jacobi_round_cta<2, double> (FP64 rounds of the p x p Rayleigh-Ritz problems of the "
-                               "subspace solver)", "fp64", 1.0, FP64_NOMINAL_TFLOPS, nominal),
-        "jacobi_round": ("k_jacobi_round_cta<8, double> (FP64 sweeps of the corner SVD where the refinement falls "
-                         "back)", "fp64", 1.0, FP64_NOMINAL_TFLOPS, nominal),
+        "jacobi_round_small": ("k_jacobi_round_cta<2, double> (FP64 rounds of general SVDs below 256 columns: none in a "
+                               "solve, whose p x p problems are refined)", "fp64", 1.0, FP64_NOMINAL_TFLOPS, nominal),
+        "jacobi_round": ("k_jacobi_round_cta<16, double> (FP64 sweeps of corner SVDs above 1024 columns where the "
+                         "refinement falls back)", "fp64", 1.0, FP64_NOMINAL_TFLOPS, nominal),
         "gemm_tf32x3": ("k_gemm_tf32x3 (tcgen05 kind::tf32, 3 split products)", "tensor", 3.0, bf16_peak / 2.0,
                         f"{pk_kind} bf16 burst / 2 (dense TF32 rate)"),
     }

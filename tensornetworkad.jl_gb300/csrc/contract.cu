@@ -3,9 +3,10 @@
 // A contraction is mapped to one GEMM: free labels of A become the rows, free
 // labels of B the columns, shared labels the inner dimension.  The DFMA GEMM
 // reads and writes tensors in any label order.  For the tensor-core GEMMs and
-// large matrix-vector products, operands whose memory order already matches a (transposed) matrix view are
-// used in place and others packed by one permutation kernel, and the output is
-// permuted when the requested label order interleaves A's and B's free labels.
+// large matrix-vector products, operands whose memory order already matches a
+// (transposed) matrix view are used in place and others packed by one permutation
+// kernel, and the output is permuted when the requested label order interleaves
+// A's and B's free labels.
 #include <cstring>
 #include <string>
 

@@ -36,8 +36,13 @@ namespace tnad {
 // updates its own columns of both parts.  The owner of the next panel updates
 // and factors that one first and leaves its other columns for the time between
 // its arrival at the barrier and the others'.  R⁻¹ = Yᵀ.  Panels of 8 on 8 CTAs
-// without that order took 107 µs, this 86 (p = 96, factor and inverse).  Also replaces the FP32 factorisation that
-// the TF32 phase used for its second pass (156 µs).
+// without that order took 107 µs, this 86 (p = 96, factor and inverse): a chain of
+// p/4 panels, half of the warps' stalls at barriers, the FP64 pipe 15% busy.
+//
+// near > 0 (a second pass): where p·max|G − I|² ≤ near, R⁻¹ to first order instead of a
+// factorisation (5 µs).  The callers' bounds are what the product that uses R⁻¹
+// rounds: 2^-26 before a 3xTF32 one, where orthogonality is then good to 1.5e-8 (an FP32
+// factorisation, which stood there before, left ~1e-7), 2^-55 before an FP64 one.
 constexpr double kPivotFloor = 1e-14;
 constexpr int kCholC = 16;    // CTAs of the cluster
 constexpr int kCholNB = 4;    // columns of a panel
@@ -48,9 +53,9 @@ constexpr int kCholPanels = (kCholMaxP / kCholNB + kCholC - 1) / kCholC;  // pan
 __global__ void __launch_bounds__(256) k_chol_inv(const double* __restrict__ G, int p, double floor_rel, float near,
                                                   double* __restrict__ Rinv, int* __restrict__ fail) {
   extern __shared__ __align__(16) double csm[];
-  double* A = csm;                                        // own columns of L, kCholPanels·8 × kCholLd
+  double* A = csm;                                        // own columns of L, kCholPanels·kCholNB × kCholLd
   double* Y = A + kCholPanels * kCholNB * kCholLd;        // own columns of L⁻¹
-  double* Lp = Y + kCholPanels * kCholNB * kCholLd;       // the current panel, 8 × kCholLd
+  double* Lp = Y + kCholPanels * kCholNB * kCholLd;       // the current panel, kCholNB × kCholLd
   __shared__ double fl_sh;
   __shared__ unsigned emax_sh;  // FP32 bits of max|E| over the own columns
   const int rank = blockIdx.x;

@@ -14,9 +14,9 @@
 //          |S_ij + λ_j R_ij| > η |λ_j − λ_i| (either order); groups are the
 //          intervals of the |λ|-sorted order spanned by such pairs
 //   Rayleigh–Ritz inside every group of size ≥ 2 whose largest |λ| is above the
-//          noise level max(4nε‖A‖_F, 8·max|S_ij| of weakly coupled pairs) (eigh of S on the group,
-//          one CTA per group, FP64 Jacobi in shared memory; S and G follow the
-//          rotation).  Eigenvalues below that level cannot yet be told apart
+//          noise level max(4nε‖A‖_F, 8·max|S_ij| of weakly coupled pairs) (eigh of
+//          S on the group, one CTA per group, FP64 Jacobi in shared memory; S and G
+//          follow the rotation).  Eigenvalues below that level cannot yet be told apart
 //          from zero; a null space stays one unsolved group, and small
 //          eigenvalues are solved once the error has dropped below them
 //   E_ij = (S_ij + λ_j R_ij)/(λ_j − λ_i) between groups, R_ij/2 inside one
@@ -24,11 +24,12 @@
 // until max|S_ij|/‖A‖_F ≤ 1e-10 and max|R_ij| ≤ 1e-8 with no group to solve (and,
 // where one stays unsolved, the coupling between groups is at the rounding
 // floor, so that only a null space does), and |E|·|S| ≤ 2^-47·‖A‖_F for that
-// update; the
-// plain path then measures S and G once more by DFMA products and takes the last
-// correction and λ_j = S_jj/G_jj from those, its iterations before that run on
-// the tensor cores (D=4, χ=64 plain energy and gradient, 6 steps: 724 → 250 ms,
-// gradient error against 64 bits 1.4e-14 → 5e-15).
+// update.  The plain path then measures S and G once more by DFMA products and takes
+// the last correction and λ_j = S_jj/G_jj from those; its iterations before that run
+// on the tensor cores (D=4, χ=64 plain energy and gradient, 6 steps: 724 → 250 ms,
+// gradient error against 64 bits 1.4e-14 → 5e-15).  In 113-bit arithmetic, n = 256:
+// residual 1.3e-15 to 2.4e-15·‖A‖₂ in the Frobenius norm over spectra like a corner's
+// (all iterations on DFMA: 1.3e-15 to 3.9e-15), ‖XᵀX − I‖_F 4.6e-15 (5.5e-15).
 // A group larger than kMaxGroup (a dense cluster of small eigenvalues, closer to
 // one another than the start's error of ~1e-6·‖A‖) is rotated by FP32 Jacobi
 // sweeps on its own block of S, whose norm is that of the group, and measured

@@ -20,7 +20,10 @@
 // rounds.  The corners and TRG splits are graded (singular values from 1 to
 // 1e-16): plain Jacobi sweeps took 9-36 of them there, on the triangular factor
 // it is 6-10, and the rank cut leaves ~250 of 400 columns of a χ = 20 split.
-// Each stage is one cooperative kernel (one launch instead of n − 1 per sweep).
+// Each factorisation and each kind of sweep is one launch (one instead of n − 1 per
+// sweep), cooperative, or a cluster where n is small.  From kPreMin columns on the
+// FP32 sweeps are followed by a host wait (the rank sizes what comes next), two
+// corrections of V as products, and W = X·V.
 // Measured on one GB300 against FP64 element rounds (k_jacobi_round_cta): TRG at
 // χ = 20, 7 steps with gradient 718 → 24 ms; D=3, χ=36 energy and gradient (n =
 // 324) 366 → 48 ms; one n = 80 decomposition 4.9 → 1.1 ms, n = 255 26.7 → 4.5 ms.
