@@ -1150,7 +1150,7 @@ __global__ void __launch_bounds__(128) k_svd_apply_q(SvdArgs a) {
 // X spans what it has to, but only up to rotations by ~ε·‖A‖/||λ_i| − |λ_j|| between
 // columns: where λ_i and λ_j have opposite signs and about the same size (exact ±λ
 // pairs, any size; or close ones), x_j is then no eigenvector and ±x_j no left vector.
-// M = XᵀAX shows it: an entry above thr_rel·σ_1, twice the rounding of M, is such a
+// M = XᵀAX shows it: an entry above thr_rel·σ_1, the rounding of M, is such a
 // coupling.  A column without one is kept, a pair takes the eigenvectors of its 2×2
 // block, and a column in a larger group (a multiplet of both signs) sets *multi,
 // upon which the caller separates them by eigenvalue sweeps (eig_separate).
@@ -1179,7 +1179,8 @@ __global__ void __launch_bounds__(128) k_svd_sym_basis(int n, const double* __re
   const int o = cnt[0] == 1 ? who[0] : -1;
   if (o >= 0) scan(o, 1);
   __syncthreads();
-  const bool pair = o >= 0 && cnt[1] == 1;  // (M is symmetric to the bit: the partner's partner is j)
+  // (M is symmetric up to rounding: at the threshold only one of the two may see the other)
+  const bool pair = o >= 0 && cnt[1] == 1 && who[1] == j;
   if (cnt[0] > 0 && !pair && threadIdx.x == 0) *multi = 1;
   const int lo = pair ? min(j, o) : j, hi = pair ? max(j, o) : j;
   double cl = 1.0, ch = 0.0, lam = M[j + (int64_t)j * n];
